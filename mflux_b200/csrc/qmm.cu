@@ -30,6 +30,7 @@
 #include "host_util.cuh"
 #include "ptx.cuh"
 #include "qmm_common.cuh"
+#include "qmm_epilogue.cuh"
 #include "qmm_t.cuh"
 #include "qmv.cuh"
 
@@ -67,6 +68,7 @@ struct Params {
   int64_t res_row_stride, res_batch_stride;
   void* y;
   int64_t y_row_stride, y_batch_stride;
+  bool wide;  // 32-byte aligned output and residual rows
   // MFX_EPI_PEER_SCATTER: partial rows go to slot [sc_rank] of the rank that owns them (see include/mfx.h)
   int sc_world, sc_rank;
   int64_t sc_rows_per_rank, sc_row_offset;
@@ -541,75 +543,8 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
           }
           __syncwarp();
         }
-      } else
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t acc[32];
-        tmem_ld_32x32(t_addr + c * 32, acc);
-        tmem_ld_wait();
-        if (row_ok) {
-#pragma unroll
-          for (int g8 = 0; g8 < 4; ++g8) {
-            const int col = c * 32 + g8 * 8;
-            if (n0 + col >= p.N) break;
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(acc[g8 * 8 + j]) + bias_s[col + j];
-            if (EPI == MFX_EPI_GELU_ERF) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = gelu_erf(v[j]);
-            } else if (EPI == MFX_EPI_GELU_TANH) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = gelu_tanh(v[j]);
-            } else if (EPI == MFX_EPI_SILU) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = silu(v[j]);
-            } else if (EPI == MFX_EPI_GATE_RESIDUAL) {
-              float rs[8];
-              if constexpr (sizeof(OUT) == 4) {
-                // the float32 residual stream is read once and written once per launch and is larger than L2:
-                // streaming loads / stores keep it from evicting the activation tiles the other n-tiles re-read
-                const float4 r0 = __ldcs(reinterpret_cast<const float4*>(rrow + col));
-                const float4 r1 = __ldcs(reinterpret_cast<const float4*>(rrow + col + 4));
-                rs[0] = r0.x; rs[1] = r0.y; rs[2] = r0.z; rs[3] = r0.w;
-                rs[4] = r1.x; rs[5] = r1.y; rs[6] = r1.z; rs[7] = r1.w;
-              } else {
-                const uint4 raw = *reinterpret_cast<const uint4*>(rrow + col);
-                const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&raw);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) rs[j] = __bfloat162float(hb[j]);
-              }
-#pragma unroll
-              for (int j = 0; j < 8; ++j) v[j] = rs[j] + gate_s[col + j] * v[j];
-            }
-            if constexpr (EPI == MFX_EPI_SWIGLU) {
-              float o[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) o[j] = silu(v[2 * j]) * v[2 * j + 1];
-              if constexpr (sizeof(OUT) == 4) {
-                *reinterpret_cast<float4*>(yrow + col / 2) = make_float4(o[0], o[1], o[2], o[3]);
-              } else {
-                __nv_bfloat162 h[2];
-                h[0] = __floats2bfloat162_rn(o[0], o[1]);
-                h[1] = __floats2bfloat162_rn(o[2], o[3]);
-                *reinterpret_cast<uint2*>(yrow + col / 2) = *reinterpret_cast<uint2*>(h);
-              }
-            } else if constexpr (sizeof(OUT) == 4) {
-              if constexpr (EPI == MFX_EPI_GATE_RESIDUAL) {
-                __stcs(reinterpret_cast<float4*>(yrow + col), make_float4(v[0], v[1], v[2], v[3]));
-                __stcs(reinterpret_cast<float4*>(yrow + col + 4), make_float4(v[4], v[5], v[6], v[7]));
-              } else {
-                *reinterpret_cast<float4*>(yrow + col) = make_float4(v[0], v[1], v[2], v[3]);
-                *reinterpret_cast<float4*>(yrow + col + 4) = make_float4(v[4], v[5], v[6], v[7]);
-              }
-            } else {
-              __nv_bfloat162 h[4];
-#pragma unroll
-              for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-              *reinterpret_cast<uint4*>(yrow + col) = *reinterpret_cast<uint4*>(h);
-            }
-          }
-        }
+      } else {
+        write_row<OUT, EPI>(t_addr, 0, BN, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
       }
       tc_fence_before();
       __syncwarp();
@@ -644,7 +579,8 @@ MFX_DEFINE_STATUS_READER(read_status)
 
 template <int BITS, uint32_t WF, int ST, int SD, typename OUT, int EPI, bool EXT>
 int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tsb, const CUtensorMap& tt,
-               const CUtensorMap& tlb, const Params& p, int grid, cudaStream_t st) {
+               const CUtensorMap& tlb, Params p, int grid, cudaStream_t st) {
+  p.wide = wide_rows<OUT, EPI>(p.y, p.y_row_stride, p.y_batch_stride, p.residual, p.res_row_stride, p.res_batch_stride);
   using L = Smem<BITS, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * (BITS == 4 ? 128 : 64) : 0>;
   // eight dequantizer warps keep up with the tensor pipe for both widths (8-bit codes go through packed float32
   // arithmetic, five instructions per pair) and draw less power than sixteen
