@@ -30,6 +30,7 @@
 #include "host_util.cuh"
 #include "ptx.cuh"
 #include "qmm_common.cuh"
+#include "qmm_dense.cuh"
 #include "qmm_epilogue.cuh"
 #include "qmm_t.cuh"
 #include "qmv.cuh"
@@ -764,7 +765,8 @@ static bool tmem_operand_kernel() {
   return on;
 }
 
-int run(const mfx_qlinear_args& a, cudaStream_t st) {
+// scratch: optional, see mfx_qlinear_ex_scratch
+int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStream_t st) {
   const bool scatter = a.epilogue == MFX_EPI_PEER_SCATTER;
   if (!a.x || (!a.y && !scatter)) return MFX_ERR_NULL;
   if (!valid_bits(a.bits) || a.group_size != 64) return MFX_ERR_UNSUPPORTED_BITS;
@@ -824,6 +826,9 @@ int run(const mfx_qlinear_args& a, cudaStream_t st) {
   }
   if (!low_rank && !scatter && qmv::eligible(a)) return qmv::run(a, prepared, codes_bytes_padded(a.N, a.K, a.bits), st);
   if (!low_rank && tmem_operand_kernel()) return qmmt::run(a, prepared, codes_bytes_padded(a.N, a.K, a.bits), st);
+  if (!scatter && scratch && scratch_bytes >= qmmd::dense_bytes(a.N, a.K) &&
+      (reinterpret_cast<uintptr_t>(scratch) & 255u) == 0)
+    return qmmd::run(a, prepared, codes_bytes_padded(a.N, a.K, a.bits), scratch, st);
   const void* codes = prepared;
   const void* sb_packed = static_cast<const uint8_t*>(prepared) + codes_bytes_padded(a.N, a.K, a.bits);
 
@@ -972,7 +977,17 @@ extern "C" {
 
 int mfx_qlinear_ex(const mfx_qlinear_args* args, void* stream) {
   if (!args) return MFX_ERR_NULL;
-  return mfx::qmm::run(*args, static_cast<cudaStream_t>(stream));
+  return mfx::qmm::run(*args, nullptr, 0, static_cast<cudaStream_t>(stream));
+}
+
+int mfx_qlinear_ex_scratch(const mfx_qlinear_args* args, void* scratch, size_t scratch_bytes, void* stream) {
+  if (!args) return MFX_ERR_NULL;
+  return mfx::qmm::run(*args, scratch, scratch_bytes, static_cast<cudaStream_t>(stream));
+}
+
+size_t mfx_qlinear_scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
+  if (rows <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || !mfx::valid_bits(bits)) return 0;
+  return mfx::qmmd::scratch_bytes(rows, N, K, bits);
 }
 
 size_t mfx_qlinear_prepared_bytes(int64_t N, int64_t K, int bits, int group_size) {

@@ -1,4 +1,4 @@
-// Epilogue of the tensor-core matmul kernel (qmm.cu): one accumulator row per thread, tensor memory
+// Epilogue of the tensor-core matmul kernels (qmm.cu, qmm_dense.cu): one accumulator row per thread, tensor memory
 // -> bias / activation / gated residual -> global memory.
 #pragma once
 #include "qmm_common.cuh"

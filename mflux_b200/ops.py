@@ -258,15 +258,18 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
             raise ValueError("lora_t must be [.., rows, ld] like x and lora_b a dense [N, ld]")
         a.lora_t, a.lora_t_row_stride, a.lora_t_batch_stride = tv.data_ptr(), t_rs, t_bs
         a.lora_b, a.lora_ld, a.lora_r = lora_b.data_ptr(), ld, int(lora_r)
+    need = lib.mfx_qlinear_scratch_bytes(rows * batch, n, k, bits)
+    # room for the decoded weight; freed to this stream's pool on return, so reused only behind this call's kernels
+    scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
     if TRACE is not None:
         _trace_begin()
-    rc = lib.mfx_qlinear_ex(byref(a), _stream())
+    rc = lib.mfx_qlinear_ex_scratch(byref(a), _ptr(scratch), need, _stream())
     _lib.check(rc, "mfx_qlinear_ex")
     if TRACE is not None:
         m = rows * batch
         _trace_end("qlinear", 2.0 * m * n * k, n * k * bits / 8 + 4.0 * n * (k // group_size) + 2.0 * m * k
                    + ov.element_size() * m * n_out)
-    LAUNCHES[0] += 1 if prepared is not None else 3
+    LAUNCHES[0] += (1 if prepared is not None else 3) + (1 if need else 0)
     return ret
 
 
