@@ -4,7 +4,7 @@
 //   * it reads the same prepared weight blob (codes with the nibble / byte order that gives two neighbouring
 //     values per mask, scale|bias pairs transposed to [group][N]);
 //   * a warp owns R groups of 8 weight rows and every eighth 128-wide slice of K; a lane loads 16 bytes of codes
-//     per group and slice (32 or 16 consecutive k of one row), several slices ahead of their use;
+//     per group and slice (32 or 16 consecutive k of one row) and the group's pair, one slice ahead of their use;
 //   * the 16 x 8 x 16 products run on mma.sync (bf16 in, f32 out) with the activation rows as A. A lane feeds the
 //     k-slots of a step with its own four consecutive k, and reads the same four k of x for A: a dot product does
 //     not care about the order of its terms, so no shuffle is needed to match the instruction's k layout;
@@ -114,28 +114,37 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
   const __nv_bfloat16* x_lo = p.x + static_cast<int64_t>(g) * p.x_row_stride;
   const __nv_bfloat16* x_hi = p.x + static_cast<int64_t>(g + 8) * p.x_row_stride;
 
-  // codes of the R rows for one slice (16 bytes each); slices are loaded one iteration ahead of their use
-  auto load_codes = [&](int s, uint4 (&wv)[R]) {
+  // codes (16 bytes) and (scale, bias) pairs of the R rows for one slice, loaded one iteration ahead of their use: a
+  // load at its point of use exposes a trip to HBM per slice. With only the codes ahead, M 1, 4 bits: N 3072, K 15360
+  // 21.6 us, N 18432, K 3072 16.7 us; with the pairs too 16.3 and 15.5 us. Two or three slices ahead need 64 to 117
+  // registers and lose more in resident blocks than they gain (17.9 and 18.9 us on the second shape).
+  auto load_slice = [&](int s, uint4 (&wv)[R], uint32_t (&pv)[R]) {
     const int k0 = s * SLICE + t * KPL;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int n = n_base + 8 * r + g;
-      wv[r] = (s < slices && k0 < p.K && n < p.N)
-                  ? __ldg(reinterpret_cast<const uint4*>(p.codes + static_cast<int64_t>(n) * words_per_row +
-                                                         k0 * BITS / 32))
-                  : make_uint4(0, 0, 0, 0);
+      const bool live = s < slices && k0 < p.K && n < p.N;
+      wv[r] = live ? __ldg(reinterpret_cast<const uint4*>(p.codes + static_cast<int64_t>(n) * words_per_row +
+                                                          k0 * BITS / 32))
+                   : make_uint4(0, 0, 0, 0);
+      pv[r] = live ? __ldg(p.sb + static_cast<int64_t>(k0 >> 6) * p.N + n) : 0u;
     }
   };
   uint4 wnext[R];
-  load_codes(warp, wnext);
+  uint32_t pnext[R];
+  load_slice(warp, wnext, pnext);
   for (int s = warp; s < slices; s += WARPS) {
     const int k0 = s * SLICE + t * KPL;      // first k of this lane in the slice
     const bool live = k0 < p.K;              // ragged last slice (K is a multiple of 64, a 4-bit slice is 128):
                                              // dead lanes feed zeros, every lane still takes part in the mma
     uint4 wv[R];
+    uint32_t pv[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) wv[r] = wnext[r];
-    load_codes(s + WARPS, wnext);
+    for (int r = 0; r < R; ++r) {
+      wv[r] = wnext[r];
+      pv[r] = pnext[r];
+    }
+    load_slice(s + WARPS, wnext, pnext);
     // activations of rows g and g + 8 for the same k (KPL values = KPL / 8 16-byte loads each)
     uint32_t xa[KPL / 2], xb[KPL / 2];
 #pragma unroll
@@ -145,11 +154,9 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
       xa[4 * i] = a.x; xa[4 * i + 1] = a.y; xa[4 * i + 2] = a.z; xa[4 * i + 3] = a.w;
       xb[4 * i] = b.x; xb[4 * i + 1] = b.y; xb[4 * i + 2] = b.z; xb[4 * i + 3] = b.w;
     }
-    const int group = k0 >> 6;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int n = n_base + 8 * r + g;
-      const uint32_t sbv = (live && n < p.N) ? __ldg(p.sb + static_cast<int64_t>(group) * p.N + n) : 0u;
+      const uint32_t sbv = pv[r];
       const uint32_t scale2 = __byte_perm(sbv, sbv, 0x1010), bias2 = __byte_perm(sbv, sbv, 0x3232);
       uint64_t sc2 = 0, bi2 = 0;
       if (BITS == 8) {   // the same scale and bias as float32 pairs
