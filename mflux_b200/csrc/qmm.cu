@@ -15,9 +15,10 @@
 //   warp 1      allocates TMEM; in the leader CTA issues tcgen05.mma.cta_group::2 (M=256, N=256, K=16)
 //   warps 4-7   epilogue: tcgen05.ld -> bias / activation / gated residual -> global, overlapped with the
 //               main loop of the next tile (two 256-column TMEM accumulators)
-//   warps 8-15  dequantizers: codes (smem) -> bf16 -> B operand tile in the swizzled K-major layout. 4-bit codes
-//               by the bf16 exponent-magic (128 + code) and one bf16 fma with the group's scale and bias; 8-bit
-//               codes by the float32 magic (2^23 + code) and packed f32x2 add + fma, rounded to bf16 at the end
+//   warps 8-    dequantizers, one or two teams of eight that take the stages in turn: codes (smem) -> bf16 -> B operand
+//               tile in the swizzled K-major layout. 4-bit codes by the bf16 exponent-magic (128 + code) and one bf16
+//               fma with the group's scale and bias; 8-bit codes by the float32 magic (2^23 + code) and packed f32x2
+//               add + fma, rounded to bf16 at the end
 // Barriers that both CTAs feed live in the leader; MMA completion is multicast to both CTAs. All mbarrier
 // waits are bounded.
 #include <cuda_bf16.h>
@@ -115,8 +116,9 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& tm, 
 }
 
 // EXT compiles the low-rank extension stages in; without it the loops below are the plain quantized matmul.
-template <int BITS, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, bool EXT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((FIXED_WARPS + NUM_DQ_WARPS) * 32, 1)
+// TEAMS x NUM_DQ_WARPS dequantizer warps; a team takes every TEAMS-th stage.
+template <int BITS, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, int TEAMS, bool EXT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((FIXED_WARPS + TEAMS * NUM_DQ_WARPS) * 32, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
            const __grid_constant__ CUtensorMap tmap_sb, const __grid_constant__ CUtensorMap tmap_t,
            const __grid_constant__ CUtensorMap tmap_lb, const Params p) {
@@ -300,7 +302,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
             break;
           }
           tc_fence_after();
-          if (lane == 0) {
+          // elect.sync, not `lane == 0`: the branch then is uniform to the compiler and the products' operands stay in
+          // uniform registers (8 bits, M 1613, N 3840, K 3840: 57.0 -> 52.9 us)
+          if (elect_one()) {
             if (!EXT || s < num_st) {
 #pragma unroll
               for (int g = 0; g < GPS; ++g) {
@@ -348,7 +352,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     // per weight row (16 warps would give eight per group and half a row per thread).
     constexpr int WPG = NUM_DQ_WARPS / GPS;        // warps per group
     constexpr int SPLIT = WPG / 4;                 // threads per weight row: 1 or 2
-    const int dq = warp - FIRST_DQ_WARP;
+    const int dq = (warp - FIRST_DQ_WARP) % NUM_DQ_WARPS;
+    const int team = (warp - FIRST_DQ_WARP) / NUM_DQ_WARPS;
+    int turn = 0;                                  // team of the next stage
     const int grp = dq / WPG;
     const int row = ((dq % WPG) / SPLIT) * 32 + lane;  // row of this CTA's 128-row weight tile
     const int part = dq % SPLIT;                       // which part of the row's 64 k-values
@@ -376,6 +382,21 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     bool ok = true;
     for (int tile = pair; tile < p.total_tiles && ok; tile += num_pairs) {
       for (int s = 0; s < num_all; ++s) {
+        if (TEAMS > 1) {
+          const bool mine = turn == team;
+          if (++turn == TEAMS) turn = 0;
+          if (!mine) {
+            if (++st == ST) {
+              st = 0;
+              ph_t ^= 1u;
+            }
+            if (++sd == SD) {
+              sd = 0;
+              ph_d ^= 1u;
+            }
+            continue;
+          }
+        }
         if (!mbar_wait(d_empty(sd), ph_d ^ 1u, DEV_TIMEOUT_DQ_EMPTY) ||
             !mbar_wait(w_full(st), ph_t, DEV_TIMEOUT_TMA_FULL)) {
           ok = false;
@@ -583,11 +604,15 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
                const CUtensorMap& tlb, Params p, int grid, cudaStream_t st) {
   p.wide = wide_rows<OUT, EPI>(p.y, p.y_row_stride, p.y_batch_stride, p.residual, p.res_row_stride, p.res_batch_stride);
   using L = Smem<BITS, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * (BITS == 4 ? 128 : 64) : 0>;
-  // eight dequantizer warps keep up with the tensor pipe for both widths (8-bit codes go through packed float32
-  // arithmetic, five instructions per pair) and draw less power than sixteen
+  // A stage is dequantized by eight warps, one thread per row and group. One team's time per stage (barrier waits, shared
+  // memory latency, arithmetic, proxy fence, arrival) is longer than the stage's products, so with three B stages two
+  // teams take turns. 4 bits, M 4096, N 12288, K 3072, GELU: 264 -> 227 us; M 4608, N 3072, K 15360: 322 -> 297 us; M
+  // 512, N 3072, K 12288: 70 -> 62 us. Eight-bit tiles leave room for two B stages, where a second team has nowhere to
+  // write ahead and costs 2-3 % (M 1613, N 20480, K 3840: 212 -> 218 us).
   constexpr int NDQ = 8;
-  constexpr int NUM_THREADS = (FIXED_WARPS + NDQ) * 32;
-  auto kern = qmm_kernel<BITS, WF, ST, SD, OUT, EPI, NDQ, EXT>;
+  constexpr int TEAMS = SD > 2 ? 2 : 1;
+  constexpr int NUM_THREADS = (FIXED_WARPS + TEAMS * NDQ) * 32;
+  auto kern = qmm_kernel<BITS, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EXT>;
   static SmemConfigured configured;  // one record per instantiation of the kernel
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::DYN_BYTES, configured)) return rc;
   kern<<<grid, NUM_THREADS, L::DYN_BYTES, st>>>(tx, tw, tsb, tt, tlb, p);
