@@ -497,19 +497,21 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
           gate_s[c] = (n < p.N) ? load_scalar(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
       }
       named_bar_sync(1, 128);
-      if (!mbar_wait_sleep(acc_full(a), aph, DEV_TIMEOUT_ACC_FULL)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
       const bool row_ok = r < p.rows;
       // SwiGLU writes one value per (gate, up) column pair: output column n/2
       OUT* yrow = static_cast<OUT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride +
                   (EPI == MFX_EPI_SWIGLU ? n0 / 2 : n0);
       const OUT* rrow = nullptr;
-      if (EPI == MFX_EPI_GATE_RESIDUAL)
+      if (EPI == MFX_EPI_GATE_RESIDUAL) {
         rrow = static_cast<const OUT*>(p.residual) + b * p.res_batch_stride +
                static_cast<int64_t>(r) * p.res_row_stride + n0;
+        if (row_ok && p.K <= PREFETCH_K) prefetch_row(rrow, 0, BN, p.N - n0);
+      }
+      if (!mbar_wait_sleep(acc_full(a), aph, DEV_TIMEOUT_ACC_FULL)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + a * BN;
       if constexpr (EPI == MFX_EPI_PEER_SCATTER) {
         // Partial rows go to slot [sc_rank] of the rank that owns each row, over NVLink, where only stores of whole

@@ -14,11 +14,12 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t (&v)[8]) {
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
+// Not volatile: a thread reads each residual element once, before it writes that element, so the loads of a chunk may
+// all be issued ahead of its stores.
 __device__ __forceinline__ void ld_global_32(const void* p, uint32_t (&v)[8]) {
-  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "l"(p)
-               : "memory");
+               : "l"(p));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -59,6 +60,17 @@ __device__ __forceinline__ void add_residual8(const OUT* rrow, const float* gate
   for (int j = 0; j < 8; ++j) v[j] = rs[j] + gate_s[j] * v[j];
 }
 
+// Asks for columns [c0, c1) of a residual row: called before the wait for the accumulator, so that the row's trip from
+// HBM overlaps the main loop. With short K the epilogue is what a tile waits for (M 14290, N 3072, K 3072: 285 -> 278 us
+// in one launch, 262 -> 253 us in two); with K of 12288 it hides behind the main loop anyway, and lines asked for
+// that early cost 1-2 %.
+constexpr int PREFETCH_K = 4096;
+template <typename OUT>
+__device__ __forceinline__ void prefetch_row(const OUT* rrow, int c0, int c1, int n_left) {
+  for (int c = c0; c < min(c1, n_left); c += 128 / static_cast<int>(sizeof(OUT)))
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(rrow + c));
+}
+
 // 32-byte accesses need the row's addresses on that boundary; the entry point only promises 16.
 template <typename OUT, int EPI>
 inline bool wide_rows(const void* y, int64_t y_row_stride, int64_t y_batch_stride, const void* residual,
@@ -85,6 +97,11 @@ __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n
     if (!row_ok) continue;
     if (wide && c + 32 <= n_left) {
       uint32_t o[8];
+      uint32_t rs[4][8];   // the chunk's residual: four loads in flight instead of one at a time
+      if constexpr (EPI == MFX_EPI_GATE_RESIDUAL && sizeof(OUT) == 4) {
+#pragma unroll
+        for (int g8 = 0; g8 < 4; ++g8) ld_global_32(rrow + c + g8 * 8, rs[g8]);
+      }
 #pragma unroll
       for (int g8 = 0; g8 < 4; ++g8) {
         const int col = c + g8 * 8;
@@ -105,10 +122,8 @@ __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n
           }
         } else if constexpr (sizeof(OUT) == 4) {
           if constexpr (EPI == MFX_EPI_GATE_RESIDUAL) {
-            uint32_t rs[8];
-            ld_global_32(rrow + col, rs);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(rs[j]) + gate_s[col + j] * v[j];
+            for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(rs[g8][j]) + gate_s[col + j] * v[j];
           }
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] = __float_as_uint(v[j]);
