@@ -150,8 +150,9 @@ class QuantizedLinear(Module):
 
     def prepared(self) -> torch.Tensor:
         """Kernel-side form of the weight, built on first use and rebuilt if the tensors were replaced."""
-        key = (self.weight.data_ptr(), self.weight._version, self.scales.data_ptr(), self.scales._version,
-               self.biases.data_ptr(), self.biases._version)
+        p = self._parameters   # not through Module.__getattr__: this runs on every call
+        w, s, b = p["weight"], p["scales"], p["biases"]
+        key = (w.data_ptr(), w._version, s.data_ptr(), s._version, b.data_ptr(), b._version)
         if self._prepared is None or self._prepared[0] != key:
             blob = ops.prepare_qlinear(self.weight.data, self.scales.data, self.biases.data, self.bits,
                                        self.group_size)
@@ -161,8 +162,8 @@ class QuantizedLinear(Module):
     def forward(self, x: torch.Tensor, *, epilogue: str | None = None, gate: torch.Tensor | None = None,
                 residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
-        return ops.qlinear(x, self.weight.data, self.scales.data, self.biases.data,
-                           None if self.bias is None else self.bias.data, bits=self.bits,
+        p = self._parameters
+        return ops.qlinear(x, p["weight"], p["scales"], p["biases"], p["bias"], bits=self.bits,
                            group_size=self.group_size, epilogue=epilogue, gate=gate, residual=residual, out=out,
                            out_dtype=out_dtype, prepared=self.prepared())
 

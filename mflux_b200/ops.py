@@ -8,6 +8,7 @@ from __future__ import annotations
 
 from ctypes import byref, c_int, c_void_p
 from ctypes import pointer as ctypes_pointer
+from functools import lru_cache
 
 import torch
 
@@ -58,12 +59,25 @@ def _cuda(t: torch.Tensor, name: str) -> torch.Tensor:
     return t
 
 
-def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+# The host's share of a call is what a call of a few rows costs (23 us of 24 for a 2-row modulation linear before these
+# shortcuts): the raw stream handle without a Stream object, plain integers for pointer arguments, and the library's
+# pure size rules remembered by their integer arguments.
+def _stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
-def _ptr(t: torch.Tensor | None) -> c_void_p:
-    return c_void_p(0 if t is None else t.data_ptr())
+def _ptr(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
+@lru_cache(maxsize=4096)
+def _prepared_bytes(n: int, k: int, bits: int, group_size: int) -> int:
+    return _lib.load().mfx_qlinear_prepared_bytes(n, k, bits, group_size)
+
+
+@lru_cache(maxsize=4096)
+def _scratch_bytes(rows: int, n: int, k: int, bits: int) -> int:
+    return _lib.load().mfx_qlinear_scratch_bytes(rows, n, k, bits)
 
 
 def poll_device_status() -> int:
@@ -141,13 +155,16 @@ def _rows_view(t: torch.Tensor, name: str):
     """(tensor, rows, batch, row_stride, batch_stride) of a [..., rows, cols] tensor whose last dim is dense."""
     if t.dim() < 2:
         raise ValueError(f"{name} must have at least 2 dims")
-    if t.stride(-1) != 1:
+    st = t.stride()
+    if st[-1] != 1:
         t = t.contiguous()
-    if t.dim() == 2:
-        return t, t.shape[0], 1, t.stride(0), 0
-    if t.dim() > 3:
+        st = t.stride()
+    if len(st) == 2:
+        return t, t.size(0), 1, st[0], 0
+    if len(st) > 3:
         t = t.reshape(-1, t.shape[-2], t.shape[-1])
-    return t, t.shape[1], t.shape[0], t.stride(1), t.stride(0)
+        st = t.stride()
+    return t, t.size(1), t.size(0), st[1], st[0]
 
 
 def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: torch.Tensor,
@@ -180,15 +197,15 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
     if x.dim() == 1:
         x = x.unsqueeze(0)
     xv, rows, batch, x_rs, x_bs = _rows_view(x, "x")
-    k = xv.shape[-1]
-    n = wq.shape[0]
-    if wq.shape[1] * 32 // bits != k:
-        raise ValueError(f"x has K={k} but the packed weight encodes K={wq.shape[1] * 32 // bits}")
+    k = xv.size(-1)
+    n, words = wq.shape
+    if words * 32 // bits != k:
+        raise ValueError(f"x has K={k} but the packed weight encodes K={words * 32 // bits}")
     if prepared is None:
         wq, scales, biases = wq.contiguous(), scales.contiguous(), biases.contiguous()
-        workspace = torch.empty(lib.mfx_qlinear_prepared_bytes(n, k, bits, group_size), dtype=torch.uint8,
-                                device=x.device)
-    n_out = n // 2 if _EPI[epilogue] == EPI_SWIGLU else n
+        workspace = torch.empty(_prepared_bytes(n, k, bits, group_size), dtype=torch.uint8, device=x.device)
+    epi = _EPI[epilogue]
+    n_out = n // 2 if epi == EPI_SWIGLU else n
     if scatter is not None:
         a = QLinearArgs()
         a.x, a.x_row_stride, a.x_batch_stride = xv.data_ptr(), x_rs, x_bs
@@ -210,13 +227,13 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
         return None
     if out is None:
         od = out_dtype or (residual.dtype if residual is not None else torch.bfloat16)
-        out = torch.empty((*xv.shape[:-1], n_out), dtype=od, device=x.device)
-        ret = out.reshape(*lead, n_out)
+        ret = ov = torch.empty((*lead, n_out), dtype=od, device=x.device)   # dense: rows follow one another
+        o_rs, o_bs = n_out, rows * n_out if batch > 1 or xv.dim() > 2 else 0
     else:
         ret = out
-    ov, o_rows, o_batch, o_rs, o_bs = _rows_view(out, "out")
-    if ov.data_ptr() != out.data_ptr() or (o_rows, o_batch) != (rows, batch) or ov.shape[-1] != n_out:
-        raise ValueError("out must be a [.., rows, N] view with a dense last dim matching x")
+        ov, o_rows, o_batch, o_rs, o_bs = _rows_view(out, "out")
+        if ov.data_ptr() != out.data_ptr() or (o_rows, o_batch) != (rows, batch) or ov.size(-1) != n_out:
+            raise ValueError("out must be a [.., rows, N] view with a dense last dim matching x")
     a = QLinearArgs()
     a.x, a.x_row_stride, a.x_batch_stride = xv.data_ptr(), x_rs, x_bs
     a.rows, a.batch, a.K, a.N = rows, batch, k, n
@@ -225,14 +242,14 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
         a.wq, a.scales, a.biases, a.sb_dtype = wq.data_ptr(), scales.data_ptr(), biases.data_ptr(), _dt(scales)
         a.workspace, a.workspace_bytes = workspace.data_ptr(), workspace.numel()
     else:
-        if prepared.dtype != torch.uint8 or prepared.numel() != lib.mfx_qlinear_prepared_bytes(n, k, bits, group_size):
+        if prepared.dtype != torch.uint8 or prepared.numel() != _prepared_bytes(n, k, bits, group_size):
             raise ValueError("prepared must be the blob prepare_qlinear returned for this weight")
         a.prepared = prepared.data_ptr()
     if bias is not None:
         bias = bias.contiguous()
         a.bias, a.bias_dtype = bias.data_ptr(), _dt(bias)
-    a.epilogue = _EPI[epilogue]
-    if a.epilogue == EPI_GATE_RESIDUAL:
+    a.epilogue = epi
+    if epi == EPI_GATE_RESIDUAL:
         if gate is None or residual is None:
             raise ValueError("gate_residual needs gate and residual")
         gate = gate.reshape(-1, n) if gate.stride(-1) == 1 else gate.reshape(-1, n).contiguous()
@@ -258,7 +275,7 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
             raise ValueError("lora_t must be [.., rows, ld] like x and lora_b a dense [N, ld]")
         a.lora_t, a.lora_t_row_stride, a.lora_t_batch_stride = tv.data_ptr(), t_rs, t_bs
         a.lora_b, a.lora_ld, a.lora_r = lora_b.data_ptr(), ld, int(lora_r)
-    need = lib.mfx_qlinear_scratch_bytes(rows * batch, n, k, bits)
+    need = _scratch_bytes(rows * batch, n, k, bits)
     # room for the decoded weight; freed to this stream's pool on return, so reused only behind this call's kernels
     scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
     if TRACE is not None:

@@ -11,13 +11,12 @@ pytestmark = pytest.mark.gpu
 
 def _both(monkeypatch, call, n, k):
     """The same call in the two-launch and in the one-launch form, whatever the rule says for its size."""
-    from mflux_b200 import _lib
+    from mflux_b200 import ops
 
-    lib = _lib.load()
     outs = []
     for need in (2 * n * k, 0):
         with monkeypatch.context() as m:
-            m.setattr(lib, "mfx_qlinear_scratch_bytes", lambda *a, need=need: need)
+            m.setattr(ops, "_scratch_bytes", lambda *a, need=need: need)
             outs.append(call())
     torch.cuda.synchronize()
     return outs
@@ -116,7 +115,7 @@ def test_short_or_misaligned_scratch_is_not_used(lib_built):
         assert bool((scratch[:need] == 0x5A).all()) != used and (scratch[need:] == 0x5A).all()
 
 
-@pytest.mark.parametrize("bits,rows", [(4, 4608), (8, 2048)])
+@pytest.mark.parametrize("bits,rows", [(4, 8192), (8, 2560)])
 def test_rule_and_call_through_it(lib_built, bits, rows):
     """The rule asks for scratch on a wide layer with many rows and not below its limits; a call that it sends through
     the two launches, prepared on the fly."""
