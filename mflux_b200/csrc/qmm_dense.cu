@@ -3,8 +3,8 @@
 // for every 256 activation rows; beside the tensor cores that costs shared-memory bandwidth (1330 cycles of it per
 // 1024 cycles of products) and, at the power limit where long steps run, energy. The decoded values are the same
 // bf16 values the one-launch kernel feeds its tensor cores, and the products run in the same order of K.
-// Measured, looped at the power limit, decode included, one launch -> two: 8 bits, M 8426, N 20480, K 3840, SwiGLU:
-// 1187 -> 1016 us; 4 bits, M 73728, N 12288, K 3072: 4695 -> 4372 us (1273 TFLOP/s); M 4608: 293.5 -> 282 us.
+// Measured, looped at the power limit, decode included, one launch -> two: 8 bits, M 8426, N 3840, K 10240: 591 -> 545 us;
+// 4 bits, M 14290, N 3072, K 3072, gated residual: 278 -> 253 us; M 73728, N 9216, K 3072: 3194 -> 3110 us (1342 TFLOP/s).
 //
 // dense_kernel: persistent, one CTA pair (cluster of 2, tcgen05 cta_group::2) per 256 x 256 output tile. Per CTA:
 //   warp 0      TMA producer: the 128 activation rows and 128 weight rows of its half of the tile, 64 k per stage,
@@ -216,18 +216,21 @@ dense_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
       if (EPI == MFX_EPI_GATE_RESIDUAL)
         gate_s[et] = (n < p.N) ? load_scalar(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
       named_bar_sync(1, EPI_WARPS * 32);
-      if (!mbar_wait_sleep(acc_full(a), (it >> 1) & 1, DEV_TIMEOUT_ACC_FULL)) break;
-      tc_fence_after();
+      const bool row_ok = r < p.rows;
       // SwiGLU writes one value per (gate, up) column pair: output column n/2
       OUT* yrow = static_cast<OUT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride +
                   (EPI == MFX_EPI_SWIGLU ? n0 / 2 : n0);
+      const int c0 = half * (BN / 2), c1 = c0 + BN / 2;
       const OUT* rrow = nullptr;
-      if (EPI == MFX_EPI_GATE_RESIDUAL)
+      if (EPI == MFX_EPI_GATE_RESIDUAL) {
         rrow = static_cast<const OUT*>(p.residual) + b * p.res_batch_stride +
                static_cast<int64_t>(r) * p.res_row_stride + n0;
+        if (row_ok && p.K <= qmm::PREFETCH_K) qmm::prefetch_row(rrow, c0, c1, p.N - n0);
+      }
+      if (!mbar_wait_sleep(acc_full(a), (it >> 1) & 1, DEV_TIMEOUT_ACC_FULL)) break;
+      tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + a * BN;
-      qmm::write_row<OUT, EPI>(t_addr, half * (BN / 2), (half + 1) * (BN / 2), p.N - n0, r < p.rows, p.wide, yrow, rrow,
-                               bias_s, gate_s);
+      qmm::write_row<OUT, EPI>(t_addr, c0, c1, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(acc_empty(a));
@@ -333,17 +336,19 @@ static int64_t num_bands(int64_t N, int64_t row_bytes, int64_t limit) {
 }
 
 // Where the two launches win. The decode costs 2.6 (4 bits) or 3.1 bytes of HBM traffic per weight whatever the row
-// count, the contraction then gains 7 % (4 bits) or 14 % (8 bits) over the one-launch kernel: even at 3600 and 1500
-// rows. The second launch costs 2-3 us, which a call of less than 1e11 (5e10) operations does not earn back. And the
-// bf16 weight needs more passes over the activations than the packed one where it does not fit a band; with few output
-// columns those reads cost more than the decoding saved (M 73728, N 3072, K 12288: 5149 against 4996 us).
+// count. Measured gains with it included, looped at the power limit:
+//   8 bits  even at 2200 rows, 3-5 % at 3000, 8-15 % at 8400 (N 3840 to 20480);
+//   4 bits  3 % at 3072 rows, 5-8 % from 4600 on where the bf16 weight fits one band (N 3072, K 3072); where it needs a
+//           second pass over the activations that the packed weight does not, even at 6100 to 8200 rows and 1-3 % from
+//           there on if that pass feeds many output columns (N 9216, 12288), a loss of 3-5 % if it feeds few (N 3072, K
+//           12288; N 3840, K 10240) or if two passes come on top (N 20480, K 3840).
+// The second launch costs 2-3 us, which a call of less than 5e10 operations does not earn back.
 size_t scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
   const int kb = kernel_bits(bits);
   const int64_t extra = num_bands(N, 2 * K, BAND_BYTES) - num_bands(N, K * kb / 8 + K / 16, 32ll << 20);
-  if (extra > 0 && N < 6144 * extra) return 0;
-  if (rows < (kb == 4 ? 3584 : 1536)) return 0;
-  if (2.0 * static_cast<double>(rows) * static_cast<double>(N) * static_cast<double>(K) < (kb == 4 ? 1e11 : 5e10))
-    return 0;
+  if (extra > 1 || (extra == 1 && N < 8192)) return 0;
+  if (rows < (kb == 8 ? 2560 : extra > 0 ? 8192 : 3072)) return 0;
+  if (2.0 * static_cast<double>(rows) * static_cast<double>(N) * static_cast<double>(K) < 5e10) return 0;
   return dense_bytes(N, K);
 }
 
