@@ -6,7 +6,7 @@
 // bits [j*bits, (j+1)*bits) of the row's bit stream, which for 4 and 8 bits is "8 / 4 codes per uint32" and for
 // 3, 5 and 6 bits (the other widths the reference's CLI offers, src/mflux/cli/defaults/defaults.py:63) lets
 // codes straddle byte and word boundaries (8 codes in 3 or 5 bytes, 4 codes in 3 bytes).
-// Eight lanes own one group (8 values each); min/max go through warp shuffles.
+// Four lanes own one group (16 values each); min/max go through warp shuffles.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -33,46 +33,62 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+constexpr int PER_THREAD = 16;   // values of one group a thread holds
+
 template <typename T>
-__device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
+__device__ __forceinline__ void load16(const T* p, float (&v)[16]) {
   if constexpr (sizeof(T) == 4) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p));
-    const float4 b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
-    const T* h = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(h[i]);
+    for (int i = 0; i < 4; ++i) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(p) + i);
+      v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p) + k);
+      const T* h = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[8 * k + i] = to_f32<T>(h[i]);
+    }
   }
 }
 
-// One thread: 8 consecutive values of a row; lanes 8g..8g+7 of a warp form one 64-wide group.
+// The quantizer's definition of a code: the correctly rounded quotient, rounded to even, clamped.
+__device__ __forceinline__ float exact_code(float d, float scale, float n_bins) {
+  float q = rintf(__fdiv_rn(d, scale));
+  if (!(fabsf(q) <= 3.0e38f)) q = 0.0f;  // constant group with scale == 0: code 0
+  return fminf(fmaxf(q, 0.0f), n_bins);
+}
+
+// One thread: 16 consecutive values of a row; lanes 4g..4g+3 of a warp form one 64-wide group.
+// A division per value was what the kernel spent its time on. It multiplies by the reciprocal of the scale instead and
+// takes the rounded product where that must be the rounded quotient too: reciprocal, product and the quotient itself
+// are each off by at most 2^-24 of their value, together 1.8e-7 of at most n_bins + 1, so a product further than that
+// from every k + 0.5 rounds like the quotient. Threads with a value nearer to one (one in 1000 at 4 bits) divide.
 template <typename T, int BITS, int QMODE>
 __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, int64_t n_groups_total,
                                                        uint32_t* __restrict__ wq, T* __restrict__ scales,
                                                        T* __restrict__ biases) {
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t group = tid >> 3;
+  const int64_t group = tid >> 2;
   const bool active = group < n_groups_total;
   const int64_t g = active ? group : n_groups_total - 1;  // keep whole warps in the shuffles
-  const int sub = static_cast<int>(tid & 7);
-  const T* src = w + g * 64 + sub * 8;
-  float v[8];
-  load8<T>(src, v);
+  const int sub = static_cast<int>(tid & 3);
+  float v[16];
+  load16<T>(w + g * 64 + sub * 16, v);
   float mx = v[0], mn = v[0];
 #pragma unroll
-  for (int i = 1; i < 8; ++i) {
+  for (int i = 1; i < 16; ++i) {
     mx = fmaxf(mx, v[i]);
     mn = fminf(mn, v[i]);
   }
 #pragma unroll
-  for (int off = 4; off >= 1; off >>= 1) {
+  for (int off = 2; off >= 1; off >>= 1) {
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
   }
-  const float n_bins = static_cast<float>((1 << BITS) - 1);
+  constexpr float n_bins = static_cast<float>((1 << BITS) - 1);
   float scale, bias;
   if (QMODE == MFX_QMODE_MLX) {
     scale = fmaxf(__fdiv_rn(__fsub_rn(mx, mn), n_bins), 1e-7f);
@@ -90,33 +106,53 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
     scale = __fdiv_rn(__fsub_rn(mx, mn), n_bins);
     bias = mn;
   }
-  uint32_t codes[8];
+  const float mag = fabsf(scale);
+  bool divide = !(mag > 1e-30f && mag < 1e30f);   // the reciprocal has to be a normal number
+  const float inv = __frcp_rn(scale);
+  constexpr float MAGIC = 12582912.0f;            // 1.5 * 2^23: adding it rounds to even at the units place
+  float q[16];
+  float far = 0.0f;                               // largest distance of a product from its integer
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float q = rintf(__fdiv_rn(__fsub_rn(v[i], bias), scale));
-    if (!(fabsf(q) <= 3.0e38f)) q = 0.0f;  // constant group with scale == 0: code 0
-    q = fminf(fmaxf(q, 0.0f), n_bins);
-    codes[i] = static_cast<uint32_t>(q);
+  for (int i = 0; i < 16; ++i) {
+    const float r = fminf(fmaxf(__fmul_rn(__fsub_rn(v[i], bias), inv), 0.0f), n_bins);
+    q[i] = __fsub_rn(__fadd_rn(r, MAGIC), MAGIC);
+    far = fmaxf(far, fabsf(__fsub_rn(r, q[i])));
+  }
+  divide |= far > 0.5f - (n_bins + 1.0f) * 2.4e-7f;
+  if (divide) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[i] = exact_code(__fsub_rn(v[i], bias), scale, n_bins);
   }
   if (!active) return;
   if (BITS == 4) {
-    uint32_t word = 0;
+    // four codes at a time as an exact float below 2^16
+    uint32_t half[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) word |= codes[i] << (4 * i);
-    wq[g * 8 + sub] = word;
+    for (int i = 0; i < 4; ++i)
+      half[i] = static_cast<uint32_t>(fmaf(fmaf(fmaf(q[4 * i + 3], 16.0f, q[4 * i + 2]), 16.0f, q[4 * i + 1]), 16.0f,
+                                           q[4 * i]));
+    reinterpret_cast<uint2*>(wq)[g * 4 + sub] = make_uint2(half[0] | (half[1] << 16), half[2] | (half[3] << 16));
   } else if (BITS == 8) {
-    uint2 words;
-    words.x = codes[0] | (codes[1] << 8) | (codes[2] << 16) | (codes[3] << 24);
-    words.y = codes[4] | (codes[5] << 8) | (codes[6] << 16) | (codes[7] << 24);
-    reinterpret_cast<uint2*>(wq)[g * 8 + sub] = words;
+    uint32_t word[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t lo = static_cast<uint32_t>(fmaf(q[4 * i + 1], 256.0f, q[4 * i]));
+      const uint32_t hi = static_cast<uint32_t>(fmaf(q[4 * i + 3], 256.0f, q[4 * i + 2]));
+      word[i] = lo | (hi << 16);
+    }
+    reinterpret_cast<uint4*>(wq)[g * 4 + sub] = make_uint4(word[0], word[1], word[2], word[3]);
   } else {
-    // 8 codes = BITS bytes of the bit stream, starting at byte (8 * thread) * BITS / 8 of the tensor
-    unsigned long long stream = 0;
+    // 8 codes = BITS bytes of the bit stream
+    uint8_t* dst = reinterpret_cast<uint8_t*>(wq) + (g * 4 + sub) * (2 * BITS);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) stream |= static_cast<unsigned long long>(codes[i]) << (BITS * i);
-    uint8_t* dst = reinterpret_cast<uint8_t*>(wq) + (g * 8 + sub) * BITS;
+    for (int k = 0; k < 2; ++k) {
+      unsigned long long stream = 0;
 #pragma unroll
-    for (int i = 0; i < BITS; ++i) dst[i] = static_cast<uint8_t>(stream >> (8 * i));
+      for (int i = 0; i < 8; ++i)
+        stream |= static_cast<unsigned long long>(static_cast<uint32_t>(q[8 * k + i])) << (BITS * i);
+#pragma unroll
+      for (int i = 0; i < BITS; ++i) dst[BITS * k + i] = static_cast<uint8_t>(stream >> (8 * i));
+    }
   }
   if (sub == 0) {
     scales[g] = from_f32<T>(scale);
@@ -124,7 +160,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
   }
 }
 
-// One thread: 8 consecutive outputs of a row.
+// One thread: 16 consecutive outputs of a row.
 template <typename SB, typename OUT, int BITS>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restrict__ wq,
                                                          const SB* __restrict__ scales,
@@ -132,46 +168,48 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
                                                          OUT* __restrict__ out) {
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= n_chunks) return;
-  const int64_t g = tid >> 3;
+  const int64_t g = tid >> 2;
   const float s = to_f32<SB>(scales[g]);
   const float b = to_f32<SB>(biases[g]);
-  uint32_t codes[8];
+  uint32_t codes[16];
   if (BITS == 4) {
-    const uint32_t word = __ldg(wq + tid);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) codes[i] = (word >> (4 * i)) & 0xF;
-  } else if (BITS == 8) {
     const uint2 words = __ldg(reinterpret_cast<const uint2*>(wq) + tid);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      codes[i] = (words.x >> (8 * i)) & 0xFF;
-      codes[4 + i] = (words.y >> (8 * i)) & 0xFF;
+    for (int i = 0; i < 8; ++i) {
+      codes[i] = (words.x >> (4 * i)) & 0xF;
+      codes[8 + i] = (words.y >> (4 * i)) & 0xF;
     }
+  } else if (BITS == 8) {
+    const uint4 words = __ldg(reinterpret_cast<const uint4*>(wq) + tid);
+    const uint32_t w4[4] = {words.x, words.y, words.z, words.w};
+#pragma unroll
+    for (int i = 0; i < 16; ++i) codes[i] = (w4[i >> 2] >> (8 * (i & 3))) & 0xFF;
   } else {
-    const uint8_t* src = reinterpret_cast<const uint8_t*>(wq) + tid * BITS;
-    unsigned long long stream = 0;
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(wq) + tid * (2 * BITS);
 #pragma unroll
-    for (int i = 0; i < BITS; ++i) stream |= static_cast<unsigned long long>(__ldg(src + i)) << (8 * i);
+    for (int k = 0; k < 2; ++k) {
+      unsigned long long stream = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) codes[i] = static_cast<uint32_t>(stream >> (BITS * i)) & ((1u << BITS) - 1u);
+      for (int i = 0; i < BITS; ++i) stream |= static_cast<unsigned long long>(__ldg(src + BITS * k + i)) << (8 * i);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) codes[8 * k + i] = static_cast<uint32_t>(stream >> (BITS * i)) & ((1u << BITS) - 1u);
+    }
   }
-  OUT res[8];
+  __align__(16) OUT res[16];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-    res[i] = from_f32<OUT>(__fadd_rn(__fmul_rn(static_cast<float>(codes[i]), s), b));
-  OUT* dst = out + tid * 8;
-  if constexpr (sizeof(OUT) == 4) {
-    reinterpret_cast<float4*>(dst)[0] = *reinterpret_cast<float4*>(&res[0]);
-    reinterpret_cast<float4*>(dst)[1] = *reinterpret_cast<float4*>(&res[4]);
-  } else {
-    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<uint4*>(&res[0]);
+  for (int i = 0; i < 16; ++i) {
+    const float c = __uint_as_float(0x4B000000u | codes[i]) - 8388608.0f;   // the code under the exponent of 2^23
+    res[i] = from_f32<OUT>(__fadd_rn(__fmul_rn(c, s), b));
   }
+  uint4* dst = reinterpret_cast<uint4*>(out + tid * 16);
+#pragma unroll
+  for (int i = 0; i < static_cast<int>(sizeof(OUT)); ++i) dst[i] = reinterpret_cast<const uint4*>(res)[i];
 }
 
 template <typename T>
 int launch_quantize(const void* w, int64_t n_groups, int bits, int qmode, uint32_t* wq, void* scales, void* biases,
                     cudaStream_t st) {
-  const int64_t threads = n_groups * 8;
+  const int64_t threads = n_groups * (64 / PER_THREAD);
   const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
   const T* wp = static_cast<const T*>(w);
   T* sp = static_cast<T*>(scales);
@@ -260,7 +298,7 @@ int mfx_dequantize_affine(const uint32_t* wq, const void* scales, const void* bi
   if (!aligned16(wq) || !aligned16(out)) return MFX_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t n_chunks = N * K / 8;
+  const int64_t n_chunks = N * K / PER_THREAD;
   switch (sb_dtype) {
     case MFX_F32: return dispatch_dequant_out<float>(wq, scales, biases, n_chunks, bits, out, out_dtype, st);
     case MFX_BF16:
