@@ -4,15 +4,15 @@
 // group_size=64, bits) for every nn.Linear of the transformer blocks of the reference
 // (e.g. src/mflux/models/flux/model/flux_transformer/joint_attention.py:14-21, feed_forward.py:8-9).
 //
-// Two CTAs on neighbouring SMs form a pair (cluster of 2, tcgen05 cta_group::2) and share one 256 x 256
-// output tile: each CTA loads the 128 activation rows of its half (A operand) and dequantizes 128 of the 256
-// weight rows (its half of the B operand); one MMA of the pair reads both halves. Per flop that halves the
+// Two CTAs on neighbouring SMs form a pair (cluster of 2, tcgen05 cta_group::2) and share one output tile of 256 rows and
+// 256, 192 or 128 columns (tile_width): each CTA loads the 128 activation rows of its half (A operand) and dequantizes
+// half of the weight rows (its half of the B operand); one MMA of the pair reads both halves. Per flop that halves the
 // dequantization work and the weight-operand shared-memory traffic of a single-CTA 128 x 256 tile, which is
 // what bounded it. A pipeline stage carries two quantization groups (128 k-values) because the issuing thread
 // loses a few hundred cycles around every wait + commit. Persistent, warp-specialised, per CTA:
 //   warp 0      TMA producer: per stage its X tile [128 x 128 k] bf16 as two 128-byte-swizzled slabs (counted
-//               on the leader's barrier), the packed codes of its 128 weight rows and their (scale, bias) pairs
-//   warp 1      allocates TMEM; in the leader CTA issues tcgen05.mma.cta_group::2 (M=256, N=256, K=16)
+//               on the leader's barrier), the packed codes of its weight rows and their (scale, bias) pairs
+//   warp 1      allocates TMEM; in the leader CTA issues tcgen05.mma.cta_group::2 (M=256, N=tile width, K=16)
 //   warps 4-7   epilogue: tcgen05.ld -> bias / activation / gated residual -> global, overlapped with the
 //               main loop of the next tile (two 256-column TMEM accumulators)
 //   warps 8-    dequantizers, one or two teams of eight that take the stages in turn: codes (smem) -> bf16 -> B operand
@@ -40,16 +40,13 @@ namespace mfx {
 namespace qmm {
 
 constexpr int BM = 128;       // activation rows per CTA (256 per pair)
-constexpr int BN = 256;       // weight rows (output columns) per pair tile
-constexpr int BN_HALF = 128;  // weight rows each CTA dequantizes
+constexpr int BN_MAX = 256;   // weight rows (output columns) per pair tile, at most; each CTA dequantizes half (BNH)
 constexpr int BK = 64;        // one quantization group
 constexpr int GPS = 2;        // quantization groups per pipeline stage
 constexpr int FIXED_WARPS = 8;  // producer, MMA, 2 spare, 4 epilogue
 constexpr int FIRST_DQ_WARP = 8;
 constexpr int FIRST_EPI_WARP = 4;
 constexpr int X_TILE_BYTES = BM * BK * 2;        // 16 KiB per group
-constexpr int WD_TILE_BYTES = BN_HALF * BK * 2;  // 16 KiB per group
-constexpr int SB_TILE_BYTES = BN_HALF * 4;       // one bf16 (scale, bias) pair per weight row
 constexpr uint32_t TMEM_COLS = 512;
 
 struct Params {
@@ -81,9 +78,11 @@ struct Params {
 
 // ST = stages of the TMA ring, SD = stages of the dequantized-weight ring; one stage = GPS groups.
 // STG = bytes of the epilogue's staging buffer (tensor-parallel scatter only).
-template <int BITS, int ST, int SD, int STG = 0>
+template <int BITS, int BNH, int ST, int SD, int STG = 0>
 struct Smem {
-  static constexpr int WQ_TILE_BYTES = BN_HALF * BK * BITS / 8;
+  static constexpr int WQ_TILE_BYTES = BNH * BK * BITS / 8;
+  static constexpr int WD_TILE_BYTES = BNH * BK * 2;   // 16 KiB per group of a 256-wide tile
+  static constexpr int SB_TILE_BYTES = BNH * 4;        // one bf16 (scale, bias) pair per weight row
   static constexpr int X_STAGE = GPS * X_TILE_BYTES;
   static constexpr int WD_STAGE = GPS * WD_TILE_BYTES;
   static constexpr int WQ_STAGE = GPS * WQ_TILE_BYTES;
@@ -93,7 +92,7 @@ struct Smem {
   static constexpr int OFF_WQ = OFF_WD + SD * WD_STAGE;
   static constexpr int OFF_SB = OFF_WQ + ST * WQ_STAGE;
   static constexpr int OFF_VEC = OFF_SB + ST * SB_STAGE;  // bias[2][256] + gate[2][256] floats
-  static constexpr int OFF_STAGE = OFF_VEC + 4 * BN * 4;
+  static constexpr int OFF_STAGE = OFF_VEC + 4 * BN_MAX * 4;
   static constexpr int OFF_BAR = OFF_STAGE + STG;
   static constexpr int NUM_BARS = 4 * ST + 2 * SD + 4;
   static constexpr int OFF_TMEM = OFF_BAR + NUM_BARS * 8;
@@ -117,7 +116,7 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& tm, 
 
 // EXT compiles the low-rank extension stages in; without it the loops below are the plain quantized matmul.
 // TEAMS x NUM_DQ_WARPS dequantizer warps; a team takes every TEAMS-th stage.
-template <int BITS, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, int TEAMS, bool EXT>
+template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, int TEAMS, bool EXT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((FIXED_WARPS + TEAMS * NUM_DQ_WARPS) * 32, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
            const __grid_constant__ CUtensorMap tmap_sb, const __grid_constant__ CUtensorMap tmap_t,
@@ -125,7 +124,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
   // The scatter epilogue stages 32 rows x SCATTER_ROW bytes per epilogue warp to turn "thread = row" into stores
   // of whole 128-byte (64-byte for 8-bit codes, where shared memory is tighter) row segments.
   constexpr int SCATTER_ROW = BITS == 4 ? 128 : 64;
-  using L = Smem<BITS, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * SCATTER_ROW : 0>;
+  using L = Smem<BITS, BNH, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * SCATTER_ROW : 0>;
+  constexpr int BN = 2 * BNH;
+  constexpr int WD_TILE_BYTES = L::WD_TILE_BYTES, SB_TILE_BYTES = L::SB_TILE_BYTES;
   // With as many TMA stages as dequantized-weight stages the two rings advance in lockstep and one "stage
   // consumed" barrier serves both: the commit after a stage's MMAs frees its activation tile and its B tile, and
   // the stage's packed codes were read before its B tile was written, so they are free by then too. That is one
@@ -245,7 +246,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     for (int tile = pair; tile < p.total_tiles && ok; tile += num_pairs) {
       int tm, tn;
       tile_coords(p, tile, tm, tn);
-      const int n0 = tn * BN + static_cast<int>(rank) * BN_HALF;
+      const int n0 = tn * BN + static_cast<int>(rank) * BNH;
       for (int s = 0; s < num_all; ++s) {
         if (!mbar_wait(c_empty(st), ph ^ 1u, DEV_TIMEOUT_TMA_EMPTY)) {
           ok = false;
@@ -282,7 +283,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
     if (rank == 0) {
-      constexpr uint32_t IDESC = make_idesc(FMT_BF16, WF, 2 * BM, BN);  // M = 256 over the pair, N = 256
+      constexpr uint32_t IDESC = make_idesc(FMT_BF16, WF, 2 * BM, BN);  // M = 256 over the pair
       int st = 0, sd = 0;
       uint32_t ph_t = 0, ph_d = 0;
       bool ok = true;
@@ -351,12 +352,13 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     // Every warp serves one quantization group of the stage: with 8 warps four warps per group and one thread
     // per weight row (16 warps would give eight per group and half a row per thread).
     constexpr int WPG = NUM_DQ_WARPS / GPS;        // warps per group
-    constexpr int SPLIT = WPG / 4;                 // threads per weight row: 1 or 2
+    constexpr int SPLIT = WPG * 32 >= 2 * BNH ? 2 : 1;   // threads per weight row
     const int dq = (warp - FIRST_DQ_WARP) % NUM_DQ_WARPS;
     const int team = (warp - FIRST_DQ_WARP) / NUM_DQ_WARPS;
     int turn = 0;                                  // team of the next stage
     const int grp = dq / WPG;
-    const int row = ((dq % WPG) / SPLIT) * 32 + lane;  // row of this CTA's 128-row weight tile
+    const int row = ((dq % WPG) / SPLIT) * 32 + lane;  // row of this CTA's BNH-row weight tile
+    const bool has_row = WPG * 32 / SPLIT == BNH || row < BNH;   // 96 rows leave the last of a group's four warps idle
     const int part = dq % SPLIT;                       // which part of the row's 64 k-values
     constexpr int ROW_BYTES = BK * BITS / 8;           // packed bytes per row per group
     constexpr int RD_CHUNKS = ROW_BYTES / 16;          // 16-byte chunks per row: 2 (4 bits) or 4 (8 bits)
@@ -408,7 +410,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
           const uint8_t* esrc = rd_base + st * L::WQ_STAGE;
           uint8_t* edst = wr_base + sd * L::WD_STAGE;
 #pragma unroll
-          for (int h = 0; h < MY_CHUNKS; ++h) {
+          for (int h = 0; h < MY_CHUNKS && has_row; ++h) {
             const uint32_t c = static_cast<uint32_t>(part * MY_CHUNKS + h);
             *reinterpret_cast<uint4*>(edst + ((c ^ static_cast<uint32_t>(row & 7)) << 4)) =
                 *reinterpret_cast<const uint4*>(esrc + rd_off[h]);
@@ -435,7 +437,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
         const uint8_t* src = rd_base + st * L::WQ_STAGE;
         uint8_t* dst = wr_base + sd * L::WD_STAGE;
 #pragma unroll
-        for (int h = 0; h < MY_CHUNKS; ++h) {
+        for (int h = 0; h < MY_CHUNKS && has_row; ++h) {
           const uint4 pk = *reinterpret_cast<const uint4*>(src + rd_off[h]);
           if (BITS == 4) {  // 4 words x 8 codes -> 4 output chunks
             const uint32_t wds[4] = {pk.x, pk.y, pk.z, pk.w};
@@ -486,11 +488,10 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
       const int b = tm / p.tiles_m_per_sample;
       const int r = (tm % p.tiles_m_per_sample) * (2 * BM) + static_cast<int>(rank) * BM + row;
       const int n0 = tn * BN;
-      float* bias_s = vec_s + a * BN;
-      float* gate_s = vec_s + 2 * BN + a * BN;
+      float* bias_s = vec_s + a * BN_MAX;
+      float* gate_s = vec_s + (2 + a) * BN_MAX;
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int c = et + 128 * h;
+      for (int c = et; c < BN; c += 128) {
         const int n = n0 + c;
         bias_s[c] = (p.bias != nullptr && n < p.N) ? load_scalar(p.bias, p.bias_dtype, n) : 0.f;
         if (EPI == MFX_EPI_GATE_RESIDUAL)
@@ -601,11 +602,12 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
 
 MFX_DEFINE_STATUS_READER(read_status)
 
-template <int BITS, uint32_t WF, int ST, int SD, typename OUT, int EPI, bool EXT>
+template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT, int EPI, bool EXT>
 int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tsb, const CUtensorMap& tt,
                const CUtensorMap& tlb, Params p, int grid, cudaStream_t st) {
   p.wide = wide_rows<OUT, EPI>(p.y, p.y_row_stride, p.y_batch_stride, p.residual, p.res_row_stride, p.res_batch_stride);
-  using L = Smem<BITS, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * (BITS == 4 ? 128 : 64) : 0>;
+  using L = Smem<BITS, BNH, ST, SD, EPI == MFX_EPI_PEER_SCATTER ? 4 * 32 * (BITS == 4 ? 128 : 64) : 0>;
+  static_assert(L::DYN_BYTES <= 227 * 1024, "shared memory of the quantized matmul");
   // A stage is dequantized by eight warps, one thread per row and group. One team's time per stage (barrier waits, shared
   // memory latency, arithmetic, proxy fence, arrival) is longer than the stage's products, so with three B stages two
   // teams take turns. 4 bits, M 4096, N 12288, K 3072, GELU: 264 -> 227 us; M 4608, N 3072, K 15360: 322 -> 297 us; M
@@ -614,7 +616,7 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   constexpr int NDQ = 8;
   constexpr int TEAMS = SD > 2 ? 2 : 1;
   constexpr int NUM_THREADS = (FIXED_WARPS + TEAMS * NDQ) * 32;
-  auto kern = qmm_kernel<BITS, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EXT>;
+  auto kern = qmm_kernel<BITS, BNH, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EXT>;
   static SmemConfigured configured;  // one record per instantiation of the kernel
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::DYN_BYTES, configured)) return rc;
   kern<<<grid, NUM_THREADS, L::DYN_BYTES, st>>>(tx, tw, tsb, tt, tlb, p);
@@ -622,29 +624,29 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   return MFX_OK;
 }
 
-template <int BITS, uint32_t WF, int ST, int SD, typename OUT, bool EXT>
+template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT, bool EXT>
 int launch_ext(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tsb, const CUtensorMap& tt,
            const CUtensorMap& tlb, const Params& p, int grid, cudaStream_t st) {
   switch (p.epilogue) {
-    case MFX_EPI_GELU_ERF: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_GELU_ERF, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
-    case MFX_EPI_GELU_TANH: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_GELU_TANH, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
-    case MFX_EPI_GATE_RESIDUAL: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_GATE_RESIDUAL, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
-    case MFX_EPI_SILU: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_SILU, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
-    case MFX_EPI_SWIGLU: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_SWIGLU, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    case MFX_EPI_GELU_ERF: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_GELU_ERF, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    case MFX_EPI_GELU_TANH: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_GELU_TANH, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    case MFX_EPI_GATE_RESIDUAL: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_GATE_RESIDUAL, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    case MFX_EPI_SILU: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_SILU, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    case MFX_EPI_SWIGLU: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_SWIGLU, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
     case MFX_EPI_PEER_SCATTER:
-      if constexpr (sizeof(OUT) == 2 && !EXT)
-        return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_PEER_SCATTER, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+      if constexpr (sizeof(OUT) == 2 && !EXT && BNH == BN_MAX / 2 && SD == 2)   // room for its staging tile
+        return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_PEER_SCATTER, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
       else
         return MFX_ERR_DTYPE;
-    default: return launch_epi<BITS, WF, ST, SD, OUT, MFX_EPI_NONE, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
+    default: return launch_epi<BITS, BNH, WF, ST, SD, OUT, MFX_EPI_NONE, EXT>(tx, tw, tsb, tt, tlb, p, grid, st);
   }
 }
 
-template <int BITS, uint32_t WF, int ST, int SD, typename OUT>
+template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT>
 int launch(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tsb, const CUtensorMap& tt,
            const CUtensorMap& tlb, const Params& p, int grid, cudaStream_t st) {
-  return p.num_ext > 0 ? launch_ext<BITS, WF, ST, SD, OUT, true>(tx, tw, tsb, tt, tlb, p, grid, st)
-                       : launch_ext<BITS, WF, ST, SD, OUT, false>(tx, tw, tsb, tt, tlb, p, grid, st);
+  return p.num_ext > 0 ? launch_ext<BITS, BNH, WF, ST, SD, OUT, true>(tx, tw, tsb, tt, tlb, p, grid, st)
+                       : launch_ext<BITS, BNH, WF, ST, SD, OUT, false>(tx, tw, tsb, tt, tlb, p, grid, st);
 }
 
 // sb[g * N + n] = bf16(scales[n, g]) | bf16(biases[n, g]) << 16
@@ -792,6 +794,28 @@ static bool tmem_operand_kernel() {
   return on;
 }
 
+// Output columns of a pair tile: 256, 192 or 128, whichever fills the pairs with the least time. Few or unluckily many
+// wide tiles leave pairs idle in the only or the last wave; a narrower tile moves as many bytes of activations for fewer
+// products, so its wave is not shorter in proportion. Time of a wave in percent of the wide one's, measured: 90 and 69
+// (4 bits), 80 and 60 (8 bits, where narrower tiles make room for the third B stage and with it the second team).
+// Measured at 256 / 192 / 128, us: M 512, N 3072, K 12288 61.9 / 55.0 / 41.6 (4 bits), 74.8 / 59.0 / 43.8 (8 bits); M
+// 1613, N 3840, K 10240 108.7 / 103.2 / 112.6 and 128.5 / 112.8 / 117.9; M 1613, N 20480, K 3840 190.5 / 210.1 / 226.8
+// and 218.0 / 225.6 / 233.6.
+static int tile_width(int64_t m_tiles, int64_t N, int64_t pairs, int kb) {
+  const int64_t percent[3] = {100, kb == 4 ? 90 : 80, kb == 4 ? 69 : 60};
+  int best = 256;
+  int64_t best_cost = 0;
+  for (int i = 0; i < 3; ++i) {
+    const int bn = 256 - 64 * i;
+    const int64_t waves = (m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
+    if (i == 0 || waves * percent[i] < best_cost) {
+      best = bn;
+      best_cost = waves * percent[i];
+    }
+  }
+  return best;
+}
+
 // scratch: optional, see mfx_qlinear_ex_scratch
 int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStream_t st) {
   const bool scatter = a.epilogue == MFX_EPI_PEER_SCATTER;
@@ -859,6 +883,10 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
   const void* codes = prepared;
   const void* sb_packed = static_cast<const uint8_t*>(prepared) + codes_bytes_padded(a.N, a.K, a.bits);
 
+  const int pairs = device_sm_count() / 2;
+  const int64_t m_tiles = (a.rows + 2 * BM - 1) / (2 * BM) * a.batch;
+  const int bn = scatter ? BN_MAX : tile_width(m_tiles, a.N, pairs, kb);
+  const uint32_t half_n = static_cast<uint32_t>(bn / 2);
   CUtensorMap tx, tw, tsb, tt, tlb;
   {
     const uint64_t dims[3] = {static_cast<uint64_t>(a.K), static_cast<uint64_t>(a.rows),
@@ -876,7 +904,7 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
     const uint64_t words_per_row = static_cast<uint64_t>(a.K) * kb / 32;
     const uint64_t dims[2] = {words_per_row, static_cast<uint64_t>(a.N)};
     const uint64_t strides[1] = {words_per_row * 4};
-    const uint32_t box[2] = {static_cast<uint32_t>(BK * kb / 32), BN_HALF};  // each CTA of a pair: 128 weight rows
+    const uint32_t box[2] = {static_cast<uint32_t>(BK * kb / 32), half_n};   // each CTA of a pair: its half of the rows
     if (int rc = encode_tmap(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, codes, dims, strides, box,
                              kb == 4 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B))
       return rc;
@@ -884,7 +912,7 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
   {
     const uint64_t dims[2] = {static_cast<uint64_t>(a.N), static_cast<uint64_t>(a.K / 64)};
     const uint64_t strides[1] = {static_cast<uint64_t>(a.N) * 4};
-    const uint32_t box[2] = {BN_HALF, 1};
+    const uint32_t box[2] = {half_n, 1};
     if (int rc = encode_tmap(&tsb, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, sb_packed, dims, strides, box,
                              CU_TENSOR_MAP_SWIZZLE_NONE))
       return rc;
@@ -902,7 +930,7 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
     // the dense tile takes the place of the packed codes in shared memory: same bytes per row (32 or 64), same swizzle
     const uint64_t bdims[2] = {static_cast<uint64_t>(a.lora_ld), static_cast<uint64_t>(a.N)};
     const uint64_t bstrides[1] = {static_cast<uint64_t>(a.lora_ld) * 2};
-    const uint32_t bbox[2] = {static_cast<uint32_t>(4 * kb), BN_HALF};
+    const uint32_t bbox[2] = {static_cast<uint32_t>(4 * kb), half_n};
     if (int rc = encode_tmap(&tlb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.lora_b, bdims, bstrides, bbox,
                              kb == 4 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B))
       return rc;
@@ -919,14 +947,14 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
   p.K = static_cast<int>(a.K);
   p.tiles_m_per_sample = static_cast<int>((a.rows + 2 * BM - 1) / (2 * BM));  // a pair covers 256 activation rows
   p.tiles_m = p.tiles_m_per_sample * p.batch;
-  p.tiles_n = static_cast<int>((a.N + BN - 1) / BN);
+  p.tiles_n = static_cast<int>((a.N + bn - 1) / bn);
   const int64_t total = static_cast<int64_t>(p.tiles_m) * p.tiles_n;
   if (total > (1ll << 30)) return MFX_ERR_TOO_LARGE;
   p.total_tiles = static_cast<int>(total);
   {
     // bands of weight rows that stay L2-resident while every activation tile passes over them: 32 MB leaves room
     // for the activation and output tiles in flight even if each die's half of the L2 keeps its own copy
-    const int64_t n_tile_bytes = static_cast<int64_t>(BN) * (a.K * kb / 8 + a.K / 64 * 4);
+    const int64_t n_tile_bytes = static_cast<int64_t>(bn) * (a.K * kb / 8 + a.K / 64 * 4);
     const int64_t bands = (n_tile_bytes * p.tiles_n + (32ll << 20) - 1) / (32ll << 20);
     p.band_n = static_cast<int>((p.tiles_n + bands - 1) / bands);
     if (p.band_n < 1) p.band_n = 1;
@@ -956,18 +984,29 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
     }
     p.sc_done = sc.done_counter;
   }
-  const int pairs = device_sm_count() / 2;
   const bool f32_out = a.y_dtype == MFX_F32 && !scatter;
   const int grid = 2 * (p.total_tiles < pairs ? p.total_tiles : pairs);
   const bool f32 = f32_out;
   if (kb == 4) {
     // the scatter epilogue's staging tile takes the room of the third dequantized-weight stage
-    if (scatter) return launch<4, FMT_BF16, 3, 2, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
-    return f32 ? launch<4, FMT_BF16, 3, 3, float>(tx, tw, tsb, tt, tlb, p, grid, st)
-               : launch<4, FMT_BF16, 3, 3, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+    if (scatter) return launch<4, 128, FMT_BF16, 3, 2, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+    if (bn == 128)
+      return f32 ? launch<4, 64, FMT_BF16, 4, 4, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+                 : launch<4, 64, FMT_BF16, 4, 4, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+    if (bn == 192)
+      return f32 ? launch<4, 96, FMT_BF16, 3, 3, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+                 : launch<4, 96, FMT_BF16, 3, 3, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+    return f32 ? launch<4, 128, FMT_BF16, 3, 3, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+               : launch<4, 128, FMT_BF16, 3, 3, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
   }
-  return f32 ? launch<8, FMT_BF16, 3, 2, float>(tx, tw, tsb, tt, tlb, p, grid, st)
-             : launch<8, FMT_BF16, 3, 2, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+  if (bn == 128)
+    return f32 ? launch<8, 64, FMT_BF16, 4, 3, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+               : launch<8, 64, FMT_BF16, 4, 3, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+  if (bn == 192)
+    return f32 ? launch<8, 96, FMT_BF16, 3, 3, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+               : launch<8, 96, FMT_BF16, 3, 3, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
+  return f32 ? launch<8, 128, FMT_BF16, 3, 2, float>(tx, tw, tsb, tt, tlb, p, grid, st)
+             : launch<8, 128, FMT_BF16, 3, 2, __nv_bfloat16>(tx, tw, tsb, tt, tlb, p, grid, st);
 }
 
 // ---------------------------------------------------------------- allocation-free variant
