@@ -842,20 +842,26 @@ MFX_DEFINE_STATUS_READER(read_status)
 namespace mfx {
 namespace attn {
 
-// Which kernel serves a call. The ping-pong kernel (two query tiles per CTA, one CTA per SM) is the faster main
-// loop (1245-1270 against 1150-1170 TFLOP/s at 16 x 24 heads x 4608 tokens), but its work items are twice as
-// large: it is chosen from 1024 keys on, and only if the last wave of CTAs leaves at most 7 % of the SMs' time
-// unused (2 x 24 heads x 7145 tokens is 9.08 waves of 148 = 91 %: 1091 against 1158 TFLOP/s, the other kernel wins).
+// Which kernel serves a call. The ping-pong kernel (two query tiles per CTA, one CTA per SM) has the faster main loop,
+// but its work items are twice as large; the pair kernel's last wave costs 0.6 of a full one when it has at most one CTA
+// per SM. Compared as waves of 256 queries per SM, the pair kernel's 3 % longer, the ping-pong kernel's by the half item
+// an odd number of 128-query tiles wastes; below 2048 keys a second wave of ping-pong CTAs never paid. Measured pair /
+// ping-pong, us: 24 heads x 4096 (2.59 waves) 188.7 / 175.5; 6 x 4608 (0.73) 71.7 / 66.0; 12 x 2500 (0.81) 44.9 / 41.9;
+// 2 x 12 x 4352 (2.76) 204.9 / 190.3; 4 x 24 x 4096 (10.38) 767 / 796; 2 x 24 x 3600 (29 tiles) 304 / 326; 24 x 2048
+// (1.30) 57.4 / 65.7; 6 x 2500 (0.41) 30.4 / 39.1.
 // MFX_FMHA_KERNEL=pingpong | pair overrides the choice.
 static bool use_pingpong(int64_t seq, int64_t seq_kv, int64_t batch, int heads) {
   const char* e = getenv("MFX_FMHA_KERNEL");
   if (e && e[0] == 'p' && e[1] == 'i') return true;
   if (e && e[0] == 'p' && e[1] == 'a') return false;
-  if (seq_kv < 1024) return false;
-  const int64_t ctas = (seq + 2 * BQ - 1) / (2 * BQ) * heads * batch;
   const int64_t sms = device_sm_count();
-  const int64_t waves = (ctas + sms - 1) / sms;
-  return ctas * 100 >= waves * sms * 93;
+  const int64_t tiles = (seq + BQ - 1) / BQ, items = (tiles + 1) / 2;
+  const int64_t pairs = tiles * heads * batch;                       // CTAs of the pair kernel, two per SM
+  const int64_t waves = (items * heads * batch + sms - 1) / sms;     // of ping-pong CTAs
+  if (seq_kv < (waves > 1 ? 2048 : 1024)) return false;
+  const int64_t rest = pairs % (2 * sms);
+  const double pair_cost = static_cast<double>(pairs / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
+  return static_cast<double>(waves) * static_cast<double>(2 * items) < pair_cost * 1.03 * static_cast<double>(tiles);
 }
 
 // Arguments of one attention call (the C entry points fill it).
