@@ -277,7 +277,12 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
         a.lora_b, a.lora_ld, a.lora_r = lora_b.data_ptr(), ld, int(lora_r)
     need = _scratch_bytes(rows * batch, n, k, bits)
     # room for the decoded weight; freed to this stream's pool on return, so reused only behind this call's kernels
-    scratch = torch.empty(need, dtype=torch.uint8, device=x.device) if need else None
+    scratch = None
+    if need:
+        try:
+            scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
+        except torch.OutOfMemoryError:
+            need = 0   # the one-launch kernel does without
     if TRACE is not None:
         _trace_begin()
     rc = lib.mfx_qlinear_ex_scratch(byref(a), _ptr(scratch), need, _stream())

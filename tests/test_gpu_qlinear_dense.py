@@ -138,3 +138,19 @@ def test_rule_and_call_through_it(lib_built, bits, rows):
     wd = ops.dequantize_affine(wq, s, bi, 64, bits, torch.float32).cpu()
     ref = x[::97].float().cpu() @ wd.t()
     assert quant.rel_l2(y[::97], ref.numpy()) <= 1e-2
+
+
+def test_no_room_for_scratch_runs_without_it(lib_built, monkeypatch):
+    from mflux_b200 import ops
+
+    n, k = 264, 128
+    g = torch.Generator(device="cpu").manual_seed(4)
+    w = (torch.randn(n, k, generator=g) * 0.05).to(torch.bfloat16).cuda()
+    x = torch.randn(40, k, generator=g).to(torch.bfloat16).cuda()
+    wq, s, bi = ops.quantize_affine(w, 64, 4)
+    prep = ops.prepare_qlinear(wq, s, bi, 4)
+    want = ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep)
+    monkeypatch.setattr(ops, "_scratch_bytes", lambda *a: 1 << 50)      # a petabyte: the allocator refuses on the host
+    before = ops.LAUNCHES[0]
+    assert torch.equal(ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep), want)
+    assert ops.LAUNCHES[0] - before == 1
