@@ -77,8 +77,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
 
 // Epilogue activations. Four warps per CTA turn 256 accumulator columns per row while the main loop fills the next
 // tile; calls of erff / tanhf per value took longer than that loop (M 4096, N 12288, K 3072, 4 bits, erf form: 371 us,
-// 290 us with the form below). Both GELUs are therefore branch-free, two special-function instructions each, and
-// without the cancellation of 1 + erf(x) or 1 + tanh(x) on the negative side.
+// 290 us with the form below, 227 us with a second dequantizer team on top). Both GELUs are therefore branch-free, two
+// special-function instructions each, and without the cancellation of 1 + erf(x) or 1 + tanh(x) on the negative side.
 //
 // gelu(v) = max(v, 0) - |v| erfc(|v| / sqrt 2) / 2. erfc(z) exp(z^2) / t is a polynomial of degree 7 in
 // t = 1 / (1 + 0.45 z), the coefficients below are half of it: least squares with weights iterated towards an even

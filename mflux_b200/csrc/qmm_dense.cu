@@ -337,7 +337,8 @@ static int64_t num_bands(int64_t N, int64_t row_bytes, int64_t limit) {
 
 // Where the two launches win. The decode costs 2.6 (4 bits) or 3.1 bytes of HBM traffic per weight whatever the row
 // count. Measured gains with it included, looped at the power limit:
-//   8 bits  even at 2200 rows, 3-5 % at 3000, 8-15 % at 8400 (N 3840 to 20480);
+//   8 bits  even at 2200 rows, 3-5 % at 3000, 8-15 % at 8400 (N 3840 to 20480), where more passes over the activations
+//           than the packed weight needs feed at least 8192 output columns each;
 //   4 bits  3 % at 3072 rows, 5-8 % from 4600 on where the bf16 weight fits one band (N 3072, K 3072); where it needs a
 //           second pass over the activations that the packed weight does not, even at 6100 to 8200 rows and 1-3 % from
 //           there on if that pass feeds many output columns (N 9216, 12288), a loss of 3-5 % if it feeds few (N 3072, K
@@ -346,7 +347,7 @@ static int64_t num_bands(int64_t N, int64_t row_bytes, int64_t limit) {
 size_t scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
   const int kb = kernel_bits(bits);
   const int64_t extra = num_bands(N, 2 * K, BAND_BYTES) - num_bands(N, K * kb / 8 + K / 16, 32ll << 20);
-  if (extra > 1 || (extra == 1 && N < 8192)) return 0;
+  if (N < 8192 * extra || (kb == 4 && extra > 1)) return 0;
   if (rows < (kb == 8 ? 2560 : extra > 0 ? 8192 : 3072)) return 0;
   if (2.0 * static_cast<double>(rows) * static_cast<double>(N) * static_cast<double>(K) < 5e10) return 0;
   return dense_bytes(N, K);
