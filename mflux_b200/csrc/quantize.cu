@@ -142,17 +142,17 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
     }
     reinterpret_cast<uint4*>(wq)[g * 4 + sub] = make_uint4(word[0], word[1], word[2], word[3]);
   } else {
-    // 8 codes = BITS bytes of the bit stream
-    uint8_t* dst = reinterpret_cast<uint8_t*>(wq) + (g * 4 + sub) * (2 * BITS);
+    // 8 codes = BITS bytes of the bit stream; 16 of them are BITS 16-bit words at an even address
+    unsigned long long lo = 0, hi = 0;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      unsigned long long stream = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        stream |= static_cast<unsigned long long>(static_cast<uint32_t>(q[8 * k + i])) << (BITS * i);
-#pragma unroll
-      for (int i = 0; i < BITS; ++i) dst[BITS * k + i] = static_cast<uint8_t>(stream >> (8 * i));
+    for (int i = 0; i < 8; ++i) {
+      lo |= static_cast<unsigned long long>(static_cast<uint32_t>(q[i])) << (BITS * i);
+      hi |= static_cast<unsigned long long>(static_cast<uint32_t>(q[8 + i])) << (BITS * i);
     }
+    const unsigned long long w0 = lo | (hi << (8 * BITS)), w1 = hi >> (64 - 8 * BITS);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(wq) + (g * 4 + sub) * BITS;
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) dst[i] = static_cast<uint16_t>(i < 4 ? w0 >> (16 * i) : w1 >> (16 * (i & 3)));
   }
   if (sub == 0) {
     scales[g] = from_f32<T>(scale);
@@ -185,14 +185,19 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
 #pragma unroll
     for (int i = 0; i < 16; ++i) codes[i] = (w4[i >> 2] >> (8 * (i & 3))) & 0xFF;
   } else {
-    const uint8_t* src = reinterpret_cast<const uint8_t*>(wq) + tid * (2 * BITS);
+    const uint16_t* src = reinterpret_cast<const uint16_t*>(wq) + tid * BITS;
+    unsigned long long w0 = 0, w1 = 0;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      unsigned long long stream = 0;
+    for (int i = 0; i < BITS; ++i) {
+      const unsigned long long v = __ldg(src + i);
+      if (i < 4) w0 |= v << (16 * i);
+      else w1 |= v << (16 * (i & 3));
+    }
+    const unsigned long long hi = (w0 >> (8 * BITS)) | (w1 << (64 - 8 * BITS));
 #pragma unroll
-      for (int i = 0; i < BITS; ++i) stream |= static_cast<unsigned long long>(__ldg(src + BITS * k + i)) << (8 * i);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) codes[8 * k + i] = static_cast<uint32_t>(stream >> (BITS * i)) & ((1u << BITS) - 1u);
+    for (int i = 0; i < 8; ++i) {
+      codes[i] = static_cast<uint32_t>(w0 >> (BITS * i)) & ((1u << BITS) - 1u);
+      codes[8 + i] = static_cast<uint32_t>(hi >> (BITS * i)) & ((1u << BITS) - 1u);
     }
   }
   __align__(16) OUT res[16];
