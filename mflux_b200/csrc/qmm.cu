@@ -569,7 +569,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
           __syncwarp();
         }
       } else {
-        write_row<OUT, EPI>(t_addr, 0, BN, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
+        write_row<OUT, EPI, false>(t_addr, 0, BN, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
       }
       tc_fence_before();
       __syncwarp();

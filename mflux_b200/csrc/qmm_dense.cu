@@ -230,7 +230,7 @@ dense_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
       if (!mbar_wait_sleep(acc_full(a), (it >> 1) & 1, DEV_TIMEOUT_ACC_FULL)) break;
       tc_fence_after();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + a * BN;
-      qmm::write_row<OUT, EPI>(t_addr, c0, c1, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
+      qmm::write_row<OUT, EPI, true>(t_addr, c0, c1, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_leader(acc_empty(a));

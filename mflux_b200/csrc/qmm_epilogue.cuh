@@ -28,13 +28,13 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // bias and activation of eight neighbouring columns (not the residual, not SwiGLU's product)
-template <int EPI>
+template <int EPI, bool CALLS>
 __device__ __forceinline__ void activate8(const uint32_t* acc, const float* bias_s, float (&v)[8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     v[j] = __uint_as_float(acc[j]) + bias_s[j];
-    if (EPI == MFX_EPI_GELU_ERF) v[j] = gelu_erf(v[j]);
-    else if (EPI == MFX_EPI_GELU_TANH) v[j] = gelu_tanh(v[j]);
+    if (EPI == MFX_EPI_GELU_ERF) v[j] = CALLS ? gelu_erf_call(v[j]) : gelu_erf(v[j]);
+    else if (EPI == MFX_EPI_GELU_TANH) v[j] = CALLS ? gelu_tanh_call(v[j]) : gelu_tanh(v[j]);
     else if (EPI == MFX_EPI_SILU) v[j] = silu(v[j]);
   }
 }
@@ -85,8 +85,9 @@ inline bool wide_rows(const void* y, int64_t y_row_stride, int64_t y_batch_strid
 
 // Writes columns [c0, c1) (multiples of 32) of one output row of a tile. t_addr = the warp's lanes of the accumulator,
 // n_left = output columns of the layer from the tile's first one on, yrow / rrow = the row's first column of this
-// tile, wide = wide_rows(). Runs converged: rows past the end (row_ok false) take part in the tensor-memory loads only.
-template <typename OUT, int EPI>
+// tile, wide = wide_rows(), CALLS = out-of-line activations. Runs converged: rows past the end (row_ok false) take part
+// in the tensor-memory loads only.
+template <typename OUT, int EPI, bool CALLS>
 __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n_left, bool row_ok, bool wide, OUT* yrow,
                                           const OUT* rrow, const float* bias_s, const float* gate_s) {
 #pragma unroll 1
@@ -106,7 +107,7 @@ __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n
       for (int g8 = 0; g8 < 4; ++g8) {
         const int col = c + g8 * 8;
         float v[8];
-        activate8<EPI>(acc + g8 * 8, bias_s + col, v);
+        activate8<EPI, CALLS>(acc + g8 * 8, bias_s + col, v);
         if constexpr (EPI == MFX_EPI_SWIGLU) {
           float s[4];
 #pragma unroll
@@ -142,7 +143,7 @@ __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n
       const int col = c + g8 * 8;
       if (col >= n_left) break;
       float v[8];
-      activate8<EPI>(acc + g8 * 8, bias_s + col, v);
+      activate8<EPI, CALLS>(acc + g8 * 8, bias_s + col, v);
       if constexpr (EPI == MFX_EPI_SWIGLU) {
         float s[4];
 #pragma unroll
