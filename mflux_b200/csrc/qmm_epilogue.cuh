@@ -85,14 +85,15 @@ inline bool wide_rows(const void* y, int64_t y_row_stride, int64_t y_batch_strid
 
 // Writes columns [c0, c1) (multiples of 32) of one output row of a tile. t_addr = the warp's lanes of the accumulator,
 // n_left = output columns of the layer from the tile's first one on, yrow / rrow = the row's first column of this
-// tile, wide = wide_rows(), CALLS = out-of-line activations. Runs converged: rows past the end (row_ok false) take part
-// in the tensor-memory loads only.
+// tile, wide = wide_rows(), CALLS = out-of-line activations. Rows past the end (row_ok false) take part in the
+// tensor-memory loads only, which are collective: lanes take different paths below, so the warp meets before each.
 template <typename OUT, int EPI, bool CALLS>
 __device__ __forceinline__ void write_row(uint32_t t_addr, int c0, int c1, int n_left, bool row_ok, bool wide, OUT* yrow,
                                           const OUT* rrow, const float* bias_s, const float* gate_s) {
 #pragma unroll 1
   for (int c = c0; c < c1; c += 32) {
     uint32_t acc[32];
+    __syncwarp();
     tmem_ld_32x32(t_addr + c, acc);
     tmem_ld_wait();
     if (!row_ok) continue;

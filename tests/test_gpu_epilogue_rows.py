@@ -40,3 +40,32 @@ def test_misaligned_rows_give_the_same_values(lib_built, bits, epi, dtype, n):
     for offset, pad in ((step, 2 * step), (0, step), (step, step)):
         assert torch.equal(run(offset, pad), want)
     assert ops.poll_device_status() == 0
+
+
+@pytest.mark.parametrize("two_launches", [False, True])
+@pytest.mark.parametrize("epi", [None, "gelu", "gelu_approx", "silu", "gate_residual", "swiglu"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("m", [17, 287, 2 * 256 + 33, 3 * 256 + 128 + 63])
+def test_warps_whose_last_rows_are_missing(lib_built, monkeypatch, two_launches, epi, dtype, m):
+    """A last row tile that ends inside a warp's 32 rows: some lanes of the warp write, the others only take part in the
+    collective accumulator loads. The same rows as from a call whose tiles are full, on a column count with whole and
+    broken 32-column chunks."""
+    from mflux_b200 import ops
+
+    n, k = 528, 192
+    g = torch.Generator(device="cpu").manual_seed(m)
+    wq, s, b = ops.quantize_affine((torch.randn(n, k, generator=g) * 0.1).to(torch.bfloat16).cuda(), 64, 4)
+    full = -(-m // 256) * 256
+    x = torch.randn(full, k, generator=g).to(torch.bfloat16).cuda()
+    bias = torch.randn(n, generator=g).to(torch.bfloat16).cuda()
+    res = torch.randn(full, n, generator=g).to(dtype).cuda()
+    monkeypatch.setattr(ops, "_scratch_bytes", lambda *a: 2 * n * k if two_launches else 0)
+
+    def run(rows):
+        kw = {"gate": bias[None], "residual": res[:rows]} if epi == "gate_residual" else {}
+        return ops.qlinear(x[:rows], wq, s, b, bias, bits=4, epilogue=epi, out_dtype=dtype, **kw)
+
+    got, want = run(m), run(full)
+    assert ops.poll_device_status() == 0
+    assert got.shape[0] == m and torch.isfinite(got.float()).all()
+    assert torch.equal(got, want[:m])
