@@ -201,9 +201,11 @@ int mfx_qlinear_ex(const mfx_qlinear_args* args /* host */, void* stream);
 /* mfx_qlinear_ex with scratch for the decoded weight. With at least 2 N K bytes (256-byte aligned device memory,
  * overwritten) the weight is decoded once to bf16 and contracted from there, in two launches; with less, for at most
  * 16 rows and for MFX_EPI_PEER_SCATTER this is mfx_qlinear_ex. The results are the same bit for bit, but for the place
- * of the low-rank products in the float32 accumulation. mfx_qlinear_scratch_bytes says how many bytes a call over
- * `rows` activation rows (all samples together) should pass: 2 N K where that form is the faster one, 0 elsewhere. */
+ * of the low-rank products in the float32 accumulation. mfx_qlinear_scratch_bytes_batch says how many bytes a call
+ * over `batch` samples of `rows` rows should pass: 2 N K where that form is the faster one, 0 elsewhere;
+ * mfx_qlinear_scratch_bytes is that for one sample. */
 size_t mfx_qlinear_scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits);
+size_t mfx_qlinear_scratch_bytes_batch(int64_t rows, int64_t batch, int64_t N, int64_t K, int bits);
 int mfx_qlinear_ex_scratch(const mfx_qlinear_args* args /* host */, void* scratch, size_t scratch_bytes, void* stream);
 
 /* The elementwise half of a tensor-parallel block on the rows this rank owns, fused with both collectives:

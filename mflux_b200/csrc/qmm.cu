@@ -801,7 +801,8 @@ static bool tmem_operand_kernel() {
 // Measured at 256 / 192 / 128, us: M 512, N 3072, K 12288 61.9 / 55.0 / 41.6 (4 bits), 74.8 / 59.0 / 43.8 (8 bits); M
 // 1613, N 3840, K 10240 108.7 / 103.2 / 112.6 and 128.5 / 112.8 / 117.9; M 1613, N 20480, K 3840 190.5 / 210.1 / 226.8
 // and 218.0 / 225.6 / 233.6.
-static int tile_width(int64_t m_tiles, int64_t N, int64_t pairs, int kb) {
+// `cost`: what that width takes, in percent of a wave of 256 columns.
+static int tile_width(int64_t m_tiles, int64_t N, int64_t pairs, int kb, int64_t* cost = nullptr) {
   const int64_t percent[3] = {100, kb == 4 ? 90 : 80, kb == 4 ? 69 : 60};
   int best = 256;
   int64_t best_cost = 0;
@@ -813,8 +814,12 @@ static int tile_width(int64_t m_tiles, int64_t N, int64_t pairs, int kb) {
       best_cost = waves * percent[i];
     }
   }
+  if (cost) *cost = best_cost;
   return best;
 }
+
+// 256-row tiles of `batch` samples of `rows` rows: a tile does not reach into the next sample.
+static int64_t row_tiles(int64_t rows, int64_t batch) { return (rows + 2 * BM - 1) / (2 * BM) * batch; }
 
 // scratch: optional, see mfx_qlinear_ex_scratch
 int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStream_t st) {
@@ -884,8 +889,7 @@ int run(const mfx_qlinear_args& a, void* scratch, size_t scratch_bytes, cudaStre
   const void* sb_packed = static_cast<const uint8_t*>(prepared) + codes_bytes_padded(a.N, a.K, a.bits);
 
   const int pairs = device_sm_count() / 2;
-  const int64_t m_tiles = (a.rows + 2 * BM - 1) / (2 * BM) * a.batch;
-  const int bn = scatter ? BN_MAX : tile_width(m_tiles, a.N, pairs, kb);
+  const int bn = scatter ? BN_MAX : tile_width(row_tiles(a.rows, a.batch), a.N, pairs, kb);
   const uint32_t half_n = static_cast<uint32_t>(bn / 2);
   CUtensorMap tx, tw, tsb, tt, tlb;
   {
@@ -1052,8 +1056,17 @@ int mfx_qlinear_ex_scratch(const mfx_qlinear_args* args, void* scratch, size_t s
 }
 
 size_t mfx_qlinear_scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
-  if (rows <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || !mfx::valid_bits(bits)) return 0;
-  return mfx::qmmd::scratch_bytes(rows, N, K, bits);
+  return mfx_qlinear_scratch_bytes_batch(rows, 1, N, K, bits);
+}
+
+size_t mfx_qlinear_scratch_bytes_batch(int64_t rows, int64_t batch, int64_t N, int64_t K, int bits) {
+  if (rows <= 0 || batch <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || !mfx::valid_bits(bits)) return 0;
+  if (rows > (1 << 30) || batch > (1 << 20) || N > (1 << 30) || K > (1 << 30)) return 0;   // refused by the call
+  const int64_t m_tiles = mfx::qmm::row_tiles(rows, batch);
+  if (m_tiles > (1 << 30)) return 0;
+  int64_t cost = 0;
+  mfx::qmm::tile_width(m_tiles, N, mfx::device_sm_count() / 2, mfx::kernel_bits(bits), &cost);
+  return mfx::qmmd::scratch_bytes(m_tiles, N, K, bits, cost);
 }
 
 size_t mfx_qlinear_prepared_bytes(int64_t N, int64_t K, int bits, int group_size) {

@@ -335,22 +335,28 @@ static int64_t num_bands(int64_t N, int64_t row_bytes, int64_t limit) {
   return ((N + BN - 1) / BN * BN * row_bytes + limit - 1) / limit;
 }
 
-// Where the two launches win. The decode costs 2.6 (4 bits) or 3.1 bytes of HBM traffic per weight whatever the row
-// count. Measured gains with it included, looped at the power limit:
-//   8 bits  even at 2200 rows, 3-5 % at 3000, 8-15 % at 8400 (N 3840 to 20480), where more passes over the activations
-//           than the packed weight needs feed at least 8192 output columns each;
-//   4 bits  3 % at 3072 rows, 5-8 % from 4600 on where the bf16 weight fits one band (N 3072, K 3072); where it needs a
-//           second pass over the activations that the packed weight does not, even at 6100 to 8200 rows and 1-3 % from
-//           there on if that pass feeds many output columns (N 9216, 12288), a loss of 3-5 % if it feeds few (N 3072, K
-//           12288; N 3840, K 10240) or if two passes come on top (N 20480, K 3840).
-// The second launch costs 2-3 us, which a call of less than 5e10 operations does not earn back.
-size_t scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
+// Where the two launches win: their cost against the best the one-launch kernel can do with its tile widths
+// (one_launch_cost), both in percent of a wave of that kernel's 256-column tiles, so that a part-filled last wave counts
+// for either side. A wave here takes 83 % of it for 8 bits and 93 % for 4 (95 % where the bf16 weight is past 32 MB); the
+// decode moves 2.6 (4 bits) or 3.1 bytes of HBM traffic per weight, which is 0.0065 of a wave per output column; the second
+// launch costs 2.5 us, a wave 8 ns per k. Two passes over the activations more than the packed weight needs, or one that
+// feeds few output columns, cost 4-bit layers more than all that gains (N 3072, K 12288: 9 % at 4608 rows, 5 % at 8426).
+// Measured, looped at the power limit, one launch / two, us. 8 bits: M 2304, N 12288, K 3072 161 / 156, 4608 317 / 285;
+// M 2816, N 3840, K 10240 (165 tiles, 2.2 waves) 208 / 224, 3328 (195 tiles) 252 / 239; M 3328, N 3072, K 3072 61.3 /
+// 63.9, 4096 75.7 / 70.9. 4 bits: M 4608, N 3072, K 3072 71.2 / 75.5, 8192 135.5 / 132.7, 18432 282 / 269; M 8192, N
+// 9216, K 3072 364 / 362, 18432 818 / 791. Below the limit the one-launch kernel gains more from the higher clock (4 bits,
+// M 8426, N 3072, K 3072: 125 / 135), so a predicted gain of less than 2.5 % does not count.
+size_t scratch_bytes(int64_t m_tiles, int64_t N, int64_t K, int bits, int64_t one_launch_cost) {
   const int kb = kernel_bits(bits);
   const int64_t extra = num_bands(N, 2 * K, BAND_BYTES) - num_bands(N, K * kb / 8 + K / 16, 32ll << 20);
   if (N < 8192 * extra || (kb == 4 && extra > 1)) return 0;
-  if (rows < (kb == 8 ? 2560 : extra > 0 ? 8192 : 3072)) return 0;
-  if (2.0 * static_cast<double>(rows) * static_cast<double>(N) * static_cast<double>(K) < 5e10) return 0;
-  return dense_bytes(N, K);
+  // (too little work to judge a cost in waves of the main loop by)
+  if (2.0 * 256.0 * static_cast<double>(m_tiles) * static_cast<double>(N) * static_cast<double>(K) < 5e10) return 0;
+  const int64_t pairs = device_sm_count() / 2;
+  const int64_t waves = (m_tiles * ((N + BN - 1) / BN) + pairs - 1) / pairs;
+  const int64_t wave = kb == 8 ? 83 : dense_bytes(N, K) <= (32u << 20) ? 93 : 95;
+  const int64_t cost = waves * wave + N * 13 / 2000 + 31000 / K;
+  return cost * 40 <= one_launch_cost * 39 ? dense_bytes(N, K) : 0;
 }
 
 int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, void* scratch, cudaStream_t st) {

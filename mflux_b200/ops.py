@@ -76,8 +76,8 @@ def _prepared_bytes(n: int, k: int, bits: int, group_size: int) -> int:
 
 
 @lru_cache(maxsize=4096)
-def _scratch_bytes(rows: int, n: int, k: int, bits: int) -> int:
-    return _lib.load().mfx_qlinear_scratch_bytes(rows, n, k, bits)
+def _scratch_bytes(rows: int, batch: int, n: int, k: int, bits: int) -> int:
+    return _lib.load().mfx_qlinear_scratch_bytes_batch(rows, batch, n, k, bits)
 
 
 def poll_device_status() -> int:
@@ -275,7 +275,7 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
             raise ValueError("lora_t must be [.., rows, ld] like x and lora_b a dense [N, ld]")
         a.lora_t, a.lora_t_row_stride, a.lora_t_batch_stride = tv.data_ptr(), t_rs, t_bs
         a.lora_b, a.lora_ld, a.lora_r = lora_b.data_ptr(), ld, int(lora_r)
-    need = _scratch_bytes(rows * batch, n, k, bits)
+    need = _scratch_bytes(rows, batch, n, k, bits)
     # room for the decoded weight; freed to this stream's pool on return, so reused only behind this call's kernels
     scratch = None
     if need:

@@ -115,7 +115,7 @@ def test_short_or_misaligned_scratch_is_not_used(lib_built):
         assert bool((scratch[:need] == 0x5A).all()) != used and (scratch[need:] == 0x5A).all()
 
 
-@pytest.mark.parametrize("bits,rows", [(4, 8192), (8, 2560)])
+@pytest.mark.parametrize("bits,rows", [(4, 18432), (8, 2560)])
 def test_rule_and_call_through_it(lib_built, bits, rows):
     """The rule asks for scratch on a wide layer with many rows and not below its limits; a call that it sends through
     the two launches, prepared on the fly."""
