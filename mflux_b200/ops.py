@@ -80,6 +80,40 @@ def _scratch_bytes(rows: int, batch: int, n: int, k: int, bits: int) -> int:
     return _lib.load().mfx_qlinear_scratch_bytes_batch(rows, batch, n, k, bits)
 
 
+# Scratch sizes a device had no room for, with the bytes that were free then, per device index. Before it refuses, the
+# allocator waits for the device and gives its whole cache back, which a step of many layers must not pay for each of
+# them: a size is asked for again once more is free than at any refusal of it or of less.
+_REFUSED: dict[int, dict[int, int]] = {}
+
+
+def _free_bytes(device: torch.device) -> int:
+    """What torch could allocate on the device: the driver's free memory and the free part of torch's own."""
+    return (torch.cuda.mem_get_info(device)[0] + torch.cuda.memory_reserved(device)
+            - torch.cuda.memory_allocated(device))
+
+
+def _scratch(need: int, device: torch.device) -> torch.Tensor | None:
+    """`need` bytes for one call, freed to the current stream's pool on return and so reused only behind that call's
+    kernels, or None where there is no room (the one-launch kernel does without)."""
+    index = device.index
+    known = [free for size, free in list(_REFUSED.get(index, {}).items()) if size <= need]
+    if known and (torch.cuda.is_current_stream_capturing() or _free_bytes(device) <= max(known)):
+        return None
+    try:
+        scratch = torch.empty(need, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        if torch.cuda.is_current_stream_capturing():   # the driver is not to be asked now
+            return None
+        refused = _REFUSED.setdefault(index, {})
+        if len(refused) >= 64:
+            refused.clear()
+        refused[need] = _free_bytes(device)
+        return None
+    if known:      # there is room again
+        _REFUSED[index] = {size: free for size, free in list(_REFUSED[index].items()) if size > need}
+    return scratch
+
+
 def poll_device_status() -> int:
     """Read and clear the device status word (0 = clean). Raises if a bounded wait gave up."""
     lib = _lib.load()
@@ -276,22 +310,16 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
         a.lora_t, a.lora_t_row_stride, a.lora_t_batch_stride = tv.data_ptr(), t_rs, t_bs
         a.lora_b, a.lora_ld, a.lora_r = lora_b.data_ptr(), ld, int(lora_r)
     need = _scratch_bytes(rows, batch, n, k, bits)
-    # room for the decoded weight; freed to this stream's pool on return, so reused only behind this call's kernels
-    scratch = None
-    if need:
-        try:
-            scratch = torch.empty(need, dtype=torch.uint8, device=x.device)
-        except torch.OutOfMemoryError:
-            need = 0   # the one-launch kernel does without
+    scratch = _scratch(need, x.device) if need else None   # room for the decoded weight
     if TRACE is not None:
         _trace_begin()
-    rc = lib.mfx_qlinear_ex_scratch(byref(a), _ptr(scratch), need, _stream())
+    rc = lib.mfx_qlinear_ex_scratch(byref(a), _ptr(scratch), 0 if scratch is None else need, _stream())
     _lib.check(rc, "mfx_qlinear_ex")
     if TRACE is not None:
         m = rows * batch
         _trace_end("qlinear", 2.0 * m * n * k, n * k * bits / 8 + 4.0 * n * (k // group_size) + 2.0 * m * k
                    + ov.element_size() * m * n_out)
-    LAUNCHES[0] += (1 if prepared is not None else 3) + (1 if need else 0)
+    LAUNCHES[0] += (1 if prepared is not None else 3) + (0 if scratch is None else 1)
     return ret
 
 
