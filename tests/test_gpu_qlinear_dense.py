@@ -151,6 +151,9 @@ def test_no_room_for_scratch_runs_without_it(lib_built, monkeypatch):
     prep = ops.prepare_qlinear(wq, s, bi, 4)
     want = ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep)
     monkeypatch.setattr(ops, "_scratch_bytes", lambda *a: 1 << 50)      # a petabyte: the allocator refuses on the host
-    before = ops.LAUNCHES[0]
-    assert torch.equal(ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep), want)
-    assert ops.LAUNCHES[0] - before == 1
+    monkeypatch.setattr(ops, "_REFUSED", {})
+    before, refused = ops.LAUNCHES[0], torch.cuda.memory_stats()["num_ooms"]
+    for _ in range(3):
+        assert torch.equal(ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep), want)
+    assert ops.LAUNCHES[0] - before == 3
+    assert torch.cuda.memory_stats()["num_ooms"] - refused == 1      # asked once, not on every call
