@@ -1,0 +1,59 @@
+"""QuantizedLinear as a torch module, on the CPU with the kernels' entry points replaced by recorders."""
+import pytest
+import torch
+
+from mflux_b200 import nn, ops
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """Records what reaches ops.qlinear."""
+    seen = []
+
+    def qlinear(x, wq, scales, biases, bias=None, **kw):
+        seen.append({"weight": wq, "scales": scales, "biases": biases, "bias": bias, **kw})
+        return x
+
+    monkeypatch.setattr(ops, "qlinear", qlinear)
+    monkeypatch.setattr(ops, "prepare_qlinear", lambda wq, s, b, bits, gs: (wq, s, b))
+    return seen
+
+
+class _Twice(torch.nn.Module):
+    def forward(self, t):
+        return 2 * t
+
+
+def _layer(bias=True):
+    layer = nn.QuantizedLinear(64, 8, bias=bias)
+    layer.scales.data.fill_(3.0)
+    if bias:
+        layer.bias.data.fill_(5.0)
+    return layer
+
+
+@pytest.mark.parametrize("name,value", [("bias", 10.0), ("scales", 6.0)])
+def test_parametrized_tensors_reach_the_call(calls, name, value):
+    layer = _layer()
+    torch.nn.utils.parametrize.register_parametrization(layer, name, _Twice())
+    layer(torch.zeros(1, 64))
+    assert (calls[0][name] == value).all()
+    if name == "scales":
+        assert (calls[0]["prepared"][1] == value).all()
+
+
+def test_a_bias_that_is_a_plain_attribute_reaches_the_call(calls):
+    layer = _layer()
+    del layer.bias
+    layer.bias = torch.full((8,), 7.0)
+    layer(torch.zeros(1, 64))
+    assert (calls[0]["bias"] == 7.0).all()
+
+
+def test_plain_parameters_and_no_bias(calls):
+    layer = _layer(bias=False)
+    layer(torch.zeros(1, 64))
+    assert calls[0]["bias"] is None and calls[0]["scales"] is layer.scales
+    layer.scales.data = layer.scales.data * 2     # replaced: the prepared form is built again
+    layer(torch.zeros(1, 64))
+    assert (calls[1]["prepared"][1] == 6.0).all()
