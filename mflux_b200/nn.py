@@ -136,12 +136,21 @@ class QuantizedLinear(Module):
 
     @classmethod
     def from_linear(cls, linear: Linear, group_size: int = 64, bits: int = 4, mode: str = "mlx"):
-        cls._check(linear.weight.shape[1], group_size, bits)
-        # without __init__, whose zero-filled tensors would only be replaced (three launches, 1/4 of the bytes written)
-        ql = cls.__new__(cls)
-        Module.__init__(ql)
-        ql._hold(*ops.quantize_affine(linear.weight.data, group_size, bits, mode),
-                 None if linear.bias is None else linear.bias.data, group_size, bits)
+        out_dims, in_dims = linear.weight.shape
+        cls._check(in_dims, group_size, bits)
+        packed = ops.quantize_affine(linear.weight.data, group_size, bits, mode)
+        bias = None if linear.bias is None else linear.bias.data
+        if cls.__init__ is QuantizedLinear.__init__:
+            # without __init__, whose zero-filled tensors would only be replaced (three launches, 1/4 of the bytes written)
+            ql = cls.__new__(cls)
+            Module.__init__(ql)
+            ql._hold(*packed, bias, group_size, bits)
+        else:      # a subclass whose __init__ sets up more than these tensors
+            ql = cls(in_dims, out_dims, bias is not None, group_size, bits, device=linear.weight.device,
+                     dtype=linear.weight.dtype)
+            ql.weight.data, ql.scales.data, ql.biases.data = packed
+            if bias is not None:
+                ql.bias.data = bias
         return ql
 
     @property

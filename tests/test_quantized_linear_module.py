@@ -57,3 +57,24 @@ def test_plain_parameters_and_no_bias(calls):
     layer.scales.data = layer.scales.data * 2     # replaced: the prepared form is built again
     layer(torch.zeros(1, 64))
     assert (calls[1]["prepared"][1] == 6.0).all()
+
+
+class _Tagged(nn.QuantizedLinear):
+    def __init__(self, *args, **kw):
+        super().__init__(*args, **kw)
+        self.tag = "set up"
+
+
+@pytest.mark.parametrize("cls", [nn.QuantizedLinear, _Tagged])
+@pytest.mark.parametrize("bias", [False, True])
+def test_from_linear_runs_the_setup_of_a_subclass(monkeypatch, cls, bias):
+    packed = (torch.ones(8, 8, dtype=torch.uint32), torch.full((8, 1), 2.0), torch.full((8, 1), 3.0))
+    monkeypatch.setattr(ops, "quantize_affine", lambda w, gs, bits, mode: packed)
+    linear = nn.Linear(64, 8, bias=bias)
+    layer = cls.from_linear(linear, bits=4)
+    assert type(layer) is cls and getattr(layer, "tag", "set up") == "set up" and (cls is not _Tagged or layer.tag)
+    for name, t in zip(("weight", "scales", "biases"), packed):
+        p = getattr(layer, name)
+        assert isinstance(p, torch.nn.Parameter) and not p.requires_grad and p.data_ptr() == t.data_ptr()
+    assert (layer.bias is None) if not bias else layer.bias.data_ptr() == linear.bias.data_ptr()
+    assert set(layer.state_dict()) == {"weight", "scales", "biases"} | ({"bias"} if bias else set())
