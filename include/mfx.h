@@ -349,6 +349,10 @@ typedef struct mfx_fmha_args {
 } mfx_fmha_args;
 int mfx_fmha_ex(const mfx_fmha_args* args /* host */, void* stream);
 
+/* How many tiles of 128 queries a thread block takes in a call of these sizes: 2 in the kernel for long sequences, 1 in
+ * the other; 0 for sizes that are not valid. (The environment variable MFX_FMHA_KERNEL=pair | pingpong overrides it.) */
+int mfx_fmha_query_tiles(int64_t seq_q, int64_t seq_kv, int64_t batch, int heads);
+
 /* out = act(a + b + c) elementwise (b, c nullable; act 0 = identity, 1 = SiLU, 2 = tanh): the conditioning-vector
  * arithmetic of time_text_embed.py:25-31, the nn.silu in front of every AdaLN linear and the mx.tanh on the
  * Z-Image gates (z_image_transformer/transformer_block.py:26-27). */

@@ -249,6 +249,7 @@ SIGNATURES = {
          c_int64, c_void_p],
     ),
     "mfx_fmha_ex": (c_int, [ctypes.POINTER(FmhaArgs), c_void_p]),
+    "mfx_fmha_query_tiles": (c_int, [c_int64, c_int64, c_int64, c_int]),
     "mfx_fmha_bias": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int, ctypes.c_float, c_void_p, c_int64,

@@ -843,25 +843,34 @@ namespace mfx {
 namespace attn {
 
 // Which kernel serves a call. The ping-pong kernel (two query tiles per CTA, one CTA per SM) has the faster main loop,
-// but its work items are twice as large; the pair kernel's last wave costs 0.6 of a full one when it has at most one CTA
-// per SM. Compared as waves of 256 queries per SM, the pair kernel's 3 % longer, the ping-pong kernel's by the half item
-// an odd number of 128-query tiles wastes; below 2048 keys a second wave of ping-pong CTAs never paid. Measured pair /
-// ping-pong, us: 24 heads x 4096 (2.59 waves) 188.7 / 175.5; 6 x 4608 (0.73) 71.7 / 66.0; 12 x 2500 (0.81) 44.9 / 41.9;
-// 2 x 12 x 4352 (2.76) 204.9 / 190.3; 4 x 24 x 4096 (10.38) 767 / 796; 2 x 24 x 3600 (29 tiles) 304 / 326; 24 x 2048
-// (1.30) 57.4 / 65.7; 6 x 2500 (0.41) 30.4 / 39.1.
+// but its work items are twice as large. It takes every call of 1024 keys or more whose waves it fills to 93 %; of the
+// others, those where it costs less by this count: waves of 256 queries per SM, the pair kernel's 3 % longer and its last
+// one 0.6 of a full one when it has at most one CTA per SM, the ping-pong kernel's lengthened by the half item that an odd
+// number of 128-query tiles wastes, and at least 2048 keys for a second wave. Measured pair / ping-pong, us, looped at the
+// power limit and (single calls below it). Full waves: 4 x 24 x 4096 (10.38 waves) 839 / 791 (717 / 679); 2 x 24 x 3600
+// (29 tiles) 351 / 329 (300 / 286); 4 x 30 x 1613 200 / 196 (169 / 172); 18 x 4 x 1024 46.3 / 44.3 (42.4 / 43.0). Others:
+// 24 x 4096 (2.59 waves) 224 / 206 (192 / 182); 2 x 12 x 4352 (2.76) 244 / 223 (209 / 195); 6 x 4608 (0.73) 76.3 / 70.3
+// (74.0 / 68.3); 12 x 2500 (0.81) 47.0 / 43.4 (45.7 / 43.2); 24 x 1024 21.5 / 21.0 (22.9 / 22.2).
+static bool pingpong_pays(int64_t seq, int64_t seq_kv, int64_t batch, int heads) {
+  if (seq_kv < 1024) return false;
+  const int64_t sms = device_sm_count();
+  const int64_t tiles = (seq + BQ - 1) / BQ, items = (tiles + 1) / 2;
+  const int64_t ctas = items * heads * batch;                        // of the ping-pong kernel
+  const int64_t waves = (ctas + sms - 1) / sms;
+  if (ctas * 100 >= waves * sms * 93) return true;
+  if (waves > 1 && seq_kv < 2048) return false;
+  const int64_t pairs = tiles * heads * batch;                       // CTAs of the pair kernel, two per SM
+  const int64_t rest = pairs % (2 * sms);
+  const double pair_cost = static_cast<double>(pairs / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
+  return static_cast<double>(waves) * static_cast<double>(2 * items) < pair_cost * 1.03 * static_cast<double>(tiles);
+}
+
 // MFX_FMHA_KERNEL=pingpong | pair overrides the choice.
 static bool use_pingpong(int64_t seq, int64_t seq_kv, int64_t batch, int heads) {
   const char* e = getenv("MFX_FMHA_KERNEL");
   if (e && e[0] == 'p' && e[1] == 'i') return true;
   if (e && e[0] == 'p' && e[1] == 'a') return false;
-  const int64_t sms = device_sm_count();
-  const int64_t tiles = (seq + BQ - 1) / BQ, items = (tiles + 1) / 2;
-  const int64_t pairs = tiles * heads * batch;                       // CTAs of the pair kernel, two per SM
-  const int64_t waves = (items * heads * batch + sms - 1) / sms;     // of ping-pong CTAs
-  if (seq_kv < (waves > 1 ? 2048 : 1024)) return false;
-  const int64_t rest = pairs % (2 * sms);
-  const double pair_cost = static_cast<double>(pairs / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
-  return static_cast<double>(waves) * static_cast<double>(2 * items) < pair_cost * 1.03 * static_cast<double>(tiles);
+  return pingpong_pays(seq, seq_kv, batch, heads);
 }
 
 // Arguments of one attention call (the C entry points fill it).
@@ -995,6 +1004,12 @@ int mfx_fmha_ex(const mfx_fmha_args* a, void* stream) {
                           a->seq_q, a->seq_kv, a->batch, a->heads, a->kv_heads, a->scale, a->key_bias,
                           a->bias_batch_stride, a->out, a->out_row_stride, a->out_batch_stride};
   return mfx::attn::run(c, static_cast<cudaStream_t>(stream));
+}
+
+int mfx_fmha_query_tiles(int64_t seq_q, int64_t seq_kv, int64_t batch, int heads) {
+  if (seq_q <= 0 || seq_kv <= 0 || batch <= 0 || heads <= 0) return 0;
+  if (seq_q > (1 << 24) || seq_kv > (1 << 24) || batch > 65535 || heads > 65535) return 0;
+  return mfx::attn::pingpong_pays(seq_q, seq_kv, batch, heads) ? 2 : 1;
 }
 
 }  // extern "C"

@@ -1,6 +1,6 @@
 """Attention calls on both sides of the choice between the two kernels (half a wave, one wave, a part-filled second and
 third wave, an odd number of 128-query tiles, the shortest key lengths of either), with and without a key-padding bias,
-against float64. The bound is the bf16 rounding of P and of the output (2^-9 each, relative) over averages of values:
+against float64; which kernel a size takes is asserted first. The bound is the bf16 rounding of P and of the output (2^-9 each, relative) over averages of values:
 5e-3 in the 2-norm."""
 import pytest
 import torch
@@ -9,11 +9,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bias", [False, True])
-@pytest.mark.parametrize("batch,heads,seq", [(1, 18, 1024), (1, 20, 1024), (1, 20, 1023), (1, 30, 2047), (1, 30, 2048),
-                                             (1, 12, 2400), (2, 6, 2500), (1, 24, 4096)])
-def test_both_sides_of_the_choice(lib_built, bias, batch, heads, seq):
-    from mflux_b200 import ops
+@pytest.mark.parametrize("batch,heads,seq,tiles", [(1, 18, 1024, 1), (1, 20, 1024, 2), (1, 20, 1023, 1), (1, 30, 2047, 1),
+                                                   (1, 30, 2048, 2), (1, 12, 2400, 1), (2, 6, 2500, 2), (1, 24, 4096, 2),
+                                                   (18, 4, 1024, 2), (2, 24, 1536, 2)])
+def test_both_sides_of_the_choice(lib_built, monkeypatch, bias, batch, heads, seq, tiles):
+    from mflux_b200 import _lib, ops
 
+    monkeypatch.delenv("MFX_FMHA_KERNEL", raising=False)
+    assert _lib.load().mfx_fmha_query_tiles(seq, seq, batch, heads) == tiles
     g = torch.Generator(device="cuda").manual_seed(heads * seq)
     qkv = torch.randn(batch, seq, 3 * heads * 128, device="cuda", generator=g).to(torch.bfloat16)
     kb = None

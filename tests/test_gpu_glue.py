@@ -207,10 +207,11 @@ def test_fmha_bias_argument_validation(lib_built):
 def test_fmha_default_kernel_choice_matches_both(lib_built, monkeypatch):
     """With the variable unset the library chooses by shape (here a grid that fills whole waves of CTAs, so the
     two-query-tile kernel); either way the result is the oracle's."""
-    from mflux_b200 import ops
+    from mflux_b200 import _lib, ops
 
     monkeypatch.delenv("MFX_FMHA_KERNEL", raising=False)
     b, s, heads = 37, 1024, 4   # 4 x 4 x 37 = 592 CTAs of two query tiles = exactly 4 waves of 148
+    assert _lib.load().mfx_fmha_query_tiles(s, s, b, heads) == 2
     g = _g(5)
     qkv = torch.randn(b, s, 3 * heads * 128, generator=g).to(torch.bfloat16).cuda()
     out = ops.fmha(qkv, heads)
