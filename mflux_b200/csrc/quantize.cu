@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
     for (int i = 0; i < 16; ++i) q[i] = exact_code(__fsub_rn(v[i], bias), scale, n_bins);
   }
   if (!active) return;
-  if (BITS == 4) {
+  if constexpr (BITS == 4) {
     // four codes at a time as an exact float below 2^16
     uint32_t half[4];
 #pragma unroll
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
       half[i] = static_cast<uint32_t>(fmaf(fmaf(fmaf(q[4 * i + 3], 16.0f, q[4 * i + 2]), 16.0f, q[4 * i + 1]), 16.0f,
                                            q[4 * i]));
     reinterpret_cast<uint2*>(wq)[g * 4 + sub] = make_uint2(half[0] | (half[1] << 16), half[2] | (half[3] << 16));
-  } else if (BITS == 8) {
+  } else if constexpr (BITS == 8) {
     uint32_t word[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -160,55 +160,65 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
   }
 }
 
-// One thread: 16 consecutive outputs of a row.
-template <typename SB, typename OUT, int BITS>
+// One thread: V (8 or 16) consecutive outputs of a row.
+template <typename SB, typename OUT, int BITS, int V>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restrict__ wq,
                                                          const SB* __restrict__ scales,
                                                          const SB* __restrict__ biases, int64_t n_chunks,
                                                          OUT* __restrict__ out) {
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= n_chunks) return;
-  const int64_t g = tid >> 2;
+  const int64_t g = tid / (64 / V);
   const float s = to_f32<SB>(scales[g]);
   const float b = to_f32<SB>(biases[g]);
-  uint32_t codes[16];
-  if (BITS == 4) {
-    const uint2 words = __ldg(reinterpret_cast<const uint2*>(wq) + tid);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      codes[i] = (words.x >> (4 * i)) & 0xF;
-      codes[8 + i] = (words.y >> (4 * i)) & 0xF;
+  uint32_t codes[V];
+  if constexpr (BITS == 4 || BITS == 8) {
+    constexpr int WORDS = V * BITS / 32;
+    uint32_t words[WORDS];
+    if constexpr (WORDS == 1) {
+      words[0] = __ldg(wq + tid);
+    } else if constexpr (WORDS == 2) {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(wq) + tid);
+      words[0] = v.x; words[1] = v.y;
+    } else {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(wq) + tid);
+      words[0] = v.x; words[1] = v.y; words[2] = v.z; words[3] = v.w;
     }
-  } else if (BITS == 8) {
-    const uint4 words = __ldg(reinterpret_cast<const uint4*>(wq) + tid);
-    const uint32_t w4[4] = {words.x, words.y, words.z, words.w};
 #pragma unroll
-    for (int i = 0; i < 16; ++i) codes[i] = (w4[i >> 2] >> (8 * (i & 3))) & 0xFF;
+    for (int i = 0; i < V; ++i) codes[i] = (words[i * BITS / 32] >> (i * BITS % 32)) & ((1u << BITS) - 1u);
   } else {
-    const uint16_t* src = reinterpret_cast<const uint16_t*>(wq) + tid * BITS;
-    unsigned long long w0 = 0, w1 = 0;
+    // eight codes are BITS bytes of the bit stream, sixteen are BITS 16-bit words at an even address
+    unsigned long long eight[V / 8];
+    if constexpr (V == 8) {
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(wq) + tid * BITS;
+      eight[0] = 0;
 #pragma unroll
-    for (int i = 0; i < BITS; ++i) {
-      const unsigned long long v = __ldg(src + i);
-      if (i < 4) w0 |= v << (16 * i);
-      else w1 |= v << (16 * (i & 3));
-    }
-    const unsigned long long hi = (w0 >> (8 * BITS)) | (w1 << (64 - 8 * BITS));
+      for (int i = 0; i < BITS; ++i) eight[0] |= static_cast<unsigned long long>(__ldg(src + i)) << (8 * i);
+    } else {
+      const uint16_t* src = reinterpret_cast<const uint16_t*>(wq) + tid * BITS;
+      unsigned long long w0 = 0, w1 = 0;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      codes[i] = static_cast<uint32_t>(w0 >> (BITS * i)) & ((1u << BITS) - 1u);
-      codes[8 + i] = static_cast<uint32_t>(hi >> (BITS * i)) & ((1u << BITS) - 1u);
+      for (int i = 0; i < BITS; ++i) {
+        const unsigned long long v = __ldg(src + i);
+        if (i < 4) w0 |= v << (16 * i);
+        else w1 |= v << (16 * (i & 3));
+      }
+      eight[0] = w0;
+      eight[1] = (w0 >> (8 * BITS)) | (w1 << (64 - 8 * BITS));
     }
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+      codes[i] = static_cast<uint32_t>(eight[i / 8] >> (BITS * (i % 8))) & ((1u << BITS) - 1u);
   }
-  __align__(16) OUT res[16];
+  __align__(16) OUT res[V];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
+  for (int i = 0; i < V; ++i) {
     const float c = __uint_as_float(0x4B000000u | codes[i]) - 8388608.0f;   // the code under the exponent of 2^23
     res[i] = from_f32<OUT>(__fadd_rn(__fmul_rn(c, s), b));
   }
-  uint4* dst = reinterpret_cast<uint4*>(out + tid * 16);
+  uint4* dst = reinterpret_cast<uint4*>(out + tid * V);
 #pragma unroll
-  for (int i = 0; i < static_cast<int>(sizeof(OUT)); ++i) dst[i] = reinterpret_cast<const uint4*>(res)[i];
+  for (int i = 0; i < V * static_cast<int>(sizeof(OUT)) / 16; ++i) dst[i] = reinterpret_cast<const uint4*>(res)[i];
 }
 
 template <typename T>
@@ -239,19 +249,34 @@ int launch_quantize(const void* w, int64_t n_groups, int bits, int qmode, uint32
   return MFX_OK;
 }
 
+template <typename SB, typename OUT, int BITS>
+void launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* biases, int64_t values, OUT* out,
+                            cudaStream_t st) {
+  auto blocks = [&](int v) { return static_cast<unsigned>((values / v + 255) / 256); };
+  // Sixteen values a thread halve the threads and the scale loads, which pays once the output fills the GPU many times
+  // over; below 32 MB fewer threads hide less of a trip to memory, and at 5 and 6 bits the gathering of ten or twelve
+  // bytes from 16-bit words outweighs it in 16-bit outputs. Buffers past L2, us, 8 / 16 values: to bf16, 12288 x 3072, 4 bits
+  // 22.0 / 21.6, 8 bits 22.8 / 21.9, 6 bits 25.4 / 26.9; 3072 x 3072, 4 bits 6.8 / 7.2, 6 bits 8.1 / 9.0; to float32,
+  // 3072 x 3072, 4 bits 13.1 / 12.7, 6 bits 14.8 / 13.6; 1024 x 3072, 3 bits 5.9 / 6.1.
+  constexpr bool few = sizeof(OUT) == 2 && (BITS == 5 || BITS == 6);
+  if (!few && values * static_cast<int64_t>(sizeof(OUT)) >= (32 << 20))
+    dequantize_kernel<SB, OUT, BITS, 16><<<blocks(16), 256, 0, st>>>(wq, scales, biases, values / 16, out);
+  else
+    dequantize_kernel<SB, OUT, BITS, 8><<<blocks(8), 256, 0, st>>>(wq, scales, biases, values / 8, out);
+}
+
 template <typename SB, typename OUT>
-int launch_dequantize(const uint32_t* wq, const void* scales, const void* biases, int64_t n_chunks, int bits,
+int launch_dequantize(const uint32_t* wq, const void* scales, const void* biases, int64_t values, int bits,
                       void* out, cudaStream_t st) {
-  const unsigned blocks = static_cast<unsigned>((n_chunks + 255) / 256);
   const SB* sp = static_cast<const SB*>(scales);
   const SB* bp = static_cast<const SB*>(biases);
   OUT* op = static_cast<OUT*>(out);
   switch (bits) {
-    case 3: dequantize_kernel<SB, OUT, 3><<<blocks, 256, 0, st>>>(wq, sp, bp, n_chunks, op); break;
-    case 4: dequantize_kernel<SB, OUT, 4><<<blocks, 256, 0, st>>>(wq, sp, bp, n_chunks, op); break;
-    case 5: dequantize_kernel<SB, OUT, 5><<<blocks, 256, 0, st>>>(wq, sp, bp, n_chunks, op); break;
-    case 6: dequantize_kernel<SB, OUT, 6><<<blocks, 256, 0, st>>>(wq, sp, bp, n_chunks, op); break;
-    case 8: dequantize_kernel<SB, OUT, 8><<<blocks, 256, 0, st>>>(wq, sp, bp, n_chunks, op); break;
+    case 3: launch_dequantize_bits<SB, OUT, 3>(wq, sp, bp, values, op, st); break;
+    case 4: launch_dequantize_bits<SB, OUT, 4>(wq, sp, bp, values, op, st); break;
+    case 5: launch_dequantize_bits<SB, OUT, 5>(wq, sp, bp, values, op, st); break;
+    case 6: launch_dequantize_bits<SB, OUT, 6>(wq, sp, bp, values, op, st); break;
+    case 8: launch_dequantize_bits<SB, OUT, 8>(wq, sp, bp, values, op, st); break;
     default: return MFX_ERR_UNSUPPORTED_BITS;
   }
   MFX_CUDA_TRY(cudaGetLastError());
@@ -259,12 +284,12 @@ int launch_dequantize(const uint32_t* wq, const void* scales, const void* biases
 }
 
 template <typename SB>
-int dispatch_dequant_out(const uint32_t* wq, const void* scales, const void* biases, int64_t n_chunks, int bits,
+int dispatch_dequant_out(const uint32_t* wq, const void* scales, const void* biases, int64_t values, int bits,
                          void* out, int out_dtype, cudaStream_t st) {
   switch (out_dtype) {
-    case MFX_F32: return launch_dequantize<SB, float>(wq, scales, biases, n_chunks, bits, out, st);
-    case MFX_BF16: return launch_dequantize<SB, __nv_bfloat16>(wq, scales, biases, n_chunks, bits, out, st);
-    case MFX_F16: return launch_dequantize<SB, __half>(wq, scales, biases, n_chunks, bits, out, st);
+    case MFX_F32: return launch_dequantize<SB, float>(wq, scales, biases, values, bits, out, st);
+    case MFX_BF16: return launch_dequantize<SB, __nv_bfloat16>(wq, scales, biases, values, bits, out, st);
+    case MFX_F16: return launch_dequantize<SB, __half>(wq, scales, biases, values, bits, out, st);
     default: return MFX_ERR_DTYPE;
   }
 }
@@ -303,12 +328,12 @@ int mfx_dequantize_affine(const uint32_t* wq, const void* scales, const void* bi
   if (!aligned16(wq) || !aligned16(out)) return MFX_ERR_ALIGN;
   if (int rc = check_arch()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t n_chunks = N * K / PER_THREAD;
+  const int64_t values = N * K;
   switch (sb_dtype) {
-    case MFX_F32: return dispatch_dequant_out<float>(wq, scales, biases, n_chunks, bits, out, out_dtype, st);
+    case MFX_F32: return dispatch_dequant_out<float>(wq, scales, biases, values, bits, out, out_dtype, st);
     case MFX_BF16:
-      return dispatch_dequant_out<__nv_bfloat16>(wq, scales, biases, n_chunks, bits, out, out_dtype, st);
-    default: return dispatch_dequant_out<__half>(wq, scales, biases, n_chunks, bits, out, out_dtype, st);
+      return dispatch_dequant_out<__nv_bfloat16>(wq, scales, biases, values, bits, out, out_dtype, st);
+    default: return dispatch_dequant_out<__half>(wq, scales, biases, values, bits, out, out_dtype, st);
   }
 }
 
