@@ -199,14 +199,18 @@ typedef struct mfx_qlinear_args {
 int mfx_qlinear_ex(const mfx_qlinear_args* args /* host */, void* stream);
 
 /* mfx_qlinear_ex with scratch for the decoded weight. With at least 2 N K bytes (256-byte aligned device memory,
- * overwritten) the weight is decoded once to bf16 and contracted from there, in two launches; with less, for at most
- * 16 rows and for MFX_EPI_PEER_SCATTER this is mfx_qlinear_ex. The results are the same bit for bit, but for the place
- * of the low-rank products in the float32 accumulation. mfx_qlinear_scratch_bytes_batch says how many bytes a call
+ * overwritten) the weight is decoded once to bf16 and contracted from there, in two launches; with less, for one sample
+ * of at most 16 rows with no epilogue beyond SiLU and no low-rank term, and for MFX_EPI_PEER_SCATTER this is
+ * mfx_qlinear_ex. The results are the same bit for bit. mfx_qlinear_scratch_bytes_batch says how many bytes a call
  * over `batch` samples of `rows` rows should pass: 2 N K where that form is the faster one, 0 elsewhere;
  * mfx_qlinear_scratch_bytes is that for one sample. */
 size_t mfx_qlinear_scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits);
 size_t mfx_qlinear_scratch_bytes_batch(int64_t rows, int64_t batch, int64_t N, int64_t K, int bits);
 int mfx_qlinear_ex_scratch(const mfx_qlinear_args* args /* host */, void* scratch, size_t scratch_bytes, void* stream);
+
+/* Output columns of a tile (256, 192 or 128) in a one-launch call of more than 16 rows; 0 for sizes that are not valid.
+ * The width changes the time, not the result. */
+int mfx_qlinear_tile_columns(int64_t rows, int64_t batch, int64_t N, int bits);
 
 /* The elementwise half of a tensor-parallel block on the rows this rank owns, fused with both collectives:
  *   wait until rs_flags[r] >= rs_target for every rank r (the partials of the preceding row-split linears),

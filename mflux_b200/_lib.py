@@ -213,6 +213,7 @@ SIGNATURES = {
     ),
     "mfx_qlinear_scratch_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int64, c_int]),
     "mfx_qlinear_scratch_bytes_batch": (ctypes.c_size_t, [c_int64, c_int64, c_int64, c_int64, c_int]),
+    "mfx_qlinear_tile_columns": (c_int, [c_int64, c_int64, c_int64, c_int]),
     "mfx_qlinear_ex_scratch": (c_int, [ctypes.POINTER(QLinearArgs), c_void_p, ctypes.c_size_t, c_void_p]),
     "mfx_qlinear_prepared_bytes": (ctypes.c_size_t, [c_int64, c_int64, c_int, c_int]),
     "mfx_qlinear_prepare": (

@@ -613,6 +613,9 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   // teams take turns. 4 bits, M 4096, N 12288, K 3072, GELU: 264 -> 227 us; M 4608, N 3072, K 15360: 322 -> 297 us; M
   // 512, N 3072, K 12288: 70 -> 62 us. Eight-bit tiles leave room for two B stages, where a second team has nowhere to
   // write ahead and costs 2-3 % (M 1613, N 20480, K 3840: 212 -> 218 us).
+  // 768 threads leave a thread 80 registers. ptxas spills in 38 of the 158 instantiations, all with two teams: 32 to 44
+  // bytes stored (68 to 88 loaded) per 32 columns of the float32 gated residual, whose four loads in flight do not fit
+  // beside the accumulator (qmm_epilogue.cuh), 4 bytes in the bf16 form of it and in the GELUs with float32 output.
   constexpr int NDQ = 8;
   constexpr int TEAMS = SD > 2 ? 2 : 1;
   constexpr int NUM_THREADS = (FIXED_WARPS + TEAMS * NDQ) * 32;
@@ -1057,6 +1060,14 @@ int mfx_qlinear_ex_scratch(const mfx_qlinear_args* args, void* scratch, size_t s
 
 size_t mfx_qlinear_scratch_bytes(int64_t rows, int64_t N, int64_t K, int bits) {
   return mfx_qlinear_scratch_bytes_batch(rows, 1, N, K, bits);
+}
+
+int mfx_qlinear_tile_columns(int64_t rows, int64_t batch, int64_t N, int bits) {
+  if (rows <= 0 || batch <= 0 || N <= 0 || !mfx::valid_bits(bits)) return 0;
+  if (rows > (1 << 30) || batch > (1 << 20) || N > (1 << 30)) return 0;
+  const int64_t m_tiles = mfx::qmm::row_tiles(rows, batch);
+  if (m_tiles > (1 << 30)) return 0;
+  return mfx::qmm::tile_width(m_tiles, N, mfx::device_sm_count() / 2, mfx::kernel_bits(bits));
 }
 
 size_t mfx_qlinear_scratch_bytes_batch(int64_t rows, int64_t batch, int64_t N, int64_t K, int bits) {

@@ -1,5 +1,5 @@
-// Device helpers shared by the two tensor-core quantized-matmul kernels (qmm.cu, qmm_t.cu): scalar loads by dtype
-// code, the 4- and 8-bit dequantizers over the prepared code layout, and the epilogue activations.
+// Device helpers shared by the tensor-core quantized-matmul kernels (qmm.cu, qmm_dense.cu, qmm_t.cu): scalar loads by
+// dtype code, the 4- and 8-bit dequantizers over the prepared code layout, and the epilogue activations.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

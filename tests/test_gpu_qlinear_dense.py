@@ -157,3 +157,32 @@ def test_no_room_for_scratch_runs_without_it(lib_built, monkeypatch):
         assert torch.equal(ops.qlinear(x, wq, s, bi, None, bits=4, prepared=prep), want)
     assert ops.LAUNCHES[0] - before == 3
     assert torch.cuda.memory_stats()["num_ooms"] - refused == 1      # asked once, not on every call
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("epi", [None, "gelu", "gate_residual", "lora"])
+def test_several_bands_and_three_tiles_per_pair(lib_built, monkeypatch, bits, epi):
+    """A bf16 weight past one band (37 column tiles, 19 and 18 to a band) and 222 tiles for 74 CTA pairs: accumulators,
+    ring and bias vectors in turn. All rows, to the bit against the one-launch kernel."""
+    from mflux_b200 import ops
+
+    m, n, k = 6 * 256 - 50, 37 * 256 - 248, 3072
+    g = torch.Generator(device="cuda").manual_seed(bits)
+    w = (torch.randn(n, k, generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    x = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(n, generator=g, device="cuda")
+    wq, s, bi = ops.quantize_affine(w, 64, bits)
+    kw = {"out_dtype": torch.float32}
+    if epi == "gate_residual":
+        kw = {"epilogue": epi, "gate": b[None], "residual": torch.randn(m, n, generator=g, device="cuda")}
+    elif epi == "lora":
+        t = torch.zeros(m, 128, device="cuda", dtype=torch.bfloat16)
+        lb = torch.zeros(n, 128, device="cuda", dtype=torch.bfloat16)
+        t[:, :72] = torch.randn(m, 72, generator=g, device="cuda")
+        lb[:, :72] = torch.randn(n, 72, generator=g, device="cuda") * 0.05
+        kw |= {"lora_t": t, "lora_b": lb, "lora_r": 72}
+    elif epi:
+        kw |= {"epilogue": epi}
+    two, one = _both(monkeypatch, lambda: ops.qlinear(x, wq, s, bi, b, bits=bits, **kw), n, k)
+    assert ops.poll_device_status() == 0
+    assert torch.isfinite(two).all() and torch.equal(two, one)

@@ -42,3 +42,17 @@ def test_rows_of_short_samples_are_counted_in_their_own_tiles(lib_built):
                                   (64, 1, 64, 64, 7), (1 << 40, 1, 64, 64, 4), (1 << 30, 1 << 20, 1 << 30, 64, 8)])
 def test_sizes_that_a_call_refuses_need_no_scratch(lib_built, args):
     assert _lib.load().mfx_qlinear_scratch_bytes_batch(*args) == 0
+
+
+@pytest.mark.parametrize("rows,batch,n,bits,width", [
+    (512, 1, 3072, 4, 128), (512, 1, 3072, 8, 128),        # few tiles: 61.9 / 55.0 / 41.6 us at 256 / 192 / 128 (K 12288)
+    (1613, 1, 3840, 8, 192),                               # 128 / 113 / 118 us (K 10240)
+    (1613, 1, 20480, 4, 256), (1613, 1, 20480, 8, 256),    # 191 / 210 / 227 and 218 / 226 / 234 us (K 3840)
+    (16, 3, 64, 4, 128)])
+def test_tile_width_by_waves(lib_built, rows, batch, n, bits, width):
+    assert _lib.load().mfx_qlinear_tile_columns(rows, batch, n, bits) == width
+
+
+@pytest.mark.parametrize("args", [(0, 1, 64, 4), (64, 0, 64, 4), (64, 1, 0, 4), (64, 1, 64, 7), (1 << 40, 1, 64, 4)])
+def test_no_tile_width_for_sizes_that_a_call_refuses(lib_built, args):
+    assert _lib.load().mfx_qlinear_tile_columns(*args) == 0
