@@ -6,6 +6,7 @@ live on a CUDA device and the library must be built.
 """
 from __future__ import annotations
 
+import os
 from ctypes import byref, c_int, c_void_p
 from ctypes import pointer as ctypes_pointer
 from functools import lru_cache
@@ -77,6 +78,8 @@ def _prepared_bytes(n: int, k: int, bits: int, group_size: int) -> int:
 
 @lru_cache(maxsize=4096)
 def _scratch_bytes(rows: int, batch: int, n: int, k: int, bits: int) -> int:
+    if os.environ.get("MFX_QMM_KERNEL") == "tmem":   # that kernel takes the calls, without scratch
+        return 0
     return _lib.load().mfx_qlinear_scratch_bytes_batch(rows, batch, n, k, bits)
 
 

@@ -1,8 +1,15 @@
 """Which form of the quantized linear a call takes, by the size rules of the library (host code; 74 CTA pairs, as on a
 B200, also where no device is present)."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 
 from mflux_b200 import _lib
+
+ROOT = Path(__file__).resolve().parent.parent
 
 
 # (rows, samples, N, K, bits), measured on a B200, one launch / two launches, us
@@ -56,3 +63,13 @@ def test_tile_width_by_waves(lib_built, rows, batch, n, bits, width):
 @pytest.mark.parametrize("args", [(0, 1, 64, 4), (64, 0, 64, 4), (64, 1, 0, 4), (64, 1, 64, 7), (1 << 40, 1, 64, 4)])
 def test_no_tile_width_for_sizes_that_a_call_refuses(lib_built, args):
     assert _lib.load().mfx_qlinear_tile_columns(*args) == 0
+
+
+def test_no_scratch_where_the_tensor_memory_kernel_takes_the_calls(lib_built):
+    """The scratch would be allocated for nothing and counted as a launch. MFX_QMM_KERNEL is read once per process."""
+    code = ("from mflux_b200 import ops; "
+            "print(ops._scratch_bytes(18432, 1, 3072, 3072, 4), ops._scratch_bytes(4608, 16, 9216, 3072, 8))")
+    for kernel, want in (("tmem", "0 0"), ("", f"{2 * 3072 * 3072} {2 * 9216 * 3072}")):
+        env = {**os.environ, "MFX_QMM_KERNEL": kernel}
+        out = subprocess.run([sys.executable, "-c", code], env=env, cwd=ROOT, capture_output=True, text=True, check=True)
+        assert out.stdout.strip() == want
