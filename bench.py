@@ -36,17 +36,19 @@ TRAFFIC_RECORD = ROOT / "profiles" / "qmm_flux_step_dram_traffic.json"
 
 
 def recorded_traffic():
-    """Mean DRAM bytes (read + write) per quantized-matmul launch of the full flux step, from the committed record
-    of an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum on the reduced-depth model at the same per-GPU
-    batch, weighted by the block counts of the full model). The record names the command that made it and the
-    SHA-256 of the kernel source it was taken on; it is reported only while that source is unchanged."""
+    """Mean DRAM bytes (read + write) per quantized linear of the full flux step (decode and contraction counted
+    together where a linear takes two launches), from the committed record of an ncu capture
+    (dram__bytes_read.sum + dram__bytes_write.sum on the reduced-depth model at the same per-GPU batch, weighted by
+    the block counts of the full model). The record names the command that made it and the SHA-256 of the kernel
+    sources it was taken on; it is reported only while those are unchanged."""
     import hashlib
 
     if not TRAFFIC_RECORD.exists():
         return None
     rec = json.loads(TRAFFIC_RECORD.read_text())
-    src = ROOT / "mflux_b200" / "csrc" / "qmm.cu"
-    if hashlib.sha256(src.read_bytes()).hexdigest() != rec.get("qmm_cu_sha256"):
+    csrc = ROOT / "mflux_b200" / "csrc"
+    sources = b"".join((csrc / name).read_bytes() for name in ("qmm.cu", "qmm_dense.cu"))
+    if hashlib.sha256(sources).hexdigest() != rec.get("qmm_sources_sha256"):
         return None
     return rec.get("dram_bytes_per_launch")
 
@@ -747,13 +749,14 @@ def main():
                     "d2h_bytes_per_step": out_h.numel() * out_h.element_size()},
             "gpu_launches": launches,
             "clocks": clocks,
-            "roofline": {"bound": "tensor", "kernel": "qmm_kernel (quantized linear)", "achieved": achieved,
+            "roofline": {"bound": "tensor", "kernel": "qmm_kernel, or decode_kernel + dense_kernel from where two launches pay "
+                                   "(quantized linear)", "achieved": achieved,
                          "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                          "peak_kind": peak_kind, "burst_peak": burst,
                          "frac_of_burst": achieved / burst if burst else None,
                          "tflops_per_sm_mhz": achieved / sm_mhz if sm_mhz else None, "launches": q_n,
                          "share_of_step_time": (q_ms / trace_steps) / step_ms if ms > 0 else None, "traffic": traffic,
-                         "traffic_unit": "DRAM bytes per launch, mean over the step's launches (ncu record under "
+                         "traffic_unit": "DRAM bytes per quantized linear, mean over the step's (ncu record under "
                                          "profiles/, null when the kernel source changed since the capture)"},
             "roofline_attention": {"bound": "tensor", "kernel": "attn::sdpa_pingpong_kernel / attn::sdpa_pair_kernel (flash attention, head dim 128)",
                                    "achieved": a_achieved, "peak": peak, "unit": "TFLOP/s",
