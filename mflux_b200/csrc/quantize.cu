@@ -213,7 +213,8 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
   __align__(16) OUT res[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) {
-    const float c = __uint_as_float(0x4B000000u | codes[i]) - 8388608.0f;   // the code under the exponent of 2^23
+    // sixteen conversions in a row wait for the converter: the code under the exponent of 2^23 instead
+    const float c = V == 8 ? static_cast<float>(codes[i]) : __uint_as_float(0x4B000000u | codes[i]) - 8388608.0f;
     res[i] = from_f32<OUT>(__fadd_rn(__fmul_rn(c, s), b));
   }
   uint4* dst = reinterpret_cast<uint4*>(out + tid * V);
@@ -254,12 +255,13 @@ void launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* bias
                             cudaStream_t st) {
   auto blocks = [&](int v) { return static_cast<unsigned>((values / v + 255) / 256); };
   // Sixteen values a thread halve the threads and the scale loads, which pays once the output fills the GPU many times
-  // over; below 32 MB fewer threads hide less of a trip to memory, and at 5 and 6 bits the gathering of ten or twelve
-  // bytes from 16-bit words outweighs it in 16-bit outputs. Buffers past L2, us, 8 / 16 values: to bf16, 12288 x 3072, 4 bits
-  // 22.0 / 21.6, 8 bits 22.8 / 21.9, 6 bits 25.4 / 26.9; 3072 x 3072, 4 bits 6.8 / 7.2, 6 bits 8.1 / 9.0; to float32,
-  // 3072 x 3072, 4 bits 13.1 / 12.7, 6 bits 14.8 / 13.6; 1024 x 3072, 3 bits 5.9 / 6.1.
+  // over (8 M values of float32, 32 M of 16 bits); below that fewer threads hide less of a trip to memory, and at 5 and 6
+  // bits the gathering of ten or twelve bytes from 16-bit words outweighs it in 16-bit outputs. Buffers past L2, us, 8 / 16
+  // values: to bf16, 12288 x 3072, 4 bits 22.4 / 22.0, 8 bits 22.9 / 21.9, 6 bits 25.5 / 26.9; 6144 x 3072, 3 bits 12.1 /
+  // 12.5; 3072 x 3072, 4 bits 6.9 / 7.2, 6 bits 8.1 / 9.0; to float32, 3072 x 3072, 4 bits 12.9 / 12.7, 6 bits 14.8 / 13.5;
+  // 1024 x 3072, 3 bits 5.9 / 6.0; 256 x 256 2.1 / 2.3.
   constexpr bool few = sizeof(OUT) == 2 && (BITS == 5 || BITS == 6);
-  if (!few && values * static_cast<int64_t>(sizeof(OUT)) >= (32 << 20))
+  if (!few && values >= (sizeof(OUT) == 4 ? 8 << 20 : 32 << 20))
     dequantize_kernel<SB, OUT, BITS, 16><<<blocks(16), 256, 0, st>>>(wq, scales, biases, values / 16, out);
   else
     dequantize_kernel<SB, OUT, BITS, 8><<<blocks(8), 256, 0, st>>>(wq, scales, biases, values / 8, out);
