@@ -161,15 +161,18 @@ class QuantizedLinear(Module):
     def output_dims(self) -> int:
         return self.weight.shape[0]
 
-    def _tensor(self, name: str) -> torch.Tensor | None:
-        """A tensor of the layer by name: past Module.__getattr__ where it is a plain parameter (this runs on every
-        call), through the attribute where it is not (parametrized, pruned or replaced by a plain tensor)."""
+    def _tensors(self):
+        """weight, scales, biases and bias: past Module.__getattr__ where all are plain parameters (this runs on every
+        call), through the attributes where one is not (parametrized, pruned or replaced by a plain tensor)."""
         p = self._parameters
-        return p[name] if name in p else getattr(self, name)
+        try:
+            return p["weight"], p["scales"], p["biases"], p["bias"]
+        except KeyError:
+            return self.weight, self.scales, self.biases, self.bias
 
     def prepared(self) -> torch.Tensor:
         """Kernel-side form of the weight, built on first use and rebuilt if the tensors were replaced."""
-        w, s, b = self._tensor("weight"), self._tensor("scales"), self._tensor("biases")
+        w, s, b, _ = self._tensors()
         key = (w.data_ptr(), w._version, s.data_ptr(), s._version, b.data_ptr(), b._version)
         if self._prepared is None or self._prepared[0] != key:
             blob = ops.prepare_qlinear(self.weight.data, self.scales.data, self.biases.data, self.bits,
@@ -180,10 +183,10 @@ class QuantizedLinear(Module):
     def forward(self, x: torch.Tensor, *, epilogue: str | None = None, gate: torch.Tensor | None = None,
                 residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
-        t = self._tensor
-        return ops.qlinear(x, t("weight"), t("scales"), t("biases"), t("bias"), bits=self.bits,
-                           group_size=self.group_size, epilogue=epilogue, gate=gate, residual=residual, out=out,
-                           out_dtype=out_dtype, prepared=self.prepared())
+        weight, scales, biases, bias = self._tensors()
+        return ops.qlinear(x, weight, scales, biases, bias, bits=self.bits, group_size=self.group_size,
+                           epilogue=epilogue, gate=gate, residual=residual, out=out, out_dtype=out_dtype,
+                           prepared=self.prepared())
 
     def dequantize(self, dtype: torch.dtype | None = None) -> torch.Tensor:
         return ops.dequantize_affine(self.weight.data, self.scales.data, self.biases.data, self.group_size, self.bits,
