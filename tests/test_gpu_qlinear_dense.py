@@ -53,8 +53,7 @@ def test_matches_oracle_and_one_launch_kernel(lib_built, monkeypatch, bits, m, n
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_epilogues_samples_and_adapters(lib_built, monkeypatch, epi, lora, dtype):
     """Samples that are row slices of a longer buffer, each with its own ragged tile; ranks inside one slab and across
-    two and four. The kernels run adapter products in other groups: the bound is the float32 accumulation of K + rank
-    terms (2^-24 sqrt(K + r) relative, 1e-6) plus one rounding of the output."""
+    two and four. Both kernels run the adapters' products after the layer's, 16 columns at a time in the same order."""
     from mflux_b200 import ops
 
     bits, n, k, bsz, rows = 4, 528, 320, 3, 301
@@ -79,11 +78,7 @@ def test_epilogues_samples_and_adapters(lib_built, monkeypatch, epi, lora, dtype
     assert ops.poll_device_status() == 0
     assert got.shape == (bsz, rows, n // 2 if epi == "swiglu" else n) and got.dtype == dtype
     assert torch.isfinite(got.float()).all()
-    if lora == 0:
-        assert torch.equal(got, one)
-    else:
-        tol = 2 ** -8 if dtype == torch.bfloat16 else 4e-6
-        assert quant.rel_l2(got, one.float().cpu().numpy()) <= tol
+    assert torch.equal(got, one)
 
 
 def test_short_or_misaligned_scratch_is_not_used(lib_built):
