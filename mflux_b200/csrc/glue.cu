@@ -13,15 +13,10 @@
 #include <cuda_fp16.h>
 
 #include "host_util.cuh"
+#include "scalar.cuh"
 
 namespace mfx {
 namespace glue {
-
-__device__ __forceinline__ float ld_scalar(const void* p, int dtype, int64_t i) {
-  if (dtype == MFX_F32) return __ldg(static_cast<const float*>(p) + i);
-  if (dtype == MFX_BF16) return __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p) + i));
-  return __half2float(__ldg(static_cast<const __half*>(p) + i));
-}
 
 template <typename T>
 __device__ __forceinline__ void load8(const T* p, float (&v)[8]) {
@@ -87,7 +82,7 @@ __device__ __forceinline__ void load_vec(const void* p, int dtype, int64_t off, 
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < E; ++i) o[i] = ld_scalar(p, dtype, off + i);
+    for (int i = 0; i < E; ++i) o[i] = load_as_float(p, dtype, off + i);
   }
 }
 template <int E>
@@ -392,9 +387,9 @@ __global__ void __launch_bounds__(256) vec_sum_act_kernel(const void* a, const v
                                                           int act, void* out, int out_dtype, int64_t n) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float v = ld_scalar(a, in_dtype, i);
-  if (b) v += ld_scalar(b, in_dtype, i);
-  if (c) v += ld_scalar(c, in_dtype, i);
+  float v = load_as_float(a, in_dtype, i);
+  if (b) v += load_as_float(b, in_dtype, i);
+  if (c) v += load_as_float(c, in_dtype, i);
   if (act == 1) v = v / (1.0f + __expf(-v));
   else if (act == 2) v = tanhf(v);
   if (out_dtype == MFX_F32) static_cast<float*>(out)[i] = v;
@@ -406,7 +401,7 @@ __global__ void __launch_bounds__(256) euler_step_kernel(const void* latents, in
                                                          int noise_dtype, float dt, void* out, int64_t n) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float v = ld_scalar(latents, lat_dtype, i) + ld_scalar(noise, noise_dtype, i) * dt;
+  const float v = load_as_float(latents, lat_dtype, i) + load_as_float(noise, noise_dtype, i) * dt;
   if (lat_dtype == MFX_F32) static_cast<float*>(out)[i] = v;
   else if (lat_dtype == MFX_BF16) static_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
   else static_cast<__half*>(out)[i] = __float2half_rn(v);
@@ -437,8 +432,8 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const void* __restri
   float o[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float bv = bias ? ld_scalar(bias, bias_dtype, col + j) : 0.f;
-    const float gv = ld_scalar(gate, gate_dtype, b * gate_batch_stride + col + j);
+    const float bv = bias ? load_as_float(bias, bias_dtype, col + j) : 0.f;
+    const float gv = load_as_float(gate, gate_dtype, b * gate_batch_stride + col + j);
     o[j] = rv[j] + gv * (yv[j] + bv);
   }
   *reinterpret_cast<float4*>(out + roff) = make_float4(o[0], o[1], o[2], o[3]);
@@ -457,7 +452,7 @@ __global__ void __launch_bounds__(256) cfg_combine_kernel(const void* __restrict
   if (row >= rows) return;
   float sn = 0.f, sc = 0.f;
   for (int c = lane; c < C; c += 32) {
-    const float a = ld_scalar(n, dtype, row * C + c), b = ld_scalar(nn, dtype, row * C + c);
+    const float a = load_as_float(n, dtype, row * C + c), b = load_as_float(nn, dtype, row * C + c);
     const float comb = mode == 0 ? a + g * (a - b) : b + g * (a - b);
     sn += a * a;
     sc += comb * comb;
@@ -465,7 +460,7 @@ __global__ void __launch_bounds__(256) cfg_combine_kernel(const void* __restrict
   float ratio = 1.f;
   if (mode == 1) ratio = sqrtf(warp_sum(sn) + 1e-12f) / sqrtf(warp_sum(sc) + 1e-12f);
   for (int c = lane; c < C; c += 32) {
-    const float a = ld_scalar(n, dtype, row * C + c), b = ld_scalar(nn, dtype, row * C + c);
+    const float a = load_as_float(n, dtype, row * C + c), b = load_as_float(nn, dtype, row * C + c);
     const float comb = mode == 0 ? a + g * (a - b) : b + g * (a - b);
     out[row * C + c] = comb * ratio;
   }

@@ -493,9 +493,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
 #pragma unroll
       for (int c = et; c < BN; c += 128) {
         const int n = n0 + c;
-        bias_s[c] = (p.bias != nullptr && n < p.N) ? load_scalar(p.bias, p.bias_dtype, n) : 0.f;
+        bias_s[c] = (p.bias != nullptr && n < p.N) ? load_as_float(p.bias, p.bias_dtype, n) : 0.f;
         if (EPI == MFX_EPI_GATE_RESIDUAL)
-          gate_s[c] = (n < p.N) ? load_scalar(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
+          gate_s[c] = (n < p.N) ? load_as_float(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
       }
       named_bar_sync(1, 128);
       const bool row_ok = r < p.rows;
@@ -504,8 +504,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
                   (EPI == MFX_EPI_SWIGLU ? n0 / 2 : n0);
       const OUT* rrow = nullptr;
       if (EPI == MFX_EPI_GATE_RESIDUAL) {
+        // rows past the end point at the sample's first row: no address of theirs leaves the buffer, read or not
         rrow = static_cast<const OUT*>(p.residual) + b * p.res_batch_stride +
-               static_cast<int64_t>(r) * p.res_row_stride + n0;
+               static_cast<int64_t>(row_ok ? r : 0) * p.res_row_stride + n0;
         if (row_ok && p.K <= PREFETCH_K) prefetch_row(rrow, 0, BN, p.N - n0);
       }
       if (!mbar_wait_sleep(acc_full(a), aph, DEV_TIMEOUT_ACC_FULL)) {
@@ -665,8 +666,8 @@ __global__ void __launch_bounds__(256) pack_scales_kernel(const void* __restrict
     uint32_t v = 0;
     if (n < N && g < G) {
       const int64_t idx = static_cast<int64_t>(n) * G + g;
-      const __nv_bfloat16 sv = __float2bfloat16_rn(load_scalar(scales, sb_dtype, idx));
-      const __nv_bfloat16 bv = __float2bfloat16_rn(load_scalar(biases, sb_dtype, idx));
+      const __nv_bfloat16 sv = __float2bfloat16_rn(load_as_float(scales, sb_dtype, idx));
+      const __nv_bfloat16 bv = __float2bfloat16_rn(load_as_float(biases, sb_dtype, idx));
       v = static_cast<uint32_t>(__bfloat16_as_ushort(sv)) | (static_cast<uint32_t>(__bfloat16_as_ushort(bv)) << 16);
     }
     tile[ty + 8 * i][tx] = v;

@@ -6,15 +6,10 @@
 
 #include "host_util.cuh"
 #include "ptx.cuh"
+#include "scalar.cuh"
 
 namespace mfx {
 namespace qmm {
-
-__device__ __forceinline__ float load_scalar(const void* p, int dtype, int64_t i) {
-  if (dtype == MFX_F32) return __ldg(static_cast<const float*>(p) + i);
-  if (dtype == MFX_BF16) return __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p) + i));
-  return __half2float(__ldg(static_cast<const __half*>(p) + i));
-}
 
 // d = (a - magic) * s + b on packed 16-bit pairs: the subtraction is exact (small integers),
 // the fma rounds once.

@@ -24,8 +24,6 @@
 namespace mfx {
 namespace qmmd {
 
-using qmm::load_scalar;
-
 constexpr int BM = 128;                   // activation rows per CTA
 constexpr int BN = 256;                   // output columns per pair tile; each CTA loads 128 weight rows
 constexpr int BK = 64;                    // k per stage: one 128-byte swizzle row
@@ -212,9 +210,9 @@ dense_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
       float* bias_s = vec_s + a * BN;
       float* gate_s = vec_s + 2 * BN + a * BN;
       const int n = n0 + et;
-      bias_s[et] = (p.bias != nullptr && n < p.N) ? load_scalar(p.bias, p.bias_dtype, n) : 0.f;
+      bias_s[et] = (p.bias != nullptr && n < p.N) ? load_as_float(p.bias, p.bias_dtype, n) : 0.f;
       if (EPI == MFX_EPI_GATE_RESIDUAL)
-        gate_s[et] = (n < p.N) ? load_scalar(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
+        gate_s[et] = (n < p.N) ? load_as_float(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
       named_bar_sync(1, EPI_WARPS * 32);
       const bool row_ok = r < p.rows;
       // SwiGLU writes one value per (gate, up) column pair: output column n/2
@@ -223,8 +221,9 @@ dense_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
       const int c0 = half * (BN / 2), c1 = c0 + BN / 2;
       const OUT* rrow = nullptr;
       if (EPI == MFX_EPI_GATE_RESIDUAL) {
+        // rows past the end point at the sample's first row: no address of theirs leaves the buffer, read or not
         rrow = static_cast<const OUT*>(p.residual) + b * p.res_batch_stride +
-               static_cast<int64_t>(r) * p.res_row_stride + n0;
+               static_cast<int64_t>(row_ok ? r : 0) * p.res_row_stride + n0;
         if (row_ok && p.K <= qmm::PREFETCH_K) qmm::prefetch_row(rrow, c0, c1, p.N - n0);
       }
       if (!mbar_wait_sleep(acc_full(a), (it >> 1) & 1, DEV_TIMEOUT_ACC_FULL)) break;

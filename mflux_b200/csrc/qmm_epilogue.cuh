@@ -14,10 +14,11 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t (&v)[8]) {
                "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                : "memory");
 }
-// Not volatile: a thread reads each residual element once, before it writes that element, so the loads of a chunk may
-// all be issued ahead of its stores.
+// Volatile, so that it stays behind the tests for rows and columns past the end: to the compiler an asm statement that is
+// not is a pure function of its operands, which it may evaluate ahead of a branch, and the address would then be out of
+// the residual. The loads of a chunk stand ahead of its stores in the source.
 __device__ __forceinline__ void ld_global_32(const void* p, uint32_t (&v)[8]) {
-  asm("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "l"(p));
 }

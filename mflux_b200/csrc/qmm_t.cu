@@ -42,7 +42,6 @@ using qmm::dequant_w4;
 using qmm::dequant_w8_f32;
 using qmm::gelu_erf;
 using qmm::gelu_tanh;
-using qmm::load_scalar;
 using qmm::silu;
 
 constexpr int WR = 128;        // weight rows per CTA (tensor-memory lanes); 256 per pair
@@ -353,9 +352,9 @@ qmm_t_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
       const int t0 = (tm % p.tiles_m_per_sample) * NT;   // first token of the tile inside its sample
       const int n = tn * (2 * WR) + static_cast<int>(rank) * WR + q * 32 + lane;
       const bool n_ok = n < p.N;
-      const float bias_v = (p.bias != nullptr && n_ok) ? load_scalar(p.bias, p.bias_dtype, n) : 0.f;
+      const float bias_v = (p.bias != nullptr && n_ok) ? load_as_float(p.bias, p.bias_dtype, n) : 0.f;
       float gate_v = 0.f;
-      if (EPI == MFX_EPI_GATE_RESIDUAL && n_ok) gate_v = load_scalar(p.gate, p.gate_dtype, b * p.gate_batch_stride + n);
+      if (EPI == MFX_EPI_GATE_RESIDUAL && n_ok) gate_v = load_as_float(p.gate, p.gate_dtype, b * p.gate_batch_stride + n);
       // SwiGLU: lane pairs (2j, 2j+1) hold (gate, up) of output column n / 2
       const int n_out = EPI == MFX_EPI_SWIGLU ? (n >> 1) : n;
       const bool writer = n_ok && (EPI != MFX_EPI_SWIGLU || (lane & 1) == 0);

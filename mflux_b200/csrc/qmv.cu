@@ -18,6 +18,7 @@
 #include <cuda_fp16.h>
 
 #include "host_util.cuh"
+#include "scalar.cuh"
 #include "qmv.cuh"
 
 namespace mfx {
@@ -39,12 +40,6 @@ struct Params {
   int y_dtype;
   int64_t y_row_stride;
 };
-
-__device__ __forceinline__ float ld_bias(const void* p, int dtype, int i) {
-  if (dtype == MFX_F32) return __ldg(static_cast<const float*>(p) + i);
-  if (dtype == MFX_BF16) return __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(p) + i));
-  return __half2float(__ldg(static_cast<const __half*>(p) + i));
-}
 
 __device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b) {
   uint32_t d;
@@ -192,7 +187,7 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
     const int m = (l >> 2) + 8 * (i >> 1);
     const int n = n_base + 8 * r + 2 * (l & 3) + (i & 1);
     if (m < p.M && n < p.N) {
-      if (p.bias) v += ld_bias(p.bias, p.bias_dtype, n);
+      if (p.bias) v += load_as_float(p.bias, p.bias_dtype, n);
       if (p.epilogue == MFX_EPI_SILU) v = v / (1.0f + __expf(-v));
       if (p.y_dtype == MFX_F32) static_cast<float*>(p.y)[m * p.y_row_stride + n] = v;
       else static_cast<__nv_bfloat16*>(p.y)[m * p.y_row_stride + n] = __float2bfloat16_rn(v);
