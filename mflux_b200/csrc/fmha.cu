@@ -180,8 +180,22 @@ __device__ __forceinline__ void exp_chunk(const uint32_t (&s)[32], uint64_t scal
   }
 }
 
-// HAS_BIAS adds a per-key additive bias (a key-padding mask) to the scaled scores before the row maximum; the
-// variant without it is the plain kernel, instruction for instruction.
+// Whether any of the `keys` (at most 64, a multiple of 32 unless the sequence ends) biases from bp on is not zero. A
+// key-padding mask is zero for all but the padded keys, and a tile of zeros is the plain kernel's tile: the biased form
+// of it (a broadcast load per four keys and an unpacked multiply-add per score, in more registers than a thread has)
+// took the whole call to 706 TFLOP/s where the plain kernel has 1072 (2 x 24 x 6900 tokens, looped). Called before the
+// wait for the scores, which hides the load.
+template <int KEYS>
+__device__ __forceinline__ bool any_bias(const float* bp, int keys, int lane) {
+  bool mine = false;
+#pragma unroll
+  for (int i = 0; i < KEYS; i += 32)
+    if (i + lane < keys) mine |= __ldg(bp + i + lane) != 0.f;   // true for NaN
+  return __any_sync(0xffffffffu, mine);
+}
+
+// HAS_BIAS adds a per-key additive bias (a key-padding mask) to the scaled scores before the row maximum, in the tiles
+// where it is not zero throughout; the variant without it is the plain kernel.
 template <bool HAS_BIAS>
 __global__ void __launch_bounds__(NUM_THREADS, CTAS_PER_SM)
 sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -325,23 +339,23 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     for (int j = 0; j < n_tiles && ok; ++j) {
       const int st = j & 1;
       const uint32_t ph = static_cast<uint32_t>((j >> 1) & 1);
+      const int keys_here = min(BKV, p.seq_kv - j * BKV) - pt * 32;  // valid keys among this warp's 32 columns
+      const float* bp = HAS_BIAS ? p.key_bias + b * p.bias_batch_stride + j * BKV + pt * 32 : nullptr;
+      const bool biased = HAS_BIAS && (any_bias<32>(bp, keys_here, lane) || !(p.scale_log2 > 0.f));
       if (!mbar_wait(s_full + 8 * st, ph, DEV_TIMEOUT_ATTN)) {
         ok = false;
         break;
       }
       tc_fence_after();
       const uint32_t t_s = t_row + COL_S + BKV * st + 32 * pt;   // own S columns; own P goes over the first 16
-      const int keys_here = min(BKV, p.seq_kv - j * BKV) - pt * 32;  // valid keys among this warp's 32 columns
       const bool tail = keys_here < 32;  // only the last tile of a ragged sequence needs key masking
       uint32_t sA[32];
       tmem_ld_32x32(t_s, sA);
       tmem_ld_fence(sA);
-      if constexpr (HAS_BIAS) {
+      if (biased) {
         // scores become s * scale * log2(e) + bias * log2(e) here; everything after works on them with scale 1.
         // All threads of the warp read the same 32 bias values (one transaction per load).
         constexpr float LOG2E = 1.4426950408889634f;
-        const int k0 = j * BKV + pt * 32;
-        const float* bp = p.key_bias + b * p.bias_batch_stride + k0;
         if (!tail) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
@@ -359,7 +373,7 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           }
         }
       }
-      const float sc = HAS_BIAS ? 1.0f : p.scale_log2;
+      const float sc = biased ? 1.0f : p.scale_log2;
       float m_mine;
       if (!tail) {
         m_mine = max_chunk(sA, -INFINITY);
@@ -371,12 +385,13 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
       }
       // the partner warp holds the other 32 columns of the same rows: swap maxima (two buffers by tile parity;
       // the barrier per tile keeps the two warps at most one tile apart)
+      if (HAS_BIAS) m_mine *= sc;   // the partner's keys may be of the other kind
       xch[st * XCH_FLOATS + xch_row + 32 * pt] = m_mine;
       named_bar_sync(1 + qd, 32 * PARTS);
       float m_all = m_mine;
 #pragma unroll
       for (int o = 0; o < PARTS; ++o) m_all = fmaxf(m_all, xch[st * XCH_FLOATS + xch_row + 32 * o]);
-      const float m_tile = m_all * sc;
+      const float m_tile = HAS_BIAS ? m_all : m_all * sc;
       // grow the reference maximum only when it would change the exponent range by more than 2^8; both warps
       // of a quarter see the same maxima and take the same branch, each rescaling its own half of O
       const bool grow = m_tile > m_ref + 8.0f;
@@ -721,10 +736,13 @@ sdpa_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     float* xch = reinterpret_cast<float*>(smem_gen + OFF_XCH2);
     const int xch_mine = ((t * 4 + qd) * 2 + hf) * 32 + lane, xch_other = ((t * 4 + qd) * 2 + (hf ^ 1)) * 32 + lane;
     const uint32_t pair_bar = 1 + t * 4 + qd;   // named barrier of the two warps that share these rows
-    const float sc = HAS_BIAS ? 1.0f : p.scale_log2;
     float m_ref = -INFINITY, l_sum = 0.f;
     bool ok = true;
     for (int j = 0; j < n_tiles && ok; ++j) {
+      const int keys_here = p.seq_kv - j * BK - 64 * hf;   // >= 64 except on the last tile of a ragged sequence
+      const float* bp = HAS_BIAS ? p.key_bias + b * p.bias_batch_stride + j * BK + 64 * hf : nullptr;
+      const bool biased = HAS_BIAS && (any_bias<64>(bp, keys_here, lane) || !(p.scale_log2 > 0.f));
+      const float sc = biased ? 1.0f : p.scale_log2;
       if (!mbar_wait(my_s_full, static_cast<uint32_t>(j & 1), DEV_TIMEOUT_ATTN)) {
         ok = false;
         break;
@@ -735,9 +753,7 @@ sdpa_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       tmem_ld_32x32(t_s + 32, sb);
       tmem_ld_fence(sa);
       tmem_ld_fence(sb);
-      const int keys_here = p.seq_kv - j * BK - 64 * hf;   // >= 64 except on the last tile of a ragged sequence
-      if constexpr (HAS_BIAS) {
-        const float* bp = p.key_bias + b * p.bias_batch_stride + j * BK + 64 * hf;
+      if (biased) {
         add_bias_chunk(sa, bp, keys_here, p.scale_log2);
         add_bias_chunk(sb, bp + 32, keys_here - 32, p.scale_log2);
       }
@@ -745,13 +761,14 @@ sdpa_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         mask_chunk(sa, keys_here);
         mask_chunk(sb, keys_here - 32);
       }
-      const float m_mine = fmaxf(max_chunk(sa, -INFINITY), max_chunk(sb, -INFINITY));
+      float m_mine = fmaxf(max_chunk(sa, -INFINITY), max_chunk(sb, -INFINITY));
+      if (HAS_BIAS) m_mine *= sc;   // the partner's keys may be of the other kind
       // the partner warp holds the other 64 keys of the same rows: swap maxima (two buffers by tile parity; the
       // barrier per tile keeps the two warps at most one tile apart)
       float* x = xch + (j & 1) * XCH2_FLOATS;
       x[xch_mine] = m_mine;
       named_bar_sync(pair_bar, 64);
-      const float m_tile = fmaxf(m_mine, x[xch_other]) * sc;
+      const float m_tile = fmaxf(m_mine, x[xch_other]) * (HAS_BIAS ? 1.0f : sc);
       // grow the reference maximum only when it would change the exponent range by more than 2^8; both warps of
       // a row see the same maxima and take the same branch, each rescaling its own half of O
       const bool grow = m_tile > m_ref + 8.0f;
