@@ -7,7 +7,7 @@
 //                 (reference: flux_transformer/common/attention_utils.py:8-36,75-80)
 //   vec_ops       conditioning-vector helpers (sum of embeddings, SiLU) and the Euler step
 //                 (reference: time_text_embed.py:25-31, linear_scheduler.py:56-58)
-// The norms give one 128-thread block to a row, the others one warp to a row or head; nothing here waits on
+// The norms give a row to a 128-thread block, the others to a warp (or a head); nothing here waits on
 // another thread block.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -85,6 +85,19 @@ __device__ __forceinline__ void load_vec(const void* p, int dtype, int64_t off, 
     for (int i = 0; i < E; ++i) o[i] = load_as_float(p, dtype, off + i);
   }
 }
+// 16 bytes of float32 or bf16 values as floats.
+__device__ __forceinline__ void load8or4(const uint4& raw, float (&o)[4]) {
+  o[0] = __uint_as_float(raw.x); o[1] = __uint_as_float(raw.y);
+  o[2] = __uint_as_float(raw.z); o[3] = __uint_as_float(raw.w);
+}
+__device__ __forceinline__ void load8or4(const uint4& raw, float (&o)[8]) {
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    o[2 * i] = __uint_as_float(w[i] << 16);
+    o[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+  }
+}
 template <int E>
 __device__ __forceinline__ void store_vec_bf16(__nv_bfloat16* p, const float (&v)[E]) {
   if constexpr (E == 8) {
@@ -94,6 +107,39 @@ __device__ __forceinline__ void store_vec_bf16(__nv_bfloat16* p, const float (&v
     *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(h);
   }
 }
+// E elements of a per-channel vector (norm weight, gate, shift, scale). With BF (every vector of the call is bf16, what the
+// models pass) load() puts the bytes into registers and get() converts them, so that a kernel asks for them before a
+// block reduction and their trip overlaps it. Otherwise get() loads where the values are used: the dtype is a run-time
+// branch per vector, and no load moves above a branch.
+template <int E, bool BF>
+struct ChannelVec {
+  __device__ __forceinline__ void load(const void*, int64_t) {}
+  __device__ __forceinline__ void get(const void* p, int dtype, int64_t off, float (&o)[E]) const {
+    load_vec<E>(p, dtype, off, o);
+  }
+};
+template <int E>
+struct ChannelVec<E, true> {
+  uint32_t raw[E / 2];
+  __device__ __forceinline__ void load(const void* ptr, int64_t off) {
+    const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(ptr) + off;
+    if constexpr (E == 8) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(q));
+      raw[0] = v.x; raw[1] = v.y; raw[2] = v.z; raw[3] = v.w;
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(q));
+      raw[0] = v.x; raw[1] = v.y;
+    }
+  }
+  __device__ __forceinline__ void get(const void*, int, int64_t, float (&o)[E]) const {
+#pragma unroll
+    for (int i = 0; i < E / 2; ++i) {
+      o[2 * i] = __uint_as_float(raw[i] << 16);
+      o[2 * i + 1] = __uint_as_float(raw[i] & 0xFFFF0000u);
+    }
+  }
+};
+
 // Sum over the 128 threads of a block; `red` is a 4-float shared array used by this call only.
 __device__ __forceinline__ float block_sum_128(float v, float* red) {
   v = warp_sum(v);
@@ -105,66 +151,138 @@ __device__ __forceinline__ float block_sum_128(float v, float* red) {
 constexpr int NORM_THREADS = 128;
 constexpr int NORM_MAX_D = 4096;
 
-// One 128-thread block per row. Thread t holds the 16-byte vectors t, t+128, ... of the row in registers (at
-// most 32 floats), so every warp-level load or store covers 512 contiguous bytes and enough blocks are resident
-// per SM to keep HBM busy; mean and variance are two block reductions over the registers (two-pass variance).
-template <typename XT>
+// The kernels' largest row; D <= NORM_MID_D (the widest of the models but one) holds a quarter fewer registers.
+constexpr int NORM_MID_D = 3072;
+
+// Blocks of 128 threads stride over the rows. Thread t holds the 16-byte vectors t, t+128, ... of its row in registers,
+// so every warp-level access covers 512 contiguous bytes; mean and variance are two block reductions over the registers
+// (two-pass variance). The next row is on its way while this one is reduced, and the shift, scale and weight of a
+// channel stay in registers for all rows of a block: a block per row spent most of its life waiting for its own loads,
+// one after the other, and read 2/3 of the row's bytes again in shift and scale. HBM bounds it: 65536 x 3072 float32 rows
+// 308 -> 218 us (5.5 TB/s), 4608 rows 18.9 -> 14.3 us (from L2), 512 rows 5.6 -> 3.6 us; 1632 x 3840 with weight 12.7 ->
+// 9.3 us.
+template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
 __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormParams p) {
   constexpr int E = 16 / sizeof(XT);
-  constexpr int MAXV = NORM_MAX_D / E / NORM_THREADS;
-  __shared__ float red[2][4];
+  constexpr int MAXV = MAX_D / E / NORM_THREADS;
+  __shared__ float red[2][2][4];
   const int t = threadIdx.x;
-  const int64_t row_id = blockIdx.x;
-  const int b = static_cast<int>(row_id / p.rows);
-  const int r = static_cast<int>(row_id % p.rows);
-  const XT* x = static_cast<const XT*>(p.x) + b * p.x_batch_stride + static_cast<int64_t>(r) * p.x_row_stride;
-  __nv_bfloat16* y = p.y + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride;
+  const unsigned total = static_cast<unsigned>(p.rows) * p.batch;   // below 2^31
   const int nvec = p.D / E;
-  float v[MAXV][E];
-  float sum = 0.f;
+  auto row_of = [&](unsigned row_id, int& b, int& r) {
+    b = static_cast<int>(row_id / p.rows);
+    r = static_cast<int>(row_id - b * p.rows);
+  };
+  uint4 raw[MAXV];
+  auto fetch = [&](unsigned row_id) {
+    int b, r;
+    row_of(row_id, b, r);
+    const XT* x = static_cast<const XT*>(p.x) + b * p.x_batch_stride + static_cast<int64_t>(r) * p.x_row_stride;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int c = t + NORM_THREADS * i;
-    if (c < nvec) {
-      load_vec<E>(x, sizeof(XT) == 4 ? MFX_F32 : MFX_BF16, static_cast<int64_t>(c) * E, v[i]);
-#pragma unroll
-      for (int j = 0; j < E; ++j) sum += v[i][j];
+    for (int i = 0; i < MAXV; ++i) {
+      const int c = t + NORM_THREADS * i;
+      if (c < nvec) raw[i] = *(reinterpret_cast<const uint4*>(x) + c);
     }
-  }
-  float mean = 0.f;
-  if (!p.rms) mean = block_sum_128(sum, red[0]) / static_cast<float>(p.D);
-  float sq = 0.f;
+  };
+  ChannelVec<E, BF> scale_v[MAXV], shift_v[MAXV], weight_v[MAXV];
+  int mods_of = -1;                       // the sample whose shift and scale are held
+  unsigned row_id = blockIdx.x;
+  int parity = 0;
+  fetch(row_id);
+  for (; row_id < total; row_id += gridDim.x, parity ^= 1) {
+    int b, r;
+    row_of(row_id, b, r);
+    float v[MAXV][E];
+    float sum = 0.f;
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int c = t + NORM_THREADS * i;
-    if (c < nvec) {
+    for (int i = 0; i < MAXV; ++i) {
+      if (t + NORM_THREADS * i < nvec) {
+        load8or4(raw[i], v[i]);
 #pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float d = v[i][j] - mean;
-        sq += d * d;
+        for (int j = 0; j < E; ++j) sum += v[i][j];
+      }
+    }
+    if (row_id + gridDim.x < total) fetch(row_id + gridDim.x);
+    if (b != mods_of) {
+#pragma unroll
+      for (int i = 0; i < MAXV; ++i) {
+        const int c = t + NORM_THREADS * i;
+        if (c < nvec) {
+          const int64_t moff = b * p.mod_batch_stride + static_cast<int64_t>(c) * E;
+          if (MOD && p.scale) scale_v[i].load(p.scale, moff);
+          if (MOD && p.shift) shift_v[i].load(p.shift, moff);
+          if (WEIGHT && mods_of < 0) weight_v[i].load(p.weight, static_cast<int64_t>(c) * E);
+        }
+      }
+      mods_of = b;
+    }
+    float mean = 0.f;
+    if (!p.rms) mean = block_sum_128(sum, red[parity][0]) / static_cast<float>(p.D);
+    float sq = 0.f;
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+      if (t + NORM_THREADS * i < nvec) {
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          const float d = v[i][j] - mean;
+          sq += d * d;
+        }
+      }
+    }
+    const float rstd = rsqrtf(block_sum_128(sq, red[parity][1]) / static_cast<float>(p.D) + p.eps);
+    __nv_bfloat16* y = p.y + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride;
+#pragma unroll
+    for (int i = 0; i < MAXV; ++i) {
+      const int c = t + NORM_THREADS * i;
+      if (c < nvec) {
+        float o[E], sc[E], sh[E], wt[E];
+        const int64_t moff = b * p.mod_batch_stride + static_cast<int64_t>(c) * E;
+        if (MOD && p.scale) scale_v[i].get(p.scale, p.mod_dtype, moff, sc);
+        if (MOD && p.shift) shift_v[i].get(p.shift, p.mod_dtype, moff, sh);
+        if (WEIGHT) weight_v[i].get(p.weight, p.weight_dtype, static_cast<int64_t>(c) * E, wt);
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+          float u = (v[i][j] - mean) * rstd;
+          if (WEIGHT) u *= wt[j];
+          if (MOD && p.scale) u *= 1.0f + sc[j];
+          if (MOD && p.shift) u += sh[j];
+          o[j] = u;
+        }
+        store_vec_bf16<E>(y + static_cast<int64_t>(c) * E, o);
       }
     }
   }
-  const float rstd = rsqrtf(block_sum_128(sq, red[1]) / static_cast<float>(p.D) + p.eps);
-#pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int c = t + NORM_THREADS * i;
-    if (c < nvec) {
-      float o[E], sc[E], sh[E], wt[E];
-      const int64_t moff = b * p.mod_batch_stride + static_cast<int64_t>(c) * E;
-      if (p.scale) load_vec<E>(p.scale, p.mod_dtype, moff, sc);
-      if (p.shift) load_vec<E>(p.shift, p.mod_dtype, moff, sh);
-      if (p.weight) load_vec<E>(p.weight, p.weight_dtype, static_cast<int64_t>(c) * E, wt);
-#pragma unroll
-      for (int j = 0; j < E; ++j) {
-        float u = (v[i][j] - mean) * rstd;
-        if (p.weight) u *= wt[j];
-        if (p.scale) u *= 1.0f + sc[j];
-        if (p.shift) u += sh[j];
-        o[j] = u;
-      }
-      store_vec_bf16<E>(y + static_cast<int64_t>(c) * E, o);
-    }
+}
+
+template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
+void launch_norm_one(const NormParams& p, cudaStream_t st) {
+  // As many blocks as are resident at a time. More only add block starts (65536 x 3072 float32 rows, us, at 4 resident
+  // blocks per SM: 4 blocks 218, 8 219, 24 224; 4608 rows 14.3, 15.2, 17.5), fewer rows than that take a block each.
+  auto kern = norm_modulate_kernel<XT, BF, MAX_D, MOD, WEIGHT>;
+  static const int per_sm = [&] {
+    int n = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NORM_THREADS, 0) == cudaSuccess && n > 0 ? n : 4;
+  }();
+  const int64_t total = static_cast<int64_t>(p.rows) * p.batch, resident = per_sm * device_sm_count();
+  kern<<<static_cast<unsigned>(total < resident ? total : resident), NORM_THREADS, 0, st>>>(p);
+}
+template <typename XT, int MAX_D>
+void launch_norm_d(const NormParams& p, cudaStream_t st) {
+  const bool mod = p.shift || p.scale, weight = p.weight != nullptr;
+  const bool bf = (!mod || p.mod_dtype == MFX_BF16) && (!weight || p.weight_dtype == MFX_BF16);
+  if (bf && mod && !weight) launch_norm_one<XT, true, MAX_D, true, false>(p, st);
+  else if (bf && !mod && weight) launch_norm_one<XT, true, MAX_D, false, true>(p, st);
+  else if (bf && mod) launch_norm_one<XT, true, MAX_D, true, true>(p, st);
+  else if (weight) launch_norm_one<XT, false, MAX_D, true, true>(p, st);
+  else launch_norm_one<XT, false, MAX_D, true, false>(p, st);
+}
+void launch_norm(int x_dtype, const NormParams& p, cudaStream_t st) {
+  if (x_dtype == MFX_F32) {
+    if (p.D <= NORM_MID_D) launch_norm_d<float, NORM_MID_D>(p, st);
+    else launch_norm_d<float, NORM_MAX_D>(p, st);
+  } else {
+    if (p.D <= NORM_MID_D) launch_norm_d<__nv_bfloat16, NORM_MID_D>(p, st);
+    else launch_norm_d<__nv_bfloat16, NORM_MAX_D>(p, st);
   }
 }
 
@@ -195,9 +313,12 @@ struct PostNormParams {
 // (z_image_transformer/transformer_block.py:31,35; context_block.py:18,21). The norm needs the whole output row
 // of the projection, so it cannot be an epilogue of a matmul tiled along N; this pass reads y once.
 // One 128-thread block per row, 4 elements per vector (8-byte loads of bf16 y, 16-byte of the f32 residual).
+// Everything of the first stage is asked for before its reduction, the second stage's vectors before the second one (with
+// the loads where the values are used a block waited for three trips to memory): 1632 x 3840 rows, both stages, 34.0 -> 19.2
+// us with the operands in HBM, 20.8 -> 12.1 us in L2; 8426 rows 104 -> 83 us.
 // With next_out the block goes on to the pre-norm of the following sub-layer on the row it just updated
 // (transformer_block.py:34 after :31, and the next block's :29-30 after :35), which saves reading the stream again.
-template <typename YT>
+template <typename YT, bool BF>
 __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const PostNormParams p) {
   constexpr int E = 4;
   constexpr int MAXV = NORM_MAX_D / E / NORM_THREADS;
@@ -209,13 +330,26 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const 
   const YT* y = static_cast<const YT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride;
   float* res = p.residual + b * p.res_batch_stride + static_cast<int64_t>(r) * p.res_row_stride;
   const int nvec = p.D / E;
-  float v[MAXV][E];
+  float v[MAXV][E], stream[MAXV][E];
+  ChannelVec<E, BF> weight_v[MAXV], gate_v[MAXV];
   float sq = 0.f;
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     const int c = t + NORM_THREADS * i;
+    if (c < nvec) load_vec<E>(y, sizeof(YT) == 4 ? MFX_F32 : MFX_BF16, static_cast<int64_t>(c) * E, v[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    const int c = t + NORM_THREADS * i;
     if (c < nvec) {
-      load_vec<E>(y, sizeof(YT) == 4 ? MFX_F32 : MFX_BF16, static_cast<int64_t>(c) * E, v[i]);
+      load_vec<E>(res, MFX_F32, static_cast<int64_t>(c) * E, stream[i]);
+      weight_v[i].load(p.weight, static_cast<int64_t>(c) * E);
+      if (p.gate) gate_v[i].load(p.gate, b * p.gate_batch_stride + static_cast<int64_t>(c) * E);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < MAXV; ++i) {
+    if (t + NORM_THREADS * i < nvec) {
 #pragma unroll
       for (int j = 0; j < E; ++j) sq += v[i][j] * v[i][j];
     }
@@ -226,9 +360,10 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const 
     const int c = t + NORM_THREADS * i;
     if (c < nvec) {
       float wt[E], gt[E], rs[E];
-      load_vec<E>(p.weight, p.weight_dtype, static_cast<int64_t>(c) * E, wt);
-      if (p.gate) load_vec<E>(p.gate, p.gate_dtype, b * p.gate_batch_stride + static_cast<int64_t>(c) * E, gt);
-      load_vec<E>(res, MFX_F32, static_cast<int64_t>(c) * E, rs);
+      weight_v[i].get(p.weight, p.weight_dtype, static_cast<int64_t>(c) * E, wt);
+      if (p.gate) gate_v[i].get(p.gate, p.gate_dtype, b * p.gate_batch_stride + static_cast<int64_t>(c) * E, gt);
+#pragma unroll
+      for (int j = 0; j < E; ++j) rs[j] = stream[i][j];
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         float u = v[i][j] * rstd * wt[j];
@@ -240,11 +375,15 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const 
     }
   }
   if (p.next_out == nullptr) return;   // uniform over the grid
+  ChannelVec<E, BF> next_weight_v[MAXV], next_scale_v[MAXV];
   float sq2 = 0.f;
 #pragma unroll
   for (int i = 0; i < MAXV; ++i) {
     const int c = t + NORM_THREADS * i;
     if (c < nvec) {
+      next_weight_v[i].load(p.next_weight, static_cast<int64_t>(c) * E);
+      if (p.next_scale)
+        next_scale_v[i].load(p.next_scale, b * p.next_scale_batch_stride + static_cast<int64_t>(c) * E);
 #pragma unroll
       for (int j = 0; j < E; ++j) sq2 += v[i][j] * v[i][j];
     }
@@ -256,9 +395,10 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const 
     const int c = t + NORM_THREADS * i;
     if (c < nvec) {
       float wt[E], sc[E], o[E];
-      load_vec<E>(p.next_weight, p.next_weight_dtype, static_cast<int64_t>(c) * E, wt);
+      next_weight_v[i].get(p.next_weight, p.next_weight_dtype, static_cast<int64_t>(c) * E, wt);
       if (p.next_scale)
-        load_vec<E>(p.next_scale, p.next_scale_dtype, b * p.next_scale_batch_stride + static_cast<int64_t>(c) * E, sc);
+        next_scale_v[i].get(p.next_scale, p.next_scale_dtype,
+                            b * p.next_scale_batch_stride + static_cast<int64_t>(c) * E, sc);
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         float u = v[i][j] * rstd2 * wt[j];
@@ -512,10 +652,7 @@ int mfx_norm_modulate(const mfx_norm_args* a, void* stream) {
   p.y_batch_stride = a->y_batch_stride;
   const int64_t total = a->rows * a->batch;
   if (total > 0x7fffffffll) return MFX_ERR_TOO_LARGE;
-  const unsigned blocks = static_cast<unsigned>(total);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a->x_dtype == MFX_F32) norm_modulate_kernel<float><<<blocks, NORM_THREADS, 0, st>>>(p);
-  else norm_modulate_kernel<__nv_bfloat16><<<blocks, NORM_THREADS, 0, st>>>(p);
+  launch_norm(a->x_dtype, p, static_cast<cudaStream_t>(stream));
   MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
@@ -685,8 +822,15 @@ int mfx_post_pre_norm(const mfx_post_pre_norm_args* a, void* stream) {
   if (a->rows * a->batch > 0x7fffffffll) return MFX_ERR_TOO_LARGE;
   const unsigned blocks = static_cast<unsigned>(a->rows * a->batch);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a->y_dtype == MFX_F32) norm_gate_residual_kernel<float><<<blocks, NORM_THREADS, 0, st>>>(p);
-  else norm_gate_residual_kernel<__nv_bfloat16><<<blocks, NORM_THREADS, 0, st>>>(p);
+  const bool bf = p.weight_dtype == MFX_BF16 && (!p.gate || p.gate_dtype == MFX_BF16) &&
+                  (!p.next_out || (p.next_weight_dtype == MFX_BF16 && (!p.next_scale || p.next_scale_dtype == MFX_BF16)));
+  if (a->y_dtype == MFX_F32) {
+    if (bf) norm_gate_residual_kernel<float, true><<<blocks, NORM_THREADS, 0, st>>>(p);
+    else norm_gate_residual_kernel<float, false><<<blocks, NORM_THREADS, 0, st>>>(p);
+  } else {
+    if (bf) norm_gate_residual_kernel<__nv_bfloat16, true><<<blocks, NORM_THREADS, 0, st>>>(p);
+    else norm_gate_residual_kernel<__nv_bfloat16, false><<<blocks, NORM_THREADS, 0, st>>>(p);
+  }
   MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
