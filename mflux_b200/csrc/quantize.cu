@@ -6,9 +6,11 @@
 // bits [j*bits, (j+1)*bits) of the row's bit stream, which for 4 and 8 bits is "8 / 4 codes per uint32" and for
 // 3, 5 and 6 bits (the other widths the reference's CLI offers, src/mflux/cli/defaults/defaults.py:63) lets
 // codes straddle byte and word boundaries (8 codes in 3 or 5 bytes, 4 codes in 3 bytes).
-// Four lanes own one group (16 values each); min/max go through warp shuffles.
+// Two or four lanes own one group; min/max go through warp shuffles.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "host_util.cuh"
 
@@ -33,25 +35,61 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
-constexpr int PER_THREAD = 16;   // values of one group a thread holds
-
-template <typename T>
-__device__ __forceinline__ void load16(const T* p, float (&v)[16]) {
-  if constexpr (sizeof(T) == 4) {
+// The PT (16 or 32) values of a thread as they lie in memory: 16-bit values two to a register, whose extremes are taken in
+// pairs.
+template <typename T, int PT>
+struct Values {
+  using Pair = typename std::conditional<std::is_same<T, __half>::value, __half2, __nv_bfloat162>::type;
+  Pair h[PT / 2];
+  __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(p) + i);
-      v[4 * i] = a.x; v[4 * i + 1] = a.y; v[4 * i + 2] = a.z; v[4 * i + 3] = a.w;
-    }
-  } else {
+    for (int i = 0; i < PT / 8; ++i) {
+      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p) + i);
+      const Pair* r = reinterpret_cast<const Pair*>(&raw);
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p) + k);
-      const T* h = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[8 * k + i] = to_f32<T>(h[i]);
+      for (int j = 0; j < 4; ++j) h[4 * i + j] = r[j];
     }
   }
+  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+    Pair hi = h[0], lo = h[0];
+#pragma unroll
+    for (int i = 1; i < PT / 2; ++i) {
+      hi = __hmax2(hi, h[i]);
+      lo = __hmin2(lo, h[i]);
+    }
+    mx = fmaxf(to_f32<T>(hi.x), to_f32<T>(hi.y));
+    mn = fminf(to_f32<T>(lo.x), to_f32<T>(lo.y));
+  }
+  __device__ __forceinline__ float get(int i) const { return to_f32<T>(i & 1 ? h[i / 2].y : h[i / 2].x); }
+};
+template <int PT>
+struct Values<float, PT> {
+  float f[PT];
+  __device__ __forceinline__ void load(const float* p) {
+#pragma unroll
+    for (int i = 0; i < PT / 4; ++i) {
+      const float4 a = __ldg(reinterpret_cast<const float4*>(p) + i);
+      f[4 * i] = a.x; f[4 * i + 1] = a.y; f[4 * i + 2] = a.z; f[4 * i + 3] = a.w;
+    }
+  }
+  __device__ __forceinline__ void extremes(float& mx, float& mn) const {
+    mx = mn = f[0];
+#pragma unroll
+    for (int i = 1; i < PT; ++i) {
+      mx = fmaxf(mx, f[i]);
+      mn = fminf(mn, f[i]);
+    }
+  }
+  __device__ __forceinline__ float get(int i) const { return f[i]; }
+};
+
+__device__ __forceinline__ uint64_t pair_f32(float lo, float hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ void split_f32(uint64_t v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
 // The quantizer's definition of a code: the correctly rounded quotient, rounded to even, clamped.
@@ -61,32 +99,32 @@ __device__ __forceinline__ float exact_code(float d, float scale, float n_bins) 
   return fminf(fmaxf(q, 0.0f), n_bins);
 }
 
-// One thread: 16 consecutive values of a row; lanes 4g..4g+3 of a warp form one 64-wide group.
-// A division per value was what the kernel spent its time on. It multiplies by the reciprocal of the scale instead and
-// takes the rounded product where that must be the rounded quotient too: reciprocal, product and the quotient itself
-// are each off by at most 2^-24 of their value, together 1.8e-7 of at most n_bins + 1, so a product further than that
-// from every k + 0.5 rounds like the quotient. Threads with a value nearer to one (one in 1000 at 4 bits) divide.
-template <typename T, int BITS, int QMODE>
-__global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, int64_t n_groups_total,
+// One thread: PT consecutive values of a row; 64 / PT neighbouring lanes form one group.
+// Instruction issue bounds it, so: sums, products and roundings go in packed pairs of float32 (each half rounds like the
+// scalar instruction), extremes of 16-bit weights in packed pairs of them, clamping in packed pairs of 16-bit integers,
+// and with PT = 32 twice as many values share the scale's handful of divisions.
+// A division per value is replaced by the reciprocal of the scale and the rounded product where that must be the rounded
+// quotient too: reciprocal, product and the quotient itself are each off by at most 2^-24 of their value, together 1.8e-7
+// of at most n_bins + 1, so a product further than that from every k + 0.5 rounds like the quotient. Values nearer to one
+// (one in 1000 at 4 bits) are divided.
+template <typename T, int BITS, int QMODE, int PT>
+__global__ void __launch_bounds__(128) quantize_kernel(const T* __restrict__ w, int64_t n_groups_total,
                                                        uint32_t* __restrict__ wq, T* __restrict__ scales,
                                                        T* __restrict__ biases) {
   const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t group = tid >> 2;
+  constexpr int LANES = 64 / PT;                  // of a group
+  const int64_t group = tid / LANES;
   const bool active = group < n_groups_total;
   const int64_t g = active ? group : n_groups_total - 1;  // keep whole warps in the shuffles
-  const int sub = static_cast<int>(tid & 3);
-  float v[16];
-  load16<T>(w + g * 64 + sub * 16, v);
-  float mx = v[0], mn = v[0];
+  const int sub = static_cast<int>(tid % LANES);
+  Values<T, PT> v;
+  v.load(w + g * 64 + sub * PT);
+  float mx, mn;
+  v.extremes(mx, mn);
 #pragma unroll
-  for (int i = 1; i < 16; ++i) {
-    mx = fmaxf(mx, v[i]);
-    mn = fminf(mn, v[i]);
-  }
-#pragma unroll
-  for (int off = 2; off >= 1; off >>= 1) {
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+  for (int o = LANES / 2; o >= 1; o >>= 1) {
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
   }
   constexpr float n_bins = static_cast<float>((1 << BITS) - 1);
   float scale, bias;
@@ -107,52 +145,81 @@ __global__ void __launch_bounds__(256) quantize_kernel(const T* __restrict__ w, 
     bias = mn;
   }
   const float mag = fabsf(scale);
-  bool divide = !(mag > 1e-30f && mag < 1e30f);   // the reciprocal has to be a normal number
+  // the reciprocal has to be a normal number; a negative limit sends every value to the division
+  const float limit = mag > 1e-30f && mag < 1e30f ? 0.5f - (n_bins + 1.0f) * 2.4e-7f : -1.0f;
   const float inv = __frcp_rn(scale);
   constexpr float MAGIC = 12582912.0f;            // 1.5 * 2^23: adding it rounds to even at the units place
-  float q[16];
-  float far = 0.0f;                               // largest distance of a product from its integer
+  const uint64_t inv2 = pair_f32(inv, inv), neg_bias2 = pair_f32(-bias, -bias), magic2 = pair_f32(MAGIC, MAGIC),
+                 neg_magic2 = pair_f32(-MAGIC, -MAGIC), minus2 = pair_f32(-1.0f, -1.0f);
+  constexpr int WORDS = (BITS * PT + 31) / 32;
+  uint32_t word[WORDS + 1];                       // the thread's codes
 #pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float r = fminf(fmaxf(__fmul_rn(__fsub_rn(v[i], bias), inv), 0.0f), n_bins);
-    q[i] = __fsub_rn(__fadd_rn(r, MAGIC), MAGIC);
-    far = fmaxf(far, fabsf(__fsub_rn(r, q[i])));
-  }
-  divide |= far > 0.5f - (n_bins + 1.0f) * 2.4e-7f;
-  if (divide) {
+  for (int i = 0; i <= WORDS; ++i) word[i] = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] = exact_code(__fsub_rn(v[i], bias), scale, n_bins);
-  }
-  if (!active) return;
-  if constexpr (BITS == 4) {
-    // four codes at a time as an exact float below 2^16
-    uint32_t half[4];
+  for (int k = 0; k < PT / 8; ++k) {              // eight values
+    float t[8], off[8];                           // MAGIC + code; distance of the product from its integer
+    float far = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      uint64_t r2 = pair_f32(v.get(8 * k + i), v.get(8 * k + i + 1)), t2, e2;
+      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(r2) : "l"(neg_bias2));
+      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r2) : "l"(inv2));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t2) : "l"(r2), "l"(magic2));
+      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(e2) : "l"(t2), "l"(neg_magic2));
+      asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(e2) : "l"(minus2), "l"(r2));
+      split_f32(t2, t[i], t[i + 1]);
+      split_f32(e2, off[i], off[i + 1]);
+      far = fmaxf(far, fmaxf(fabsf(off[i]), fabsf(off[i + 1])));
+    }
+    if (far > limit) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (!(fabsf(off[i]) <= limit))
+          t[i] = __fadd_rn(exact_code(__fsub_rn(v.get(8 * k + i), bias), scale, n_bins), MAGIC);
+    }
+    // codes clamped to [0, n_bins] in 16-bit pairs (i, i + 4): the low half of MAGIC + code is the code, also below zero
+    uint32_t c[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      half[i] = static_cast<uint32_t>(fmaf(fmaf(fmaf(q[4 * i + 3], 16.0f, q[4 * i + 2]), 16.0f, q[4 * i + 1]), 16.0f,
-                                           q[4 * i]));
-    reinterpret_cast<uint2*>(wq)[g * 4 + sub] = make_uint2(half[0] | (half[1] << 16), half[2] | (half[3] << 16));
-  } else if constexpr (BITS == 8) {
-    uint32_t word[4];
+      c[i] = __vimin_s16x2_relu(__byte_perm(__float_as_uint(t[i]), __float_as_uint(t[i + 4]), 0x5410),
+                                ((1u << BITS) - 1u) * 0x10001u);
+    if constexpr (BITS == 4) {
+      word[k] = c[0] + c[1] * 16u + c[2] * 256u + c[3] * 4096u;
+    } else if constexpr (BITS == 8) {
+      word[2 * k] = __byte_perm(c[0] + c[1] * 256u, c[2] + c[3] * 256u, 0x5410);
+      word[2 * k + 1] = __byte_perm(c[0] + c[1] * 256u, c[2] + c[3] * 256u, 0x7632);
+    } else {
+      // eight codes are 8 * BITS bits of the stream, from bit 8 * BITS * k of the thread's
+      unsigned long long eight = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t lo = static_cast<uint32_t>(fmaf(q[4 * i + 1], 256.0f, q[4 * i]));
-      const uint32_t hi = static_cast<uint32_t>(fmaf(q[4 * i + 3], 256.0f, q[4 * i + 2]));
-      word[i] = lo | (hi << 16);
+      for (int i = 0; i < 4; ++i) {
+        eight |= static_cast<unsigned long long>(c[i] & 0xFFFFu) << (BITS * i);
+        eight |= static_cast<unsigned long long>(c[i] >> 16) << (BITS * (i + 4));
+      }
+      constexpr int LEN = 8 * BITS;
+      const int at = (LEN * k) / 32, sh = (LEN * k) % 32;
+      word[at] |= static_cast<uint32_t>(eight << sh);
+      if (sh + LEN > 32) word[at + 1] |= static_cast<uint32_t>((eight << sh) >> 32);
     }
-    reinterpret_cast<uint4*>(wq)[g * 4 + sub] = make_uint4(word[0], word[1], word[2], word[3]);
-  } else {
-    // 8 codes = BITS bytes of the bit stream; 16 of them are BITS 16-bit words at an even address
-    unsigned long long lo = 0, hi = 0;
+  }
+  if (!active) return;
+  if constexpr (BITS == 4 || BITS == 8) {
+    uint32_t* dst = wq + (g * LANES + sub) * WORDS;
+    if constexpr (WORDS == 2) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(word[0], word[1]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      lo |= static_cast<unsigned long long>(static_cast<uint32_t>(q[i])) << (BITS * i);
-      hi |= static_cast<unsigned long long>(static_cast<uint32_t>(q[8 + i])) << (BITS * i);
+      for (int i = 0; i < WORDS; i += 4)
+        *reinterpret_cast<uint4*>(dst + i) = make_uint4(word[i], word[i + 1], word[i + 2], word[i + 3]);
     }
-    const unsigned long long w0 = lo | (hi << (8 * BITS)), w1 = hi >> (64 - 8 * BITS);
-    uint16_t* dst = reinterpret_cast<uint16_t*>(wq) + (g * 4 + sub) * BITS;
+  } else if constexpr (PT == 32) {
+    uint32_t* dst = wq + (g * LANES + sub) * BITS;
 #pragma unroll
-    for (int i = 0; i < BITS; ++i) dst[i] = static_cast<uint16_t>(i < 4 ? w0 >> (16 * i) : w1 >> (16 * (i & 3)));
+    for (int i = 0; i < BITS; ++i) dst[i] = word[i];
+  } else {                                        // 16 codes are BITS 16-bit words at an even address
+    uint16_t* dst = reinterpret_cast<uint16_t*>(wq) + (g * LANES + sub) * BITS;
+#pragma unroll
+    for (int i = 0; i < BITS; ++i) dst[i] = static_cast<uint16_t>(word[i / 2] >> (16 * (i & 1)));
   }
   if (sub == 0) {
     scales[g] = from_f32<T>(scale);
@@ -222,30 +289,42 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
   for (int i = 0; i < V * static_cast<int>(sizeof(OUT)) / 16; ++i) dst[i] = reinterpret_cast<const uint4*>(res)[i];
 }
 
+template <typename T, int BITS, int PT>
+void launch_quantize_pt(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases, cudaStream_t st) {
+  const unsigned blocks = static_cast<unsigned>((n_groups * (64 / PT) + 127) / 128);
+  if (qmode == MFX_QMODE_MLX)
+    quantize_kernel<T, BITS, MFX_QMODE_MLX, PT><<<blocks, 128, 0, st>>>(w, n_groups, wq, scales, biases);
+  else
+    quantize_kernel<T, BITS, MFX_QMODE_DOC, PT><<<blocks, 128, 0, st>>>(w, n_groups, wq, scales, biases);
+}
+
+// Values a thread takes of 16-bit weights: 32 share the scale's divisions once there are threads enough without 16. us,
+// 16 / 32 values, bf16, 4 bits (8 bits): 12288 x 3072 28.0 / 25.5 (32.6 / 29.0), 3072 x 3072 9.2 / 8.9 (10.2 / 9.7), 1024 x
+// 512 2.65 / 3.24 (2.99 / 3.76); before, at 16 values and unpacked, 41.7 (44.4), 13.5 (13.6) and 2.9 (3.0). Float32 weights
+// would need 128 bytes per thread at 32: 28 us at 16 for 12288 x 3072, 37 at 32 (29 before).
+constexpr int64_t LARGE_WEIGHT = 4 << 20;
+template <typename T, int BITS>
+void launch_quantize_bits(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases, cudaStream_t st) {
+  if constexpr (sizeof(T) == 2) {
+    if (n_groups * 64 >= LARGE_WEIGHT) return launch_quantize_pt<T, BITS, 32>(w, n_groups, qmode, wq, scales, biases, st);
+  }
+  launch_quantize_pt<T, BITS, 16>(w, n_groups, qmode, wq, scales, biases, st);
+}
+
 template <typename T>
 int launch_quantize(const void* w, int64_t n_groups, int bits, int qmode, uint32_t* wq, void* scales, void* biases,
                     cudaStream_t st) {
-  const int64_t threads = n_groups * (64 / PER_THREAD);
-  const unsigned blocks = static_cast<unsigned>((threads + 255) / 256);
   const T* wp = static_cast<const T*>(w);
   T* sp = static_cast<T*>(scales);
   T* bp = static_cast<T*>(biases);
-#define MFX_QUANT_CASE(B)                                                                        \
-  case B:                                                                                       \
-    if (qmode == MFX_QMODE_MLX)                                                                 \
-      quantize_kernel<T, B, MFX_QMODE_MLX><<<blocks, 256, 0, st>>>(wp, n_groups, wq, sp, bp);   \
-    else                                                                                        \
-      quantize_kernel<T, B, MFX_QMODE_DOC><<<blocks, 256, 0, st>>>(wp, n_groups, wq, sp, bp);   \
-    break;
   switch (bits) {
-    MFX_QUANT_CASE(3)
-    MFX_QUANT_CASE(4)
-    MFX_QUANT_CASE(5)
-    MFX_QUANT_CASE(6)
-    MFX_QUANT_CASE(8)
+    case 3: launch_quantize_bits<T, 3>(wp, n_groups, qmode, wq, sp, bp, st); break;
+    case 4: launch_quantize_bits<T, 4>(wp, n_groups, qmode, wq, sp, bp, st); break;
+    case 5: launch_quantize_bits<T, 5>(wp, n_groups, qmode, wq, sp, bp, st); break;
+    case 6: launch_quantize_bits<T, 6>(wp, n_groups, qmode, wq, sp, bp, st); break;
+    case 8: launch_quantize_bits<T, 8>(wp, n_groups, qmode, wq, sp, bp, st); break;
     default: return MFX_ERR_UNSUPPORTED_BITS;
   }
-#undef MFX_QUANT_CASE
   MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
