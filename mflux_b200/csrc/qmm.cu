@@ -13,9 +13,9 @@
 //   warp 0      TMA producer: per stage its X tile [128 x 128 k] bf16 as two 128-byte-swizzled slabs (counted
 //               on the leader's barrier), the packed codes of its weight rows and their (scale, bias) pairs
 //   warp 1      allocates TMEM; in the leader CTA issues tcgen05.mma.cta_group::2 (M=256, N=tile width, K=16)
-//   warps 4-7   epilogue: tcgen05.ld -> bias / activation / gated residual -> global, overlapped with the
-//               main loop of the next tile (two 256-column TMEM accumulators)
-//   warps 8-    dequantizers, one or two teams of eight that take the stages in turn: codes (smem) -> bf16 -> B operand
+//   warps 4-    epilogue, four warps (eight where an activation is computed): tcgen05.ld -> bias / activation / gated
+//               residual -> global, overlapped with the main loop of the next tile (two 256-column TMEM accumulators)
+//   behind them dequantizers, one or two teams of eight that take the stages in turn: codes (smem) -> bf16 -> B operand
 //               tile in the swizzled K-major layout. 4-bit codes by the bf16 exponent-magic (128 + code) and one bf16
 //               fma with the group's scale and bias; 8-bit codes by the float32 magic (2^23 + code) and packed f32x2
 //               add + fma, rounded to bf16 at the end
@@ -43,9 +43,7 @@ constexpr int BM = 128;       // activation rows per CTA (256 per pair)
 constexpr int BN_MAX = 256;   // weight rows (output columns) per pair tile, at most; each CTA dequantizes half (BNH)
 constexpr int BK = 64;        // one quantization group
 constexpr int GPS = 2;        // quantization groups per pipeline stage
-constexpr int FIXED_WARPS = 8;  // producer, MMA, 2 spare, 4 epilogue
-constexpr int FIRST_DQ_WARP = 8;
-constexpr int FIRST_EPI_WARP = 4;
+constexpr int FIRST_EPI_WARP = 4;   // behind the producers, the MMA issuer and a spare warp
 constexpr int X_TILE_BYTES = BM * BK * 2;        // 16 KiB per group
 constexpr uint32_t TMEM_COLS = 512;
 
@@ -115,9 +113,11 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& tm, 
 }
 
 // EXT compiles the low-rank extension stages in; without it the loops below are the plain quantized matmul.
-// TEAMS x NUM_DQ_WARPS dequantizer warps; a team takes every TEAMS-th stage.
-template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, int TEAMS, bool EXT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((FIXED_WARPS + TEAMS * NUM_DQ_WARPS) * 32, 1)
+// TEAMS x NUM_DQ_WARPS dequantizer warps; a team takes every TEAMS-th stage. EPI_WARPS: 4, or 8 with two per 32 rows.
+template <int BITS, int BNH, uint32_t WF, int ST, int SD, typename OUT, int EPI, int NUM_DQ_WARPS, int TEAMS,
+          int EPI_WARPS, bool EXT>
+__global__ void __cluster_dims__(2, 1, 1)
+__launch_bounds__((FIRST_EPI_WARP + EPI_WARPS + TEAMS * NUM_DQ_WARPS) * 32, 1)
 qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
            const __grid_constant__ CUtensorMap tmap_sb, const __grid_constant__ CUtensorMap tmap_t,
            const __grid_constant__ CUtensorMap tmap_lb, const Params p) {
@@ -132,6 +132,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
   // the stage's packed codes were read before its B tile was written, so they are free by then too. That is one
   // tcgen05.commit and eight dequantizer arrivals less per stage.
   constexpr bool UNIFIED = (ST == SD);
+  constexpr int FIRST_DQ_WARP = FIRST_EPI_WARP + EPI_WARPS;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -180,7 +181,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(acc_full(s), 1);
-      mbar_init(acc_empty(s), 8);               // 4 epilogue warps in each CTA
+      mbar_init(acc_empty(s), 2 * EPI_WARPS);
     }
     fence_mbar_init();
     tma_prefetch_desc(&tmap_x);
@@ -476,7 +477,9 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
   } else if (warp >= FIRST_EPI_WARP) {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3;            // TMEM lane quarter this warp may read
-    const int et = threadIdx.x - FIRST_EPI_WARP * 32;  // 0..127
+    const int et = threadIdx.x - FIRST_EPI_WARP * 32;
+    const int part = (warp - FIRST_EPI_WARP) >> 2;      // which of the warps of a quarter: its share of the columns
+    constexpr int COLS = BN / (EPI_WARPS / 4);
     const int row = q * 32 + lane;
     bool ok = true;
     int it = 0;
@@ -491,13 +494,13 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
       float* bias_s = vec_s + a * BN_MAX;
       float* gate_s = vec_s + (2 + a) * BN_MAX;
 #pragma unroll
-      for (int c = et; c < BN; c += 128) {
+      for (int c = et; c < BN; c += EPI_WARPS * 32) {
         const int n = n0 + c;
         bias_s[c] = (p.bias != nullptr && n < p.N) ? load_as_float(p.bias, p.bias_dtype, n) : 0.f;
         if (EPI == MFX_EPI_GATE_RESIDUAL)
           gate_s[c] = (n < p.N) ? load_as_float(p.gate, p.gate_dtype, b * p.gate_batch_stride + n) : 0.f;
       }
-      named_bar_sync(1, 128);
+      named_bar_sync(1, EPI_WARPS * 32);
       const bool row_ok = r < p.rows;
       // SwiGLU writes one value per (gate, up) column pair: output column n/2
       OUT* yrow = static_cast<OUT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride +
@@ -507,7 +510,7 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
         // rows past the end point at the sample's first row: no address of theirs leaves the buffer, read or not
         rrow = static_cast<const OUT*>(p.residual) + b * p.res_batch_stride +
                static_cast<int64_t>(row_ok ? r : 0) * p.res_row_stride + n0;
-        if (row_ok && p.K <= PREFETCH_K) prefetch_row(rrow, 0, BN, p.N - n0);
+        if (row_ok && p.K <= PREFETCH_K) prefetch_row(rrow, part * COLS, (part + 1) * COLS, p.N - n0);
       }
       if (!mbar_wait_sleep(acc_full(a), aph, DEV_TIMEOUT_ACC_FULL)) {
         ok = false;
@@ -570,7 +573,8 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
           __syncwarp();
         }
       } else {
-        write_row<OUT, EPI, false>(t_addr, 0, BN, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s, gate_s);
+        write_row<OUT, EPI, false>(t_addr, part * COLS, (part + 1) * COLS, p.N - n0, row_ok, p.wide, yrow, rrow, bias_s,
+                                   gate_s);
       }
       tc_fence_before();
       __syncwarp();
@@ -614,13 +618,20 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   // teams take turns. 4 bits, M 4096, N 12288, K 3072, GELU: 264 -> 227 us; M 4608, N 3072, K 15360: 322 -> 297 us; M
   // 512, N 3072, K 12288: 70 -> 62 us. Eight-bit tiles leave room for two B stages, where a second team has nowhere to
   // write ahead and costs 2-3 % (M 1613, N 20480, K 3840: 212 -> 218 us).
-  // 768 threads leave a thread 80 registers. ptxas spills in 38 of the 158 instantiations, all with two teams: 32 to 44
-  // bytes stored (68 to 88 loaded) per 32 columns of the float32 gated residual, whose four loads in flight do not fit
-  // beside the accumulator (qmm_epilogue.cuh), 4 bytes in the bf16 form of it and in the GELUs with float32 output.
+  // 768 threads leave a thread 80 registers, 896 with eight epilogue warps 72. ptxas spills 20 to 32
+  // bytes per 32 columns of the float32 gated residual, whose four loads in flight do not fit beside the accumulator
+  // (qmm_epilogue.cuh), 4 to 8 bytes in the bf16 form of it and in the GELUs.
   constexpr int NDQ = 8;
   constexpr int TEAMS = SD > 2 ? 2 : 1;
-  constexpr int NUM_THREADS = (FIXED_WARPS + TEAMS * NDQ) * 32;
-  auto kern = qmm_kernel<BITS, BNH, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EXT>;
+  // Four epilogue warps keep up with the main loop where they add a bias or a residual, not where each value goes through
+  // erff, tanhf or an exponential: a tile then waits for its predecessor's epilogue. Eight share the columns. M 4096, N
+  // 12288, K 3072, 4 bits, us: erf form 299 -> 273 (260 -> 233 below the power limit), tanh form 280 -> 264 (240 -> 227),
+  // without activation 250; M 2000, N 3072, K 3072, SiLU 49.2 -> 42.8. Eight without one cost 1 % (146.6 -> 149.5 at 8
+  // bits, M 1632, N 11520, K 3840), and leave the gated residual 72 registers instead of 80.
+  constexpr int EPI_WARPS =
+      EPI == MFX_EPI_GELU_ERF || EPI == MFX_EPI_GELU_TANH || EPI == MFX_EPI_SILU || EPI == MFX_EPI_SWIGLU ? 8 : 4;
+  constexpr int NUM_THREADS = (FIRST_EPI_WARP + EPI_WARPS + TEAMS * NDQ) * 32;
+  auto kern = qmm_kernel<BITS, BNH, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EPI_WARPS, EXT>;
   static SmemConfigured configured;  // one record per instantiation of the kernel
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::DYN_BYTES, configured)) return rc;
   kern<<<grid, NUM_THREADS, L::DYN_BYTES, st>>>(tx, tw, tsb, tt, tlb, p);

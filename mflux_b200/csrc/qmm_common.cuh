@@ -61,17 +61,17 @@ __device__ __forceinline__ uint2 dequant_w8_f32(uint32_t q, uint64_t sc2, uint64
 
 // Epilogue activations in float32, on CUDA's own erff, tanhf and __expf: within 2^-21 |v| of the exact value everywhere,
 // 4e-8 to 5e-8 in the 2-norm for |v| < 1. Cheaper forms (ex2.approx / rcp.approx, a polynomial for erfc) were up to four
-// times further off there; they made M 4096, N 12288, K 3072, 4 bits, take 261 us (erf form) and 252 us (tanh form)
-// where these take 299 and 276 us.
+// times further off there. M 4096, N 12288, K 3072, 4 bits, with four epilogue warps, us: cheaper forms 261 (erf) and 252
+// (tanh), these 299 and 276; with the eight that such calls have now, these 273 and 264.
 __device__ __forceinline__ float gelu_erf(float v) { return 0.5f * v * (1.0f + erff(v * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_tanh(float v) {
   const float u = 0.7978845608028654f * (v + 0.044715f * v * v * v);
   return 0.5f * v * (1.0f + tanhf(u));
 }
 __device__ __forceinline__ float silu(float v) { return v / (1.0f + __expf(-v)); }
-// The same out of line. Where four epilogue warps have to keep up with the main loop the call per value is what a tile
-// waits for (the shapes above: 352 and 349 us with calls); where eight share the work, as in the dense kernel, the
-// smaller code is the faster one (16 x 4096 rows, N 12288, K 3072, tanh form: 3743 us with calls, 3819 us inline).
+// The same out of line. Beside the dequantizers the call per value is what a tile waits for (the shapes above, four
+// epilogue warps: 352 and 349 us with calls); in the dense kernel the smaller code is the faster one (16 x 4096 rows, N
+// 12288, K 3072, tanh form: 3743 us with calls, 3819 us inline).
 static __device__ __noinline__ float gelu_erf_call(float v) { return gelu_erf(v); }
 static __device__ __noinline__ float gelu_tanh_call(float v) { return gelu_tanh(v); }
 
