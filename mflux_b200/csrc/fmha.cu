@@ -30,6 +30,7 @@
 #include <cstdlib>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 
 namespace mfx {
@@ -241,6 +242,8 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  allow_successor();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -605,6 +608,8 @@ sdpa_pingpong_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  allow_successor();
 
   if (warp == PRODUCER_WARP) {
     // ------------------------------------------------------------ TMA producer
@@ -965,15 +970,14 @@ int run(const Call& c, cudaStream_t stream) {
       if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(pp::sdpa_pingpong_kernel<true>),
                                        pp::DYN_BYTES2, configured))
         return rc;
-      pp::sdpa_pingpong_kernel<true><<<grid, pp::NT, pp::DYN_BYTES2, stream>>>(tq, tk, tv, p);
+      MFX_CUDA_TRY(launch_overlapped(pp::sdpa_pingpong_kernel<true>, grid, pp::NT, pp::DYN_BYTES2, stream, tq, tk, tv, p));
     } else {
       static SmemConfigured configured;
       if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(pp::sdpa_pingpong_kernel<false>),
                                        pp::DYN_BYTES2, configured))
         return rc;
-      pp::sdpa_pingpong_kernel<false><<<grid, pp::NT, pp::DYN_BYTES2, stream>>>(tq, tk, tv, p);
+      MFX_CUDA_TRY(launch_overlapped(pp::sdpa_pingpong_kernel<false>, grid, pp::NT, pp::DYN_BYTES2, stream, tq, tk, tv, p));
     }
-    MFX_CUDA_TRY(cudaGetLastError());
     return MFX_OK;
   }
   dim3 grid(static_cast<unsigned>((seq + BQ - 1) / BQ), static_cast<unsigned>(heads), static_cast<unsigned>(batch));
@@ -981,14 +985,13 @@ int run(const Call& c, cudaStream_t stream) {
     static SmemConfigured configured;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(sdpa_pair_kernel<true>), DYN_BYTES, configured))
       return rc;
-    sdpa_pair_kernel<true><<<grid, NUM_THREADS, DYN_BYTES, stream>>>(tq, tk, tv, p);
+    MFX_CUDA_TRY(launch_overlapped(sdpa_pair_kernel<true>, grid, NUM_THREADS, DYN_BYTES, stream, tq, tk, tv, p));
   } else {
     static SmemConfigured configured;
     if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(sdpa_pair_kernel<false>), DYN_BYTES, configured))
       return rc;
-    sdpa_pair_kernel<false><<<grid, NUM_THREADS, DYN_BYTES, stream>>>(tq, tk, tv, p);
+    MFX_CUDA_TRY(launch_overlapped(sdpa_pair_kernel<false>, grid, NUM_THREADS, DYN_BYTES, stream, tq, tk, tv, p));
   }
-  MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
 

@@ -13,6 +13,7 @@
 #include <cuda_fp16.h>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 #include "scalar.cuh"
 
 namespace mfx {
@@ -163,6 +164,8 @@ constexpr int NORM_MID_D = 3072;
 // 9.3 us.
 template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
 __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormParams p) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   constexpr int E = 16 / sizeof(XT);
   constexpr int MAXV = MAX_D / E / NORM_THREADS;
   __shared__ float red[2][2][4];
@@ -186,7 +189,7 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormP
   };
   ChannelVec<E, BF> scale_v[MAXV], shift_v[MAXV], weight_v[MAXV];
   int mods_of = -1;                       // the sample whose shift and scale are held
-  unsigned row_id = blockIdx.x;
+  unsigned row_id = block;
   int parity = 0;
   fetch(row_id);
   for (; row_id < total; row_id += gridDim.x, parity ^= 1) {
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormP
 }
 
 template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
-void launch_norm_one(const NormParams& p, cudaStream_t st) {
+cudaError_t launch_norm_one(const NormParams& p, cudaStream_t st) {
   // As many blocks as are resident at a time. More only add block starts (65536 x 3072 float32 rows, us, at 4 resident
   // blocks per SM: 4 blocks 218, 8 219, 24 224; 4608 rows 14.3, 15.2, 17.5), fewer rows than that take a block each.
   auto kern = norm_modulate_kernel<XT, BF, MAX_D, MOD, WEIGHT>;
@@ -264,26 +267,25 @@ void launch_norm_one(const NormParams& p, cudaStream_t st) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NORM_THREADS, 0) == cudaSuccess && n > 0 ? n : 4;
   }();
   const int64_t total = static_cast<int64_t>(p.rows) * p.batch, resident = per_sm * device_sm_count();
-  kern<<<static_cast<unsigned>(total < resident ? total : resident), NORM_THREADS, 0, st>>>(p);
+  return launch_overlapped(kern, static_cast<unsigned>(total < resident ? total : resident), NORM_THREADS, 0, st, p);
 }
 template <typename XT, int MAX_D>
-void launch_norm_d(const NormParams& p, cudaStream_t st) {
+cudaError_t launch_norm_d(const NormParams& p, cudaStream_t st) {
   const bool mod = p.shift || p.scale, weight = p.weight != nullptr;
   const bool bf = (!mod || p.mod_dtype == MFX_BF16) && (!weight || p.weight_dtype == MFX_BF16);
-  if (bf && mod && !weight) launch_norm_one<XT, true, MAX_D, true, false>(p, st);
-  else if (bf && !mod && weight) launch_norm_one<XT, true, MAX_D, false, true>(p, st);
-  else if (bf && mod) launch_norm_one<XT, true, MAX_D, true, true>(p, st);
-  else if (weight) launch_norm_one<XT, false, MAX_D, true, true>(p, st);
-  else launch_norm_one<XT, false, MAX_D, true, false>(p, st);
+  if (bf && mod && !weight) return launch_norm_one<XT, true, MAX_D, true, false>(p, st);
+  if (bf && !mod && weight) return launch_norm_one<XT, true, MAX_D, false, true>(p, st);
+  if (bf && mod) return launch_norm_one<XT, true, MAX_D, true, true>(p, st);
+  if (weight) return launch_norm_one<XT, false, MAX_D, true, true>(p, st);
+  return launch_norm_one<XT, false, MAX_D, true, false>(p, st);
 }
-void launch_norm(int x_dtype, const NormParams& p, cudaStream_t st) {
+cudaError_t launch_norm(int x_dtype, const NormParams& p, cudaStream_t st) {
   if (x_dtype == MFX_F32) {
-    if (p.D <= NORM_MID_D) launch_norm_d<float, NORM_MID_D>(p, st);
-    else launch_norm_d<float, NORM_MAX_D>(p, st);
-  } else {
-    if (p.D <= NORM_MID_D) launch_norm_d<__nv_bfloat16, NORM_MID_D>(p, st);
-    else launch_norm_d<__nv_bfloat16, NORM_MAX_D>(p, st);
+    if (p.D <= NORM_MID_D) return launch_norm_d<float, NORM_MID_D>(p, st);
+    return launch_norm_d<float, NORM_MAX_D>(p, st);
   }
+  if (p.D <= NORM_MID_D) return launch_norm_d<__nv_bfloat16, NORM_MID_D>(p, st);
+  return launch_norm_d<__nv_bfloat16, NORM_MAX_D>(p, st);
 }
 
 struct PostNormParams {
@@ -320,11 +322,13 @@ struct PostNormParams {
 // (transformer_block.py:34 after :31, and the next block's :29-30 after :35), which saves reading the stream again.
 template <typename YT, bool BF>
 __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const PostNormParams p) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   constexpr int E = 4;
   constexpr int MAXV = NORM_MAX_D / E / NORM_THREADS;
   __shared__ float red[4], red2[4];
   const int t = threadIdx.x;
-  const int64_t row_id = blockIdx.x;
+  const int64_t row_id = block;
   const int b = static_cast<int>(row_id / p.rows);
   const int r = static_cast<int>(row_id % p.rows);
   const YT* y = static_cast<const YT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride;
@@ -432,9 +436,11 @@ struct RopeParams {
 // arithmetic; the RMS reduction runs inside a half warp.
 constexpr int ROPE_HEADS = 4;
 __global__ void __launch_bounds__(256) qknorm_rope_kernel(const RopeParams p) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = (p.heads + ROPE_HEADS - 1) / ROPE_HEADS;
-  const int64_t item = static_cast<int64_t>(blockIdx.x) * 8 + warp;
+  const int64_t item = static_cast<int64_t>(block) * 8 + warp;
   const int64_t total = static_cast<int64_t>(p.batch) * p.seq * groups;
   if (item >= total) return;
   const int h0 = static_cast<int>(item % groups) * ROPE_HEADS;
@@ -499,8 +505,10 @@ __global__ void __launch_bounds__(256) qknorm_rope_kernel(const RopeParams p) {
 __global__ void __launch_bounds__(256) act_mul_kernel(__nv_bfloat16* y, int64_t y_row_stride, int64_t y_batch_stride,
                                                           const __nv_bfloat16* g, int64_t g_row_stride,
                                                           int64_t g_batch_stride, int rows, int batch, int D, int act) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   const int vec_per_row = D / 8;
-  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t idx = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
   const int64_t total = static_cast<int64_t>(batch) * rows * vec_per_row;
   if (idx >= total) return;
   const int c = static_cast<int>(idx % vec_per_row) * 8;
@@ -525,7 +533,9 @@ __global__ void __launch_bounds__(256) act_mul_kernel(__nv_bfloat16* y, int64_t 
 // out[i] = f(a[i] (+ b[i]) (+ c[i])), f = identity, SiLU or tanh; out dtype bf16 or f32.
 __global__ void __launch_bounds__(256) vec_sum_act_kernel(const void* a, const void* b, const void* c, int in_dtype,
                                                           int act, void* out, int out_dtype, int64_t n) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float v = load_as_float(a, in_dtype, i);
   if (b) v += load_as_float(b, in_dtype, i);
@@ -539,7 +549,9 @@ __global__ void __launch_bounds__(256) vec_sum_act_kernel(const void* a, const v
 // latents_out = latents + noise * dt  (flow-matching Euler step)
 __global__ void __launch_bounds__(256) euler_step_kernel(const void* latents, int lat_dtype, const void* noise,
                                                          int noise_dtype, float dt, void* out, int64_t n) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float v = load_as_float(latents, lat_dtype, i) + load_as_float(noise, noise_dtype, i) * dt;
   if (lat_dtype == MFX_F32) static_cast<float*>(out)[i] = v;
@@ -558,7 +570,9 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const void* __restri
                                                             float* out, int64_t res_row_stride,
                                                             int64_t res_batch_stride, int64_t rows_per_batch,
                                                             int64_t D, int64_t n_vec) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // one 8-element vector
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;  // one 8-element vector
   if (i >= n_vec) return;
   const int64_t vec_per_row = D >> 3;
   const int64_t row = i / vec_per_row;
@@ -587,8 +601,10 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const void* __restri
 __global__ void __launch_bounds__(256) cfg_combine_kernel(const void* __restrict__ n, const void* __restrict__ nn,
                                                           int dtype, float g, int mode, float* __restrict__ out,
                                                           int64_t rows, int C) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + warp;
+  const int64_t row = static_cast<int64_t>(block) * 8 + warp;
   if (row >= rows) return;
   float sn = 0.f, sc = 0.f;
   for (int c = lane; c < C; c += 32) {
@@ -652,8 +668,7 @@ int mfx_norm_modulate(const mfx_norm_args* a, void* stream) {
   p.y_batch_stride = a->y_batch_stride;
   const int64_t total = a->rows * a->batch;
   if (total > 0x7fffffffll) return MFX_ERR_TOO_LARGE;
-  launch_norm(a->x_dtype, p, static_cast<cudaStream_t>(stream));
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_norm(a->x_dtype, p, static_cast<cudaStream_t>(stream)));
   return MFX_OK;
 }
 
@@ -675,10 +690,10 @@ int mfx_act_mul(void* y, int64_t y_row_stride, int64_t y_batch_stride, const voi
   if (rows > (1ll << 30) || batch > 65535) return MFX_ERR_TOO_LARGE;
   if (int rc = check_arch()) return rc;
   const int64_t total = rows * batch * (D / 8);
-  glue::act_mul_kernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+  MFX_CUDA_TRY(launch_overlapped(glue::act_mul_kernel, static_cast<unsigned>((total + 255) / 256), 256, 0,
+      static_cast<cudaStream_t>(stream),
       static_cast<__nv_bfloat16*>(y), y_row_stride, y_batch_stride, static_cast<const __nv_bfloat16*>(gate),
-      g_row_stride, g_batch_stride, static_cast<int>(rows), static_cast<int>(batch), static_cast<int>(D), act);
-  MFX_CUDA_TRY(cudaGetLastError());
+      g_row_stride, g_batch_stride, static_cast<int>(rows), static_cast<int>(batch), static_cast<int>(D), act));
   return MFX_OK;
 }
 
@@ -715,8 +730,8 @@ int mfx_qknorm_rope_gqa(void* qkv, int64_t row_stride, int64_t batch_stride, int
   p.cos_sin = cos_sin;
   p.eps = eps;
   const int64_t total = seq * batch * ((heads + glue::ROPE_HEADS - 1) / glue::ROPE_HEADS);
-  qknorm_rope_kernel<<<static_cast<unsigned>((total + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(qknorm_rope_kernel, static_cast<unsigned>((total + 7) / 8), 256, 0,
+                                 static_cast<cudaStream_t>(stream), p));
   return MFX_OK;
 }
 
@@ -727,9 +742,8 @@ int mfx_vec_sum_act(const void* a, const void* b, const void* c, int in_dtype, i
   if (n <= 0 || act < 0 || act > 2) return MFX_ERR_SHAPE;
   if (!valid_dtype(in_dtype) || (out_dtype != MFX_F32 && out_dtype != MFX_BF16)) return MFX_ERR_DTYPE;
   if (int rc = check_arch()) return rc;
-  glue::vec_sum_act_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      a, b, c, in_dtype, act, out, out_dtype, n);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(glue::vec_sum_act_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0,
+                                 static_cast<cudaStream_t>(stream), a, b, c, in_dtype, act, out, out_dtype, n));
   return MFX_OK;
 }
 
@@ -740,9 +754,8 @@ int mfx_euler_step(const void* latents, int lat_dtype, const void* noise, int no
   if (n <= 0) return MFX_ERR_SHAPE;
   if (!valid_dtype(lat_dtype) || !valid_dtype(noise_dtype)) return MFX_ERR_DTYPE;
   if (int rc = check_arch()) return rc;
-  glue::euler_step_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      latents, lat_dtype, noise, noise_dtype, dt, out, n);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(glue::euler_step_kernel, static_cast<unsigned>((n + 255) / 256), 256, 0,
+                                 static_cast<cudaStream_t>(stream), latents, lat_dtype, noise, noise_dtype, dt, out, n));
   return MFX_OK;
 }
 
@@ -759,10 +772,9 @@ int mfx_gate_residual(const void* y, int y_dtype, const void* bias, int bias_dty
   if (res_row_stride < D) return MFX_ERR_SHAPE;
   if (int rc = check_arch()) return rc;
   const int64_t n_vec = batch * rows * D / 8;
-  glue::gate_residual_kernel<<<static_cast<unsigned>((n_vec + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      y, y_dtype, bias, bias_dtype, gate, gate_dtype, gate_batch_stride, residual, out, res_row_stride, res_batch_stride, rows,
-      D, n_vec);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(glue::gate_residual_kernel, static_cast<unsigned>((n_vec + 255) / 256), 256, 0,
+      static_cast<cudaStream_t>(stream), y, y_dtype, bias, bias_dtype, gate, gate_dtype, gate_batch_stride, residual, out, res_row_stride, res_batch_stride, rows,
+      D, n_vec));
   return MFX_OK;
 }
 
@@ -824,14 +836,10 @@ int mfx_post_pre_norm(const mfx_post_pre_norm_args* a, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool bf = p.weight_dtype == MFX_BF16 && (!p.gate || p.gate_dtype == MFX_BF16) &&
                   (!p.next_out || (p.next_weight_dtype == MFX_BF16 && (!p.next_scale || p.next_scale_dtype == MFX_BF16)));
-  if (a->y_dtype == MFX_F32) {
-    if (bf) norm_gate_residual_kernel<float, true><<<blocks, NORM_THREADS, 0, st>>>(p);
-    else norm_gate_residual_kernel<float, false><<<blocks, NORM_THREADS, 0, st>>>(p);
-  } else {
-    if (bf) norm_gate_residual_kernel<__nv_bfloat16, true><<<blocks, NORM_THREADS, 0, st>>>(p);
-    else norm_gate_residual_kernel<__nv_bfloat16, false><<<blocks, NORM_THREADS, 0, st>>>(p);
-  }
-  MFX_CUDA_TRY(cudaGetLastError());
+  auto kern = a->y_dtype == MFX_F32 ? (bf ? norm_gate_residual_kernel<float, true> : norm_gate_residual_kernel<float, false>)
+                                    : (bf ? norm_gate_residual_kernel<__nv_bfloat16, true>
+                                          : norm_gate_residual_kernel<__nv_bfloat16, false>);
+  MFX_CUDA_TRY(launch_overlapped(kern, blocks, NORM_THREADS, 0, st, p));
   return MFX_OK;
 }
 
@@ -867,9 +875,9 @@ int mfx_cfg_combine(const void* noise, const void* noise_negative, int dtype, fl
   if (rows <= 0 || channels <= 0 || channels > 1024 || (mode != 0 && mode != 1)) return MFX_ERR_SHAPE;
   if (!valid_dtype(dtype)) return MFX_ERR_DTYPE;
   if (int rc = check_arch()) return rc;
-  glue::cfg_combine_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      noise, noise_negative, dtype, guidance, mode, out, rows, static_cast<int>(channels));
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(glue::cfg_combine_kernel, static_cast<unsigned>((rows + 7) / 8), 256, 0,
+                                 static_cast<cudaStream_t>(stream), noise, noise_negative, dtype, guidance, mode, out, rows,
+                                 static_cast<int>(channels)));
   return MFX_OK;
 }
 

@@ -29,6 +29,7 @@
 #include <string.h>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "qmm_common.cuh"
 #include "qmm_dense.cuh"
@@ -197,6 +198,8 @@ qmm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ C
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  allow_successor();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer of the activation tiles
@@ -634,8 +637,7 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   auto kern = qmm_kernel<BITS, BNH, WF, ST, SD, OUT, EPI, NDQ, TEAMS, EPI_WARPS, EXT>;
   static SmemConfigured configured;  // one record per instantiation of the kernel
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), L::DYN_BYTES, configured)) return rc;
-  kern<<<grid, NUM_THREADS, L::DYN_BYTES, st>>>(tx, tw, tsb, tt, tlb, p);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(kern, grid, NUM_THREADS, L::DYN_BYTES, st, tx, tw, tsb, tt, tlb, p));
   return MFX_OK;
 }
 

@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 #include "ptx.cuh"
 #include "qmm_common.cuh"
 #include "qmm_dense.cuh"
@@ -121,6 +122,8 @@ dense_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__
   cluster_sync_all();  // both CTAs' barriers exist before anyone signals across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  wait_for_predecessor();
+  allow_successor();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -255,7 +258,9 @@ constexpr int DEC_ITERS = 3;
 template <int BITS>
 __global__ void __launch_bounds__(256) decode_kernel(const uint8_t* __restrict__ codes, const uint32_t* __restrict__ sb,
                                                      int N, int K, __nv_bfloat16* __restrict__ out) {
-  const int n = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int n = block * 8 + (threadIdx.x >> 5);
   if (n >= N) return;
   const int kb = blockIdx.y * (DEC_ITERS * 512) + (threadIdx.x & 31) * 16;
   const int64_t row = static_cast<int64_t>(n) * K;
@@ -311,8 +316,7 @@ int launch(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& tt, 
   auto kern = dense_kernel<OUT, EPI, EXT>;
   static SmemConfigured configured;  // one record per instantiation of the kernel
   if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), DYN_BYTES, configured)) return rc;
-  kern<<<grid, NUM_THREADS, DYN_BYTES, st>>>(tx, tw, tt, tlb, p);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(kern, grid, NUM_THREADS, DYN_BYTES, st, tx, tw, tt, tlb, p));
   return MFX_OK;
 }
 
@@ -367,9 +371,7 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, voi
                    static_cast<unsigned>((K + DEC_ITERS * 512 - 1) / (DEC_ITERS * 512)));
   if (dgrid.y > 65535) return MFX_ERR_TOO_LARGE;
   __nv_bfloat16* w = static_cast<__nv_bfloat16*>(scratch);
-  if (kb == 4) decode_kernel<4><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
-  else decode_kernel<8><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
-  MFX_CUDA_TRY(cudaGetLastError());
+  MFX_CUDA_TRY(launch_overlapped(kb == 4 ? decode_kernel<4> : decode_kernel<8>, dgrid, 256, 0, st, codes, sb, N, K, w));
 
   CUtensorMap tx, tw, tt, tlb;
   const uint32_t box[3] = {BK, 128, 1};

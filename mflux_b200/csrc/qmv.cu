@@ -18,6 +18,7 @@
 #include <cuda_fp16.h>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 #include "scalar.cuh"
 #include "qmv.cuh"
 
@@ -91,13 +92,15 @@ __device__ __forceinline__ void deq8_word(uint32_t w, uint64_t sc2, uint64_t bi2
 // R = groups of 8 weight rows per warp (the A fragments are reused across them). BITS = 4 or 8.
 template <int BITS, int R>
 __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
   constexpr int KPL = 128 / BITS;            // k values a lane covers per slice with one 16-byte load: 32 or 16
   constexpr int SLICE = 4 * KPL;             // k per slice: 128 (4-bit) or 64 (8-bit)
   constexpr int STEPS = KPL / 4;             // mma steps per slice: 8 or 4
   __shared__ float red[WARPS][R][32][4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int n_base = blockIdx.x * (8 * R);
+  const int n_base = block * (8 * R);
   const int words_per_row = p.K * BITS / 32;
   const int slices = (p.K + SLICE - 1) / SLICE;
 
@@ -218,14 +221,9 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, cud
   // registers and leave two blocks per SM: 10-25 % slower on 9216 to 18432 rows)
   const bool wide = (a.N + 15) / 16 >= 2 * device_sm_count();
   const unsigned blocks = static_cast<unsigned>(wide ? (a.N + 15) / 16 : (a.N + 7) / 8);
-  if (kernel_bits(a.bits) == 4) {
-    if (wide) qmv_kernel<4, 2><<<blocks, THREADS, 0, st>>>(p);
-    else qmv_kernel<4, 1><<<blocks, THREADS, 0, st>>>(p);
-  } else {
-    if (wide) qmv_kernel<8, 2><<<blocks, THREADS, 0, st>>>(p);
-    else qmv_kernel<8, 1><<<blocks, THREADS, 0, st>>>(p);
-  }
-  MFX_CUDA_TRY(cudaGetLastError());
+  auto kern = kernel_bits(a.bits) == 4 ? (wide ? qmv_kernel<4, 2> : qmv_kernel<4, 1>)
+                                       : (wide ? qmv_kernel<8, 2> : qmv_kernel<8, 1>);
+  MFX_CUDA_TRY(launch_overlapped(kern, blocks, THREADS, 0, st, p));
   return MFX_OK;
 }
 

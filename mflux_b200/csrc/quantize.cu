@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "host_util.cuh"
+#include "launch.cuh"
 
 namespace mfx {
 namespace {
@@ -111,7 +112,9 @@ template <typename T, int BITS, int QMODE, int PT>
 __global__ void __launch_bounds__(128) quantize_kernel(const T* __restrict__ w, int64_t n_groups_total,
                                                        uint32_t* __restrict__ wq, T* __restrict__ scales,
                                                        T* __restrict__ biases) {
-  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int64_t tid = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
   constexpr int LANES = 64 / PT;                  // of a group
   const int64_t group = tid / LANES;
   const bool active = group < n_groups_total;
@@ -233,7 +236,9 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
                                                          const SB* __restrict__ scales,
                                                          const SB* __restrict__ biases, int64_t n_chunks,
                                                          OUT* __restrict__ out) {
-  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const unsigned block = wait_for_predecessor();
+  allow_successor();
+  const int64_t tid = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
   if (tid >= n_chunks) return;
   const int64_t g = tid / (64 / V);
   const float s = to_f32<SB>(scales[g]);
@@ -290,12 +295,12 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
 }
 
 template <typename T, int BITS, int PT>
-void launch_quantize_pt(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases, cudaStream_t st) {
+cudaError_t launch_quantize_pt(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases,
+                               cudaStream_t st) {
   const unsigned blocks = static_cast<unsigned>((n_groups * (64 / PT) + 127) / 128);
-  if (qmode == MFX_QMODE_MLX)
-    quantize_kernel<T, BITS, MFX_QMODE_MLX, PT><<<blocks, 128, 0, st>>>(w, n_groups, wq, scales, biases);
-  else
-    quantize_kernel<T, BITS, MFX_QMODE_DOC, PT><<<blocks, 128, 0, st>>>(w, n_groups, wq, scales, biases);
+  return launch_overlapped(qmode == MFX_QMODE_MLX ? quantize_kernel<T, BITS, MFX_QMODE_MLX, PT>
+                                                  : quantize_kernel<T, BITS, MFX_QMODE_DOC, PT>,
+                           blocks, 128, 0, st, w, n_groups, wq, scales, biases);
 }
 
 // Values a thread takes of 16-bit weights: 32 share the scale's divisions once there are threads enough without 16. us,
@@ -304,11 +309,12 @@ void launch_quantize_pt(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T
 // would need 128 bytes per thread at 32: 28 us at 16 for 12288 x 3072, 37 at 32 (29 before).
 constexpr int64_t LARGE_WEIGHT = 4 << 20;
 template <typename T, int BITS>
-void launch_quantize_bits(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases, cudaStream_t st) {
+cudaError_t launch_quantize_bits(const T* w, int64_t n_groups, int qmode, uint32_t* wq, T* scales, T* biases,
+                                 cudaStream_t st) {
   if constexpr (sizeof(T) == 2) {
     if (n_groups * 64 >= LARGE_WEIGHT) return launch_quantize_pt<T, BITS, 32>(w, n_groups, qmode, wq, scales, biases, st);
   }
-  launch_quantize_pt<T, BITS, 16>(w, n_groups, qmode, wq, scales, biases, st);
+  return launch_quantize_pt<T, BITS, 16>(w, n_groups, qmode, wq, scales, biases, st);
 }
 
 template <typename T>
@@ -318,20 +324,19 @@ int launch_quantize(const void* w, int64_t n_groups, int bits, int qmode, uint32
   T* sp = static_cast<T*>(scales);
   T* bp = static_cast<T*>(biases);
   switch (bits) {
-    case 3: launch_quantize_bits<T, 3>(wp, n_groups, qmode, wq, sp, bp, st); break;
-    case 4: launch_quantize_bits<T, 4>(wp, n_groups, qmode, wq, sp, bp, st); break;
-    case 5: launch_quantize_bits<T, 5>(wp, n_groups, qmode, wq, sp, bp, st); break;
-    case 6: launch_quantize_bits<T, 6>(wp, n_groups, qmode, wq, sp, bp, st); break;
-    case 8: launch_quantize_bits<T, 8>(wp, n_groups, qmode, wq, sp, bp, st); break;
+    case 3: MFX_CUDA_TRY((launch_quantize_bits<T, 3>(wp, n_groups, qmode, wq, sp, bp, st))); break;
+    case 4: MFX_CUDA_TRY((launch_quantize_bits<T, 4>(wp, n_groups, qmode, wq, sp, bp, st))); break;
+    case 5: MFX_CUDA_TRY((launch_quantize_bits<T, 5>(wp, n_groups, qmode, wq, sp, bp, st))); break;
+    case 6: MFX_CUDA_TRY((launch_quantize_bits<T, 6>(wp, n_groups, qmode, wq, sp, bp, st))); break;
+    case 8: MFX_CUDA_TRY((launch_quantize_bits<T, 8>(wp, n_groups, qmode, wq, sp, bp, st))); break;
     default: return MFX_ERR_UNSUPPORTED_BITS;
   }
-  MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
 
 template <typename SB, typename OUT, int BITS>
-void launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* biases, int64_t values, OUT* out,
-                            cudaStream_t st) {
+cudaError_t launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* biases, int64_t values, OUT* out,
+                                   cudaStream_t st) {
   auto blocks = [&](int v) { return static_cast<unsigned>((values / v + 255) / 256); };
   // Sixteen values a thread halve the threads and the scale loads, which pays once the output fills the GPU many times
   // over (8 M values of float32, 32 M of 16 bits); below that fewer threads hide less of a trip to memory, and at 5 and 6
@@ -341,9 +346,9 @@ void launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* bias
   // 1024 x 3072, 3 bits 5.9 / 6.0; 256 x 256 2.1 / 2.3.
   constexpr bool few = sizeof(OUT) == 2 && (BITS == 5 || BITS == 6);
   if (!few && values >= (sizeof(OUT) == 4 ? 8 << 20 : 32 << 20))
-    dequantize_kernel<SB, OUT, BITS, 16><<<blocks(16), 256, 0, st>>>(wq, scales, biases, values / 16, out);
-  else
-    dequantize_kernel<SB, OUT, BITS, 8><<<blocks(8), 256, 0, st>>>(wq, scales, biases, values / 8, out);
+    return launch_overlapped(dequantize_kernel<SB, OUT, BITS, 16>, blocks(16), 256, 0, st, wq, scales, biases, values / 16,
+                             out);
+  return launch_overlapped(dequantize_kernel<SB, OUT, BITS, 8>, blocks(8), 256, 0, st, wq, scales, biases, values / 8, out);
 }
 
 template <typename SB, typename OUT>
@@ -353,14 +358,13 @@ int launch_dequantize(const uint32_t* wq, const void* scales, const void* biases
   const SB* bp = static_cast<const SB*>(biases);
   OUT* op = static_cast<OUT*>(out);
   switch (bits) {
-    case 3: launch_dequantize_bits<SB, OUT, 3>(wq, sp, bp, values, op, st); break;
-    case 4: launch_dequantize_bits<SB, OUT, 4>(wq, sp, bp, values, op, st); break;
-    case 5: launch_dequantize_bits<SB, OUT, 5>(wq, sp, bp, values, op, st); break;
-    case 6: launch_dequantize_bits<SB, OUT, 6>(wq, sp, bp, values, op, st); break;
-    case 8: launch_dequantize_bits<SB, OUT, 8>(wq, sp, bp, values, op, st); break;
+    case 3: MFX_CUDA_TRY((launch_dequantize_bits<SB, OUT, 3>(wq, sp, bp, values, op, st))); break;
+    case 4: MFX_CUDA_TRY((launch_dequantize_bits<SB, OUT, 4>(wq, sp, bp, values, op, st))); break;
+    case 5: MFX_CUDA_TRY((launch_dequantize_bits<SB, OUT, 5>(wq, sp, bp, values, op, st))); break;
+    case 6: MFX_CUDA_TRY((launch_dequantize_bits<SB, OUT, 6>(wq, sp, bp, values, op, st))); break;
+    case 8: MFX_CUDA_TRY((launch_dequantize_bits<SB, OUT, 8>(wq, sp, bp, values, op, st))); break;
     default: return MFX_ERR_UNSUPPORTED_BITS;
   }
-  MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
 
