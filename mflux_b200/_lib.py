@@ -291,8 +291,22 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
+    _host().bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in
+                   ("mfx_qlinear_ex", "mfx_qlinear_scratch_bytes_batch", "mfx_qlinear_prepared_bytes")))
     _lib = lib
     return lib
+
+
+def _host():
+    """The native form of a quantized linear's call (csrc/host_call.cpp)."""
+    import torch  # noqa: F401  (brings the libraries the module is linked against)
+
+    try:
+        from . import _host as host
+    except ImportError as e:
+        raise RuntimeError("mflux_b200/_host.so is missing or was built for another torch: run `python -m "
+                           f"mflux_b200.build` ({e})") from e
+    return host
 
 
 def check(status: int, what: str) -> None:

@@ -1,15 +1,17 @@
-"""In-tree build of libmfx.so (sm_100a only) with nvcc. No GPU is needed to build.
+"""In-tree build of libmfx.so (sm_100a only) with nvcc and of the host module _host.so with g++. No GPU is needed to build.
 
 Usage: python -m mflux_b200.build [--force] [--verbose]
-Objects are rebuilt only when their source (or a header) is newer. The shared library lands next
-to this file so that it travels with the source tree.
+Objects are rebuilt only when their source (or a header) is newer. The shared libraries land next
+to this file so that they travel with the source tree.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -17,6 +19,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OBJ = PKG / "build"
 LIB = PKG / "libmfx.so"
+HOST = PKG / "_host.so"
 ROOT = PKG.parent
 
 NVCC_FLAGS = [
@@ -45,6 +48,22 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
         return True
     t = obj.stat().st_mtime
     return any(p.stat().st_mtime > t for p in [src, *headers])
+
+
+def build_host(force: bool, headers: list[Path]) -> None:
+    """The CPython module of csrc/host_call.cpp, against the headers and libraries of the installed torch."""
+    src = CSRC / "host_call.cpp"
+    if not force and not _stale(HOST, src, headers):
+        return
+    torch = Path(importlib.util.find_spec("torch").origin).parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+           "-I", str(ROOT / "include"), "-I", str(torch / "include"), "-I", str(torch / "include/torch/csrc/api/include"),
+           "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"], str(src), "-o", str(HOST),
+           "-L", str(torch / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"build of {HOST.name} failed:\n{r.stdout}\n{r.stderr}")
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -78,6 +97,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_host(force, headers)
     return LIB
 
 

@@ -184,6 +184,10 @@ class QuantizedLinear(Module):
                 residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
         weight, scales, biases, bias = self._tensors()
+        if out is None and gate is None and residual is None and out_dtype is None and self._prepared is not None:
+            y = ops.plain_qlinear(x, weight, scales, biases, bias, self._prepared, self.bits, self.group_size, epilogue)
+            if y is not None:
+                return y
         return ops.qlinear(x, weight, scales, biases, bias, bits=self.bits, group_size=self.group_size,
                            epilogue=epilogue, gate=gate, residual=residual, out=out, out_dtype=out_dtype,
                            prepared=self.prepared())

@@ -326,6 +326,24 @@ def qlinear(x: torch.Tensor, wq: torch.Tensor, scales: torch.Tensor, biases: tor
     return ret
 
 
+_native = None
+
+
+def plain_qlinear(x, wq, scales, biases, bias, prepared, bits: int, group_size: int, epilogue: str | None):
+    """The common form of a module's call in native code, or None where qlinear() has to take it (csrc/host_call.cpp says
+    when). `prepared` is nn.QuantizedLinear's (key, blob) pair; a key that no longer fits its tensors gives None too."""
+    global _native
+    if TRACE is not None:
+        return None
+    if _native is None:
+        _lib.load()
+        _native = _lib._host().linear
+    y = _native(x, wq, scales, biases, bias, prepared, bits, group_size, _EPI[epilogue])
+    if y is not None:
+        LAUNCHES[0] += 1
+    return y
+
+
 def norm_modulate(x: torch.Tensor, shift: torch.Tensor | None = None, scale: torch.Tensor | None = None, *,
                   weight: torch.Tensor | None = None, eps: float = 1e-6, rms: bool = False,
                   out: torch.Tensor | None = None) -> torch.Tensor:
