@@ -36,6 +36,12 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+__device__ __forceinline__ void st_32(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z),
+               "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+
 // The PT (16 or 32) values of a thread as they lie in memory: 16-bit values two to a register, whose extremes are taken in
 // pairs.
 template <typename T, int PT>
@@ -235,7 +241,7 @@ template <typename SB, typename OUT, int BITS, int V>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restrict__ wq,
                                                          const SB* __restrict__ scales,
                                                          const SB* __restrict__ biases, int64_t n_chunks,
-                                                         OUT* __restrict__ out) {
+                                                         bool wide, OUT* __restrict__ out) {
   const unsigned block = wait_for_predecessor();
   allow_successor();
   const int64_t tid = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
@@ -290,8 +296,15 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
     res[i] = from_f32<OUT>(__fadd_rn(__fmul_rn(c, s), b));
   }
   uint4* dst = reinterpret_cast<uint4*>(out + tid * V);
+  const uint4* from = reinterpret_cast<const uint4*>(res);
+  constexpr int VECS = V * static_cast<int>(sizeof(OUT)) / 16;
+  if (VECS > 1 && wide) {
 #pragma unroll
-  for (int i = 0; i < V * static_cast<int>(sizeof(OUT)) / 16; ++i) dst[i] = reinterpret_cast<const uint4*>(res)[i];
+    for (int i = 0; i + 1 < VECS; i += 2) st_32(dst + i, from[i], from[i + 1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) dst[i] = from[i];
+  }
 }
 
 template <typename T, int BITS, int PT>
@@ -338,17 +351,17 @@ template <typename SB, typename OUT, int BITS>
 cudaError_t launch_dequantize_bits(const uint32_t* wq, const SB* scales, const SB* biases, int64_t values, OUT* out,
                                    cudaStream_t st) {
   auto blocks = [&](int v) { return static_cast<unsigned>((values / v + 255) / 256); };
-  // Sixteen values a thread halve the threads and the scale loads, which pays once the output fills the GPU many times
-  // over (8 M values of float32, 32 M of 16 bits); below that fewer threads hide less of a trip to memory, and at 5 and 6
-  // bits the gathering of ten or twelve bytes from 16-bit words outweighs it in 16-bit outputs. Buffers past L2, us, 8 / 16
-  // values: to bf16, 12288 x 3072, 4 bits 22.4 / 22.0, 8 bits 22.9 / 21.9, 6 bits 25.5 / 26.9; 6144 x 3072, 3 bits 12.1 /
-  // 12.5; 3072 x 3072, 4 bits 6.9 / 7.2, 6 bits 8.1 / 9.0; to float32, 3072 x 3072, 4 bits 12.9 / 12.7, 6 bits 14.8 / 13.5;
-  // 1024 x 3072, 3 bits 5.9 / 6.0; 256 x 256 2.1 / 2.3.
-  constexpr bool few = sizeof(OUT) == 2 && (BITS == 5 || BITS == 6);
-  if (!few && values >= (sizeof(OUT) == 4 ? 8 << 20 : 32 << 20))
+  // Sixteen values a thread, stored 32 bytes at a time, from 8 M values on; below that fewer threads hide less of a trip to
+  // memory. Stores are what bounds it: 16 bytes at a time leave half of every sector to a second instruction. Buffers past
+  // L2, us, 16-byte stores / 8 values and 32-byte stores where 8 values have them / 16: to bf16, 12288 x 3072, 4 bits 21.9 /
+  // 21.9 / 17.0, 6 bits 25.2 / 24.4 / 20.7, 3072 x 3072, 4 bits 5.0 / 5.6 / 4.3, 6 bits 6.1 / 6.2 / 5.3, 3072 x 1024, 4 bits
+  // 2.7 / 2.5 / 2.5; to float32, 12288 x 3072, 4 bits 42.9 / - / 26.9, 3072 x 1024 4.9 / 3.0 / 3.6.
+  const bool wide = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;   // the entry point promises 16
+  if (wide && values >= (8 << 20))
     return launch_overlapped(dequantize_kernel<SB, OUT, BITS, 16>, blocks(16), 256, 0, st, wq, scales, biases, values / 16,
-                             out);
-  return launch_overlapped(dequantize_kernel<SB, OUT, BITS, 8>, blocks(8), 256, 0, st, wq, scales, biases, values / 8, out);
+                             wide, out);
+  return launch_overlapped(dequantize_kernel<SB, OUT, BITS, 8>, blocks(8), 256, 0, st, wq, scales, biases, values / 8, wide,
+                           out);
 }
 
 template <typename SB, typename OUT>
