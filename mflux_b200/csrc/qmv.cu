@@ -9,13 +9,17 @@
 //     k-slots of a step with its own four consecutive k, and reads the same four k of x for A: a dot product does
 //     not care about the order of its terms, so no shuffle is needed to match the instruction's k layout;
 //   * the eight warps' partial sums meet in shared memory; bias, SiLU and the store follow.
-// Measured, the kernel moves 1.0-2.0 TB/s and its time follows the number of weights, not their bytes: the
-// legacy mma.sync path (one m16n8k16 per 128 weights) and the per-weight unpack bound it, not HBM.
+// Measured, the kernel moves 1.0-2.0 TB/s and its time follows the number of weights, not their bytes: five instructions
+// per weight (issue slots 65 % busy while a block runs) and the trips to memory of short-lived blocks bound it, not HBM. At
+// most eight rows over a large weight go to the kernel in namespace stream below.
 // Reference call sites: every nn.Linear that is applied to a conditioning vector, e.g. the AdaLayerNormZero
 // linears (src/mflux/models/flux/model/flux_transformer/ada_layer_norm_zero.py:16-18) and the time/text
 // embedders (time_text_embed.py:19-31); after quantization they are mlx.nn.QuantizedLinear like all others.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "host_util.cuh"
 #include "launch.cuh"
@@ -198,6 +202,312 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
   }
 }
 
+// At most eight rows over a large weight: one block of 16 warps per SM, every warp with a ring of its own in shared memory
+// that cp.async fills a piece ahead, so that the copies run on while the warps compute. A piece is 16 weight rows x 256
+// bytes of codes (512 or 256 k) and their (scale, bias) pairs. S warps share a tile of 16 rows; tiles are dealt out to the
+// blocks in turn.
+// Instructions are the next bound, so no weight is formed: the products are Sum x (128 + code) (4 bits) or Sum x code (8
+// bits) of one group on mma.sync, with the weights as the 16-row operand, and scale, bias and the offset come in once per
+// group, in float32: scale * (P - 128 X) + bias * X with X = Sum x, which every block computes once. That leaves out the
+// rounding of the weights to bf16, too: 1e-6 (4 bits) and 1e-7 (8 bits) from float64 in the 2-norm, where the other kernels
+// are 1.1e-3 off.
+namespace stream {
+
+constexpr int NWARPS = 16;
+constexpr int ROWS = 16;                    // weight rows per tile
+constexpr int MAX_SMEM = 227 * 1024;
+constexpr int ROW_BYTES = 256;              // codes of one row in a piece
+constexpr int RING = 2;                     // 128-byte pieces with 4 or 5 in a ring: 10 % slower
+constexpr int CODES_BYTES = ROWS * ROW_BYTES;
+
+template <int BITS>
+struct Piece {
+  static constexpr int K = ROW_BYTES * 8 / BITS;       // 512 or 256
+  static constexpr int GROUPS = K / 64;                // 8 or 4
+  static constexpr int BYTES = CODES_BYTES + GROUPS * ROWS * 4;
+};
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// 16 codes of one weight row in K order as the A fragments of four products, pairs 2 i and 2 i + 1 of product i; 4 bits:
+// 128 + code, 8 bits: the code, both exact in bf16.
+__device__ __forceinline__ void unpack16(const uint2& w, uint32_t (&a)[8]) {
+  const uint32_t v[2] = {w.x, w.y};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) a[i] = ((v[i >> 2] >> (4 * (i & 3))) & 0x000F000Fu) | MAGIC;
+}
+__device__ __forceinline__ void unpack16(const uint4& w, uint32_t (&a)[8]) {
+  constexpr uint32_t TWO23 = 0x4B000000u;
+  const uint64_t neg = 0xCB000000CB000000ull;  // (-2^23, -2^23)
+  const uint32_t v[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {                // prepared byte order e0, e2, e1, e3
+    uint64_t f;
+    asm("mov.b64 %0, {%1, %2};"
+        : "=l"(f)
+        : "r"(__byte_perm(v[i >> 1], TWO23, i & 1 ? 0x7441 : 0x7440)),
+          "r"(__byte_perm(v[i >> 1], TWO23, i & 1 ? 0x7443 : 0x7442)));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f) : "l"(neg));
+    uint32_t lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(f));
+    a[i] = __byte_perm(lo, hi, 0x7632);        // eight significant bits: the upper halves are exact
+  }
+}
+
+// Shared memory: rings | partial sums [NWARPS][4][32] | X [K / 64][8] | x [M][K] bf16, rows 16 bytes apart (two rows of a
+// quarter warp then read different halves of the banks).
+template <int BITS>
+__host__ __device__ constexpr int x_offset() {
+  return NWARPS * RING * Piece<BITS>::BYTES + NWARPS * 4 * 32 * 4;
+}
+
+// One output term by term, on weights rounded to bf16. For sums that are not finite: where an activation is infinite or near
+// the largest float, P and 128 X (or bias * X) are infinities of either sign although the terms' own sum is not NaN.
+template <int BITS>
+__device__ __noinline__ float direct_dot(const uint32_t* row, const uint32_t* sb, int64_t sb_stride,
+                                         const __nv_bfloat16* x_row, int K) {
+  const unsigned short* x = reinterpret_cast<const unsigned short*>(x_row);
+  float sum = 0.f;
+  for (int k = 0; k < K; ++k) {
+    const uint32_t pair = __ldg(sb + (k >> 6) * sb_stride);
+    constexpr int PER_WORD = 32 / BITS;
+    const int e = k % PER_WORD;                // prepared order: nibbles e0,e2,e4,e6,e1,e3,e5,e7; bytes e0,e2,e1,e3
+    const int at = BITS == 4 ? (e >> 1) + 4 * (e & 1) : (e >> 1) + 2 * (e & 1);
+    const uint32_t code = (__ldg(row + k / PER_WORD) >> (BITS * at)) & ((1u << BITS) - 1u);
+    const float w = fmaf(static_cast<float>(code), __uint_as_float(pair << 16), __uint_as_float(pair & 0xFFFF0000u));
+    const float xv = __uint_as_float(static_cast<uint32_t>(__ldg(x + k)) << 16);
+    sum = fmaf(__bfloat162float(__float2bfloat16_rn(w)), xv, sum);
+  }
+  return sum;
+}
+
+template <int BITS>
+int smem_bytes(int M, int K) {
+  return x_offset<BITS>() + K / 64 * 32 + M * (2 * K + 16);
+}
+
+template <int BITS, int S>
+__global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) {
+  using P = Piece<BITS>;
+  using Codes = typename std::conditional<BITS == 4, uint2, uint4>::type;   // a lane's 16 codes of a group
+  constexpr int TILES = NWARPS / S;          // tiles a block works on at a time
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int block = static_cast<int>(wait_for_predecessor());
+  allow_successor();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int part = warp % S, slot = warp / S;
+  const int groups = p.K >> 6;
+  const int tiles = (p.N + ROWS - 1) / ROWS;
+  const int pieces = (groups + P::GROUPS - 1) / P::GROUPS;
+  const int mine = part < pieces ? (pieces - part + S - 1) / S : 0;          // pieces of a tile that are this warp's
+  const int rounds = (tiles + TILES * static_cast<int>(gridDim.x) - 1) / (TILES * static_cast<int>(gridDim.x));
+  const int64_t row_bytes = static_cast<int64_t>(p.K) * BITS / 8;
+  uint8_t* ring = smem + warp * (RING * P::BYTES);
+  const uint32_t ring_s = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
+  float* red = reinterpret_cast<float*>(smem + NWARPS * RING * P::BYTES);
+  float* xsum = reinterpret_cast<float*>(smem + x_offset<BITS>());
+  auto tile_of = [&](int round) { return (round * TILES + slot) * static_cast<int>(gridDim.x) + block; };
+
+  // piece number `k` of this warp's sequence (rounds one after the other) into ring slot k % RING
+  int next = 0, next_round = 0, next_piece = part;
+  auto issue = [&]() {
+    if (next_round < rounds && mine > 0) {
+      const int tile = tile_of(next_round);
+      if (tile < tiles) {
+        const uint32_t dst = ring_s + (next % RING) * P::BYTES;
+        const int n0 = tile * ROWS;
+        const int64_t off = static_cast<int64_t>(next_piece) * ROW_BYTES;
+#pragma unroll
+        for (int i = 0; i < CODES_BYTES / 16 / 32; ++i) {
+          const int id = i * 32 + lane, row = id / (ROW_BYTES / 16), c = id % (ROW_BYTES / 16);
+          // 16-byte chunks swizzled so that the rows of a quarter or half warp read different banks
+          const int cs = BITS == 4 ? c ^ ((row & 3) << 1) : c ^ ((row & 1) << 2);
+          if (off + c * 16 < row_bytes)
+            cp_async16(dst + row * ROW_BYTES + cs * 16,
+                       reinterpret_cast<const uint8_t*>(p.codes) + min(n0 + row, p.N - 1) * row_bytes + off + c * 16);
+        }
+        const int grp = next_piece * P::GROUPS + (lane >> 2), n = n0 + (lane & 3) * 4;
+        if (lane < P::GROUPS * 4 && grp < groups && n < p.N)
+          cp_async16(dst + CODES_BYTES + lane * 16, p.sb + static_cast<int64_t>(grp) * p.N + n);
+      }
+      ++next;
+      next_piece += S;
+      if (next_piece >= pieces) {
+        next_piece = part;
+        ++next_round;
+      }
+    }
+    cp_async_commit();
+  };
+  for (int i = 0; i < RING - 1; ++i) issue();
+
+  const int x_pitch = 2 * p.K + 16;
+  uint8_t* xs_mem = smem + x_offset<BITS>() + groups * 32;
+  for (int m = 0; m < p.M; ++m)
+    for (int c = threadIdx.x; c < p.K / 8; c += NWARPS * 32)
+      *reinterpret_cast<uint4*>(xs_mem + m * x_pitch + c * 16) =
+          __ldg(reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride) + c);
+  const uint8_t* x_mine = xs_mem + min(g, p.M - 1) * x_pitch + t * 32;
+
+  // X[group][m]: four lanes sum a group of one row, 16 activations each
+  for (int i = threadIdx.x; i < groups * p.M * 4; i += NWARPS * 32) {
+    const int m = (i >> 2) / groups, grp = (i >> 2) - m * groups;
+    const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride + grp * 64 + (i & 3) * 16);
+    const uint4 v0 = __ldg(src), v1 = __ldg(src + 1);
+    const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+    float a = 0.f, b = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      a += __uint_as_float(w[j] << 16);
+      b += __uint_as_float(w[j] & 0xFFFF0000u);
+    }
+    a += b;
+    const unsigned quad = 0xFu << (threadIdx.x & 28);    // the four lanes take the branch together
+    a += __shfl_xor_sync(quad, a, 1);
+    a += __shfl_xor_sync(quad, a, 2);
+    if ((i & 3) == 0) xsum[grp * 8 + m] = a;
+  }
+  __syncthreads();
+
+  int k = 0;
+  for (int round = 0; round < rounds; ++round) {
+    const int tile = tile_of(round);
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < mine; ++i, ++k) {
+      __syncwarp();                          // the slot the next copies go to has been read
+      issue();
+      cp_async_wait<RING - 1>();
+      __syncwarp();                          // every lane's copies of piece k have landed
+      if (tile >= tiles) continue;
+      const uint8_t* src = ring + (k % RING) * P::BYTES;
+      const int g0 = (part + i * S) * P::GROUPS;
+#pragma unroll
+      for (int j = 0; j < P::GROUPS; ++j) {
+        if (g0 + j >= groups) break;
+        const uint4 v0 = *reinterpret_cast<const uint4*>(x_mine + (g0 + j) * 128);
+        const uint4 v1 = *reinterpret_cast<const uint4*>(x_mine + (g0 + j) * 128 + 16);
+        const int at = BITS == 4 ? ((2 * j) ^ ((g & 3) << 1)) * 16 + t * 8 : ((4 * j) ^ ((g & 1) << 2)) * 16 + t * 16;
+        uint32_t lo[8], hi[8];
+        unpack16(*reinterpret_cast<const Codes*>(src + g * ROW_BYTES + at), lo);
+        unpack16(*reinterpret_cast<const Codes*>(src + (g + 8) * ROW_BYTES + at), hi);
+        const uint32_t* pr = reinterpret_cast<const uint32_t*>(src + CODES_BYTES) + j * ROWS + g;
+        const uint32_t p_lo = pr[0], p_hi = pr[8];
+        const float2 xs = *reinterpret_cast<const float2*>(xsum + (g0 + j) * 8 + 2 * t);
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_16816(d, lo[0], hi[0], lo[1], hi[1], v0.x, v0.y);
+        mma_16816(d, lo[2], hi[2], lo[3], hi[3], v0.z, v0.w);
+        mma_16816(d, lo[4], hi[4], lo[5], hi[5], v1.x, v1.y);
+        mma_16816(d, lo[6], hi[6], lo[7], hi[7], v1.z, v1.w);
+        if (BITS == 4) {
+          d[0] = fmaf(-128.f, xs.x, d[0]);
+          d[1] = fmaf(-128.f, xs.y, d[1]);
+          d[2] = fmaf(-128.f, xs.x, d[2]);
+          d[3] = fmaf(-128.f, xs.y, d[3]);
+        }
+        const float s_lo = __uint_as_float(p_lo << 16), b_lo = __uint_as_float(p_lo & 0xFFFF0000u);
+        const float s_hi = __uint_as_float(p_hi << 16), b_hi = __uint_as_float(p_hi & 0xFFFF0000u);
+        acc[0] = fmaf(s_lo, d[0], fmaf(b_lo, xs.x, acc[0]));
+        acc[1] = fmaf(s_lo, d[1], fmaf(b_lo, xs.y, acc[1]));
+        acc[2] = fmaf(s_hi, d[2], fmaf(b_hi, xs.x, acc[2]));
+        acc[3] = fmaf(s_hi, d[3], fmaf(b_hi, xs.y, acc[3]));
+      }
+    }
+    if constexpr (S > 1) {
+      if (round > 0) __syncthreads();        // the sums of the round before have been read
+#pragma unroll
+      for (int i = 0; i < 4; ++i) red[(warp * 4 + i) * 32 + lane] = acc[i];
+      __syncthreads();
+      if (part == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int o = 1; o < S; ++o) acc[i] += red[((warp + o) * 4 + i) * 32 + lane];
+      }
+    }
+    if (part != 0 || tile >= tiles) continue;
+    // accumulator i of lane (g, t): weight row g + 8 * (i >> 1) of the tile, activation row 2 t + (i & 1)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int n = tile * ROWS + 8 * h + g;
+      if (n >= p.N) continue;
+      const float bias = p.bias ? load_as_float(p.bias, p.bias_dtype, n) : 0.f;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int row = 2 * t + i;
+        if (row >= p.M) continue;
+        float v = acc[2 * h + i];
+        if (!(fabsf(v) <= 3.0e38f)) 
+          v = direct_dot<BITS>(p.codes + n * (row_bytes / 4), p.sb + n, p.N, p.x + row * p.x_row_stride, p.K);
+        v += bias;
+        if (p.epilogue == MFX_EPI_SILU) v = v / (1.0f + __expf(-v));
+        if (p.y_dtype == MFX_F32) static_cast<float*>(p.y)[row * p.y_row_stride + n] = v;
+        else static_cast<__nv_bfloat16*>(p.y)[row * p.y_row_stride + n] = __float2bfloat16_rn(v);
+      }
+    }
+  }
+}
+
+template <int BITS, int S>
+int launch(const Params& p, cudaStream_t st) {
+  static SmemConfigured configured;
+  if (int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(stream_kernel<BITS, S>), MAX_SMEM, configured)) return rc;
+  const int blocks = std::min(device_sm_count(), (p.N + ROWS - 1) / ROWS);
+  MFX_CUDA_TRY(launch_overlapped(stream_kernel<BITS, S>, blocks, NWARPS * 32, smem_bytes<BITS>(p.M, p.K), st, p));
+  return MFX_OK;
+}
+
+// Warps per tile: the fewest that leave a warp three pieces with all tiles at work in one round (the second and third piece
+// come in under the first), else those with the fewest pieces per warp over all rounds. us at 1 / 2 / 4 / 8, one row: N 18432,
+// K 3072, 4 bits 13.1 / 12.4 / 15.8 / 16.3; N 9216, K 3072, 8 bits 12.9 / 10.7 / 10.1 / 11.0; N 20480, K 3840, 8 bits 24.0 /
+// 25.1 / 23.1 / 23.1; N 3072, K 15360, 4 bits 37.2 / 20.8 / 16.7 / 15.6.
+template <int BITS>
+int split(const Params& p) {
+  const int64_t tiles = (p.N + ROWS - 1) / ROWS, pieces = (p.K + Piece<BITS>::K - 1) / Piece<BITS>::K;
+  const int64_t warps = static_cast<int64_t>(NWARPS) * device_sm_count();
+  int best = 1;
+  int64_t best_cost = 0;
+  for (int s = 1; s <= 8; s *= 2) {
+    const int64_t rounds = (tiles * s + warps - 1) / warps, each = (pieces + s - 1) / s;
+    if (rounds == 1 && each <= 3) return s;
+    if (s == 1 || rounds * each < best_cost) {
+      best = s;
+      best_cost = rounds * each;
+    }
+  }
+  return best;
+}
+
+template <int BITS>
+int run(const Params& p, cudaStream_t st) {
+  switch (split<BITS>(p)) {
+    case 1: return launch<BITS, 1>(p, st);
+    case 2: return launch<BITS, 2>(p, st);
+    case 4: return launch<BITS, 4>(p, st);
+    default: return launch<BITS, 8>(p, st);
+  }
+}
+
+// From 24 M weights on; with fewer the start of a block of this size is what a call takes (N 6144, K 3072, 4 bits, three
+// rows: 8.6 us against 7.5), from there on us, the other kernel / this one: N 9216, K 3072, 4 bits, two rows 10.1 / 9.2; one
+// row, 4 bits, N 18432, K 3072 15.8 / 12.4 and N 3072, K 15360 16.4 / 15.6; 8 bits, N 12288, K 3072 15.4 / 12.7, N 20480, K
+// 3840 27.0 / 23.1; eight rows N 18432, K 3072, 4 bits 16.6 / 15.2, N 11520, K 3840, 8 bits 18.6 / 17.9. A plain read of the
+// 33 MB of the third takes 6.2 us.
+template <int BITS>
+bool pays(const Params& p) {
+  return p.M <= 8 && static_cast<int64_t>(p.N) * p.K >= (24ll << 20) && p.K <= (1 << 20) &&
+         smem_bytes<BITS>(p.M, p.K) <= MAX_SMEM;
+}
+
+}  // namespace stream
+
 bool eligible(const mfx_qlinear_args& a) {
   return a.batch == 1 && a.rows <= 16 && (a.epilogue == MFX_EPI_NONE || a.epilogue == MFX_EPI_SILU);
 }
@@ -217,6 +527,8 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, cud
   p.y = a.y;
   p.y_dtype = a.y_dtype;
   p.y_row_stride = a.y_row_stride;
+  if (kernel_bits(a.bits) == 4 ? stream::pays<4>(p) : stream::pays<8>(p))
+    return kernel_bits(a.bits) == 4 ? stream::run<4>(p, st) : stream::run<8>(p, st);
   // 16 rows per block while that still gives every SM two blocks, else 8 rows per block (32 rows per block take 100
   // registers and leave two blocks per SM: 10-25 % slower on 9216 to 18432 rows)
   const bool wide = (a.N + 15) / 16 >= 2 * device_sm_count();
