@@ -258,9 +258,8 @@ constexpr int DEC_ITERS = 3;
 template <int BITS>
 __global__ void __launch_bounds__(256) decode_kernel(const uint8_t* __restrict__ codes, const uint32_t* __restrict__ sb,
                                                      int N, int K, __nv_bfloat16* __restrict__ out) {
-  const unsigned block = wait_for_predecessor();
   allow_successor();
-  const int n = block * 8 + (threadIdx.x >> 5);
+  const int n = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (n >= N) return;
   const int kb = blockIdx.y * (DEC_ITERS * 512) + (threadIdx.x & 31) * 16;
   const int64_t row = static_cast<int64_t>(n) * K;
@@ -371,7 +370,12 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, voi
                    static_cast<unsigned>((K + DEC_ITERS * 512 - 1) / (DEC_ITERS * 512)));
   if (dgrid.y > 65535) return MFX_ERR_TOO_LARGE;
   __nv_bfloat16* w = static_cast<__nv_bfloat16*>(scratch);
-  MFX_CUDA_TRY(launch_overlapped(kb == 4 ? decode_kernel<4> : decode_kernel<8>, dgrid, 256, 0, st, codes, sb, N, K, w));
+  // An ordinary launch: its thousands of blocks, started early, would sit on the SMs that the kernel before is still to use
+  // (8 bits, M 4096, N 12288, K 3072: 252.1 us, overlapped 255.0, both kernels ordinary 252.5; M 73728, N 9216, 4 bits: 3018,
+  // 3027, 3032).
+  if (kb == 4) decode_kernel<4><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
+  else decode_kernel<8><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
+  MFX_CUDA_TRY(cudaGetLastError());
 
   CUtensorMap tx, tw, tt, tlb;
   const uint32_t box[3] = {BK, 128, 1};
