@@ -773,8 +773,8 @@ int mfx_gate_residual(const void* y, int y_dtype, const void* bias, int bias_dty
   if (int rc = check_arch()) return rc;
   const int64_t n_vec = batch * rows * D / 8;
   MFX_CUDA_TRY(launch_overlapped(glue::gate_residual_kernel, static_cast<unsigned>((n_vec + 255) / 256), 256, 0,
-      static_cast<cudaStream_t>(stream), y, y_dtype, bias, bias_dtype, gate, gate_dtype, gate_batch_stride, residual, out, res_row_stride, res_batch_stride, rows,
-      D, n_vec));
+      static_cast<cudaStream_t>(stream), y, y_dtype, bias, bias_dtype, gate, gate_dtype, gate_batch_stride, residual, out,
+      res_row_stride, res_batch_stride, rows, D, n_vec));
   return MFX_OK;
 }
 

@@ -10,8 +10,8 @@
 //     not care about the order of its terms, so no shuffle is needed to match the instruction's k layout;
 //   * the eight warps' partial sums meet in shared memory; bias, SiLU and the store follow.
 // Measured, the kernel moves 1.0-2.0 TB/s and its time follows the number of weights, not their bytes: five instructions
-// per weight (issue slots 65 % busy while a block runs) and the trips to memory of short-lived blocks bound it, not HBM. At
-// most eight rows over a large weight go to the kernel in namespace stream below.
+// per weight (issue slots 65 % busy while a block runs) and the trips to memory of short-lived blocks bound it, not HBM. A
+// few rows over a large weight go to the kernel in namespace stream below.
 // Reference call sites: every nn.Linear that is applied to a conditioning vector, e.g. the AdaLayerNormZero
 // linears (src/mflux/models/flux/model/flux_transformer/ada_layer_norm_zero.py:16-18) and the time/text
 // embedders (time_text_embed.py:19-31); after quantization they are mlx.nn.QuantizedLinear like all others.
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
   }
 }
 
-// At most eight rows over a large weight: one block of 16 warps per SM, every warp with a ring of its own in shared memory
+// A few rows over a large weight: one block of 16 warps per SM, every warp with a ring of its own in shared memory
 // that cp.async fills a piece ahead, so that the copies run on while the warps compute. A piece is 16 weight rows x 256
 // bytes of codes (512 or 256 k) and their (scale, bias) pairs. S warps share a tile of 16 rows; tiles are dealt out to the
 // blocks in turn.
@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) 
   // X[group][m]: four lanes sum a group of one row, 16 activations each
   for (int i = threadIdx.x; i < groups * p.M * 4; i += NWARPS * 32) {
     const int m = (i >> 2) / groups, grp = (i >> 2) - m * groups;
-    const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride + grp * 64 + (i & 3) * 16);
+    const uint4* src =
+        reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride + grp * 64 + (i & 3) * 16);
     const uint4 v0 = __ldg(src), v1 = __ldg(src + 1);
     const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     float a = 0.f, b = 0.f;
@@ -464,22 +465,22 @@ int launch(const Params& p, cudaStream_t st) {
   return MFX_OK;
 }
 
-// Warps per tile: the fewest that leave a warp three pieces with all tiles at work in one round (the second and third piece
-// come in under the first), else those with the fewest pieces per warp over all rounds. us at 1 / 2 / 4 / 8, one row: N 18432,
-// K 3072, 4 bits 13.1 / 12.4 / 15.8 / 16.3; N 9216, K 3072, 8 bits 12.9 / 10.7 / 10.1 / 11.0; N 20480, K 3840, 8 bits 24.0 /
-// 25.1 / 23.1 / 23.1; N 3072, K 15360, 4 bits 37.2 / 20.8 / 16.7 / 15.6.
+// Warps per tile, by pieces a warp has over all rounds, a piece and a half for the barriers of every further round and 1.2 for
+// every doubling of the warps that add their sums. us at 1 / 2 / 4 / 8, one row: N 18432, K 3072, 4 bits 13.1 / 12.4 / 15.8 /
+// 16.3; N 9216, K 3072, 4 bits 10.6 / 9.2 / 10.4 / 10.8, 8 bits 12.9 / 10.7 / 10.1 / 11.0; N 12288, K 3072, 8 bits 16.5 / 12.7
+// / 13.9 / 14.2; N 20480, K 3840, 8 bits 24.0 / 25.1 / 23.1 / 23.1; N 3072, K 15360, 4 bits 37.2 / 20.8 / 16.7 / 15.6.
 template <int BITS>
 int split(const Params& p) {
   const int64_t tiles = (p.N + ROWS - 1) / ROWS, pieces = (p.K + Piece<BITS>::K - 1) / Piece<BITS>::K;
   const int64_t warps = static_cast<int64_t>(NWARPS) * device_sm_count();
   int best = 1;
-  int64_t best_cost = 0;
-  for (int s = 1; s <= 8; s *= 2) {
+  int64_t best_cost = 0;                       // in tenths of a piece
+  for (int s = 1, doublings = 0; s <= 8; s *= 2, ++doublings) {
     const int64_t rounds = (tiles * s + warps - 1) / warps, each = (pieces + s - 1) / s;
-    if (rounds == 1 && each <= 3) return s;
-    if (s == 1 || rounds * each < best_cost) {
+    const int64_t cost = 10 * rounds * each + 15 * (rounds - 1) + 12 * doublings;
+    if (s == 1 || cost < best_cost) {
       best = s;
-      best_cost = rounds * each;
+      best_cost = cost;
     }
   }
   return best;
@@ -496,13 +497,16 @@ int run(const Params& p, cudaStream_t st) {
 }
 
 // From 24 M weights on; with fewer the start of a block of this size is what a call takes (N 6144, K 3072, 4 bits, three
-// rows: 8.6 us against 7.5), from there on us, the other kernel / this one: N 9216, K 3072, 4 bits, two rows 10.1 / 9.2; one
-// row, 4 bits, N 18432, K 3072 15.8 / 12.4 and N 3072, K 15360 16.4 / 15.6; 8 bits, N 12288, K 3072 15.4 / 12.7, N 20480, K
-// 3840 27.0 / 23.1; eight rows N 18432, K 3072, 4 bits 16.6 / 15.2, N 11520, K 3840, 8 bits 18.6 / 17.9. A plain read of the
-// 33 MB of the third takes 6.2 us.
+// rows: 8.6 us against 7.5). The other kernel / this one, at 1, 4, 8 rows: 4 bits, N 9216, K 3072 10.1 / 8.6, 10.2 / 9.7,
+// 10.9 / 11.4; N 11520, K 4096 13.2 / 12.4, 13.3 / 13.5, 14.3 / 15.5; N 12288, K 4096 15.9 / 12.6, 15.9 / 13.8, 16.1 / 15.6;
+// N 20480, K 3840 21.5 / 19.4, 21.8 / 20.6, 22.5 / 22.3; 8 bits, N 8192, K 4096 14.1 / 11.5, 14.1 / 12.7, 14.1 / 14.6; N 15360,
+// K 3840 21.1 / 17.7, 21.2 / 18.9, 21.3 / 20.7. Every row costs here (it is copied into each block's shared memory and its sums
+// per group are formed there) and almost nothing there, so more rows need more weights to read; at 4 bits, three rows, N
+// 10240, K 3840 13.1 / 13.4. A plain read of the 33 MB of the 8-bit N 8192, K 4096 takes 6.2 us.
 template <int BITS>
 bool pays(const Params& p) {
-  return p.M <= 8 && static_cast<int64_t>(p.N) * p.K >= (24ll << 20) && p.K <= (1 << 20) &&
+  const int64_t weights = static_cast<int64_t>(p.N) * p.K;
+  return p.M <= (weights >= (48ll << 20) ? 8 : BITS / 2) && weights >= (24ll << 20) && p.K <= (1 << 20) &&
          smem_bytes<BITS>(p.M, p.K) <= MAX_SMEM;
 }
 
@@ -535,7 +539,11 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, cud
   const unsigned blocks = static_cast<unsigned>(wide ? (a.N + 15) / 16 : (a.N + 7) / 8);
   auto kern = kernel_bits(a.bits) == 4 ? (wide ? qmv_kernel<4, 2> : qmv_kernel<4, 1>)
                                        : (wide ? qmv_kernel<8, 2> : qmv_kernel<8, 1>);
-  MFX_CUDA_TRY(launch_overlapped(kern, blocks, THREADS, 0, st, p));
+  // An ordinary launch: with more blocks than fit at once, those that start early only hold back the ones before them
+  // (overlapped / ordinary: five rows, N 3840, K 12288, 4 bits 20.3 / 17.9 us, four rows, N 3072, K 4096, 8 bits 8.4 / 7.6;
+  // two rows, N 15360, K 256, 8 bits 3.9 / 4.1).
+  kern<<<blocks, THREADS, 0, st>>>(p);
+  MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;
 }
 
