@@ -499,14 +499,15 @@ int run(const Params& p, cudaStream_t st) {
 // From 24 M weights on; with fewer the start of a block of this size is what a call takes (N 6144, K 3072, 4 bits, three
 // rows: 8.6 us against 7.5). The other kernel / this one, at 1, 4, 8 rows: 4 bits, N 9216, K 3072 10.1 / 8.6, 10.2 / 9.7,
 // 10.9 / 11.4; N 11520, K 4096 13.2 / 12.4, 13.3 / 13.5, 14.3 / 15.5; N 12288, K 4096 15.9 / 12.6, 15.9 / 13.8, 16.1 / 15.6;
-// N 20480, K 3840 21.5 / 19.4, 21.8 / 20.6, 22.5 / 22.3; 8 bits, N 8192, K 4096 14.1 / 11.5, 14.1 / 12.7, 14.1 / 14.6; N 15360,
+// N 20480, K 3840 21.5 / 19.4, 21.8 / 20.6, 22.5 / 22.3; 8 bits, N 8192, K 4096 14.1 / 11.5, 14.1 / 12.7, 14.1 / 14.6; N 12288, K
+// 3072 15.5 / 12.3, 15.5 / 13.4, 15.6 / 14.6; N 15360,
 // K 3840 21.1 / 17.7, 21.2 / 18.9, 21.3 / 20.7. Every row costs here (it is copied into each block's shared memory and its sums
 // per group are formed there) and almost nothing there, so more rows need more weights to read; at 4 bits, three rows, N
 // 10240, K 3840 13.1 / 13.4. A plain read of the 33 MB of the 8-bit N 8192, K 4096 takes 6.2 us.
 template <int BITS>
 bool pays(const Params& p) {
   const int64_t weights = static_cast<int64_t>(p.N) * p.K;
-  return p.M <= (weights >= (48ll << 20) ? 8 : BITS / 2) && weights >= (24ll << 20) && p.K <= (1 << 20) &&
+  return p.M <= (weights >= ((BITS == 4 ? 48ll : 36ll) << 20) ? 8 : BITS / 2) && weights >= (24ll << 20) && p.K <= (1 << 20) &&
          smem_bytes<BITS>(p.M, p.K) <= MAX_SMEM;
 }
 

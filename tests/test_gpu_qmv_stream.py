@@ -1,4 +1,4 @@
-"""Few rows over weights of 24 M (two or four rows) and 48 M (eight) and more: every share of a tile's pieces among warps (1, 2, 4, 8), one and several
+"""Few rows over weights of 24 M (two or four rows) and 48 or 36 M (eight) and more: every share of a tile's pieces among warps (1, 2, 4, 8), one and several
 rounds of tiles, a last tile of eight rows, a last piece of one group, activations with row strides, against float64 on the
 packed weights. Bound: float32 sums of up to 15360 terms and, for 4 bits, the offset of 128 that is taken out again (2^-24 of
 128 Sum |x| per group against a result of about 5 |x| sqrt(64) codes: 2e-5 in the worst case, a tenth of it on average)."""
@@ -25,7 +25,7 @@ def test_against_float64(lib_built, n, k, bits):
     q, prepared, w = _weight(n, k, bits)
     g = torch.Generator(device="cuda").manual_seed(1)
     bias = torch.randn(n, device="cuda", generator=g)
-    most = 8 if n * k >= 48 << 20 else 2 if bits <= 4 else 4
+    most = 8 if n * k >= (48 if bits <= 4 else 36) << 20 else 2 if bits <= 4 else 4
     for rows, epilogue in ((1, None), (2, "silu"), (3, None), (4, None), (5, None), (8, None), (9, None)):
         x = torch.randn(rows, k + 64, device="cuda", generator=g).to(torch.bfloat16)[:, 32:32 + k]
         ref = x.double() @ w.t() + bias.double()
