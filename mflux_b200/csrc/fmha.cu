@@ -191,7 +191,7 @@ __device__ __forceinline__ bool any_bias(const float* bp, int keys, int lane) {
   bool mine = false;
 #pragma unroll
   for (int i = 0; i < KEYS; i += 32)
-    if (i + lane < keys) mine |= __ldg(bp + i + lane) != 0.f;   // true for NaN
+    if (i + lane < keys) mine |= bp[i + lane] != 0.f;   // true for NaN
   return __any_sync(0xffffffffu, mine);
 }
 
@@ -362,7 +362,7 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         if (!tail) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const float4 bv = __ldg(reinterpret_cast<const float4*>(bp) + i);
+            const float4 bv = reinterpret_cast<const float4*>(bp)[i];
             sA[4 * i + 0] = __float_as_uint(fmaf(__uint_as_float(sA[4 * i + 0]), p.scale_log2, bv.x * LOG2E));
             sA[4 * i + 1] = __float_as_uint(fmaf(__uint_as_float(sA[4 * i + 1]), p.scale_log2, bv.y * LOG2E));
             sA[4 * i + 2] = __float_as_uint(fmaf(__uint_as_float(sA[4 * i + 2]), p.scale_log2, bv.z * LOG2E));
@@ -371,7 +371,7 @@ sdpa_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         } else {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const float bv = i < keys_here ? __ldg(bp + i) : 0.f;
+            const float bv = i < keys_here ? bp[i] : 0.f;
             sA[i] = __float_as_uint(fmaf(__uint_as_float(sA[i]), p.scale_log2, bv * LOG2E));
           }
         }
@@ -538,7 +538,7 @@ __device__ __forceinline__ void add_bias_chunk(uint32_t (&s)[32], const float* b
   if (valid >= 32) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const float4 bv = __ldg(reinterpret_cast<const float4*>(bp) + i);
+      const float4 bv = reinterpret_cast<const float4*>(bp)[i];
       s[4 * i + 0] = __float_as_uint(fmaf(__uint_as_float(s[4 * i + 0]), scale_log2, bv.x * LOG2E));
       s[4 * i + 1] = __float_as_uint(fmaf(__uint_as_float(s[4 * i + 1]), scale_log2, bv.y * LOG2E));
       s[4 * i + 2] = __float_as_uint(fmaf(__uint_as_float(s[4 * i + 2]), scale_log2, bv.z * LOG2E));
@@ -547,7 +547,7 @@ __device__ __forceinline__ void add_bias_chunk(uint32_t (&s)[32], const float* b
   } else {
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
-      const float bv = i < valid ? __ldg(bp + i) : 0.f;
+      const float bv = i < valid ? bp[i] : 0.f;
       s[i] = __float_as_uint(fmaf(__uint_as_float(s[i]), scale_log2, bv * LOG2E));
     }
   }

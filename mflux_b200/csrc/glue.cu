@@ -125,10 +125,10 @@ struct ChannelVec<E, true> {
   __device__ __forceinline__ void load(const void* ptr, int64_t off) {
     const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(ptr) + off;
     if constexpr (E == 8) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(q));
+      const uint4 v = *reinterpret_cast<const uint4*>(q);
       raw[0] = v.x; raw[1] = v.y; raw[2] = v.z; raw[3] = v.w;
     } else {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(q));
+      const uint2 v = *reinterpret_cast<const uint2*>(q);
       raw[0] = v.x; raw[1] = v.y;
     }
   }
@@ -164,7 +164,7 @@ constexpr int NORM_MID_D = 3072;
 // 9.3 us.
 template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
 __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormParams p) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
   constexpr int E = 16 / sizeof(XT);
   constexpr int MAXV = MAX_D / E / NORM_THREADS;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormP
   };
   ChannelVec<E, BF> scale_v[MAXV], shift_v[MAXV], weight_v[MAXV];
   int mods_of = -1;                       // the sample whose shift and scale are held
-  unsigned row_id = block;
+  unsigned row_id = blockIdx.x;
   int parity = 0;
   fetch(row_id);
   for (; row_id < total; row_id += gridDim.x, parity ^= 1) {
@@ -322,13 +322,13 @@ struct PostNormParams {
 // (transformer_block.py:34 after :31, and the next block's :29-30 after :35), which saves reading the stream again.
 template <typename YT, bool BF>
 __global__ void __launch_bounds__(NORM_THREADS) norm_gate_residual_kernel(const PostNormParams p) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
   constexpr int E = 4;
   constexpr int MAXV = NORM_MAX_D / E / NORM_THREADS;
   __shared__ float red[4], red2[4];
   const int t = threadIdx.x;
-  const int64_t row_id = block;
+  const int64_t row_id = blockIdx.x;
   const int b = static_cast<int>(row_id / p.rows);
   const int r = static_cast<int>(row_id % p.rows);
   const YT* y = static_cast<const YT*>(p.y) + b * p.y_batch_stride + static_cast<int64_t>(r) * p.y_row_stride;
@@ -436,11 +436,11 @@ struct RopeParams {
 // arithmetic; the RMS reduction runs inside a half warp.
 constexpr int ROPE_HEADS = 4;
 __global__ void __launch_bounds__(256) qknorm_rope_kernel(const RopeParams p) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int groups = (p.heads + ROPE_HEADS - 1) / ROPE_HEADS;
-  const int64_t item = static_cast<int64_t>(block) * 8 + warp;
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * 8 + warp;
   const int64_t total = static_cast<int64_t>(p.batch) * p.seq * groups;
   if (item >= total) return;
   const int h0 = static_cast<int>(item % groups) * ROPE_HEADS;
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(256) qknorm_rope_kernel(const RopeParams p) {
   for (int i = 0; i < ROPE_HEADS; ++i)
     raw[i] = h0 + i < my_heads ? *reinterpret_cast<const uint4*>(base + i * 128) : make_uint4(0, 0, 0, 0);
   const float4* csp = reinterpret_cast<const float4*>(p.cos_sin + (static_cast<int64_t>(s) * 64 + 4 * l) * 2);
-  const float4 cs0 = __ldg(csp), cs1 = __ldg(csp + 1);
+  const float4 cs0 = csp[0], cs1 = csp[1];
   const void* w = which == 0 ? (s < p.split ? p.qw_a : p.qw_b) : (s < p.split ? p.kw_a : p.kw_b);
   float wt[8];
   load_vec<8>(w, p.w_dtype, l * 8, wt);
@@ -505,10 +505,10 @@ __global__ void __launch_bounds__(256) qknorm_rope_kernel(const RopeParams p) {
 __global__ void __launch_bounds__(256) act_mul_kernel(__nv_bfloat16* y, int64_t y_row_stride, int64_t y_batch_stride,
                                                           const __nv_bfloat16* g, int64_t g_row_stride,
                                                           int64_t g_batch_stride, int rows, int batch, int D, int act) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
   const int vec_per_row = D / 8;
-  const int64_t idx = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t total = static_cast<int64_t>(batch) * rows * vec_per_row;
   if (idx >= total) return;
   const int c = static_cast<int>(idx % vec_per_row) * 8;
@@ -533,9 +533,9 @@ __global__ void __launch_bounds__(256) act_mul_kernel(__nv_bfloat16* y, int64_t 
 // out[i] = f(a[i] (+ b[i]) (+ c[i])), f = identity, SiLU or tanh; out dtype bf16 or f32.
 __global__ void __launch_bounds__(256) vec_sum_act_kernel(const void* a, const void* b, const void* c, int in_dtype,
                                                           int act, void* out, int out_dtype, int64_t n) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
-  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float v = load_as_float(a, in_dtype, i);
   if (b) v += load_as_float(b, in_dtype, i);
@@ -549,9 +549,9 @@ __global__ void __launch_bounds__(256) vec_sum_act_kernel(const void* a, const v
 // latents_out = latents + noise * dt  (flow-matching Euler step)
 __global__ void __launch_bounds__(256) euler_step_kernel(const void* latents, int lat_dtype, const void* noise,
                                                          int noise_dtype, float dt, void* out, int64_t n) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
-  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float v = load_as_float(latents, lat_dtype, i) + load_as_float(noise, noise_dtype, i) * dt;
   if (lat_dtype == MFX_F32) static_cast<float*>(out)[i] = v;
@@ -563,16 +563,16 @@ __global__ void __launch_bounds__(256) euler_step_kernel(const void* latents, in
 // x[b, r, :] = residual[b, r, :] + gate[b, :] * (y[b, r, :] + bias[:]); residual/x float32 (in place allowed),
 // y bf16 or f32. Used after the all-reduce of a row-split (tensor-parallel) linear, where the gated residual
 // cannot be an epilogue of the matmul because the partial sums of all ranks must be added first.
-__global__ void __launch_bounds__(256) gate_residual_kernel(const void* __restrict__ y, int y_dtype,
-                                                            const void* __restrict__ bias, int bias_dtype,
-                                                            const void* __restrict__ gate, int gate_dtype,
+__global__ void __launch_bounds__(256) gate_residual_kernel(const void* y, int y_dtype,
+                                                            const void* bias, int bias_dtype,
+                                                            const void* gate, int gate_dtype,
                                                             int64_t gate_batch_stride, const float* residual,
                                                             float* out, int64_t res_row_stride,
                                                             int64_t res_batch_stride, int64_t rows_per_batch,
                                                             int64_t D, int64_t n_vec) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
-  const int64_t i = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;  // one 8-element vector
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // one 8-element vector
   if (i >= n_vec) return;
   const int64_t vec_per_row = D >> 3;
   const int64_t row = i / vec_per_row;
@@ -598,13 +598,13 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const void* __restri
 // mode 0: out = n + g * (n - n_neg)                              (z_image.py:209)
 // mode 1: comb = n_neg + g * (n - n_neg); out = comb * ||n|| / ||comb|| over the channel axis, eps 1e-12
 //         (QwenImage.compute_guided_noise, qwen_image.py:165-174)
-__global__ void __launch_bounds__(256) cfg_combine_kernel(const void* __restrict__ n, const void* __restrict__ nn,
-                                                          int dtype, float g, int mode, float* __restrict__ out,
+__global__ void __launch_bounds__(256) cfg_combine_kernel(const void* n, const void* nn,
+                                                          int dtype, float g, int mode, float* out,
                                                           int64_t rows, int C) {
-  const unsigned block = wait_for_predecessor();
+  wait_for_predecessor();
   allow_successor();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = static_cast<int64_t>(block) * 8 + warp;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + warp;
   if (row >= rows) return;
   float sn = 0.f, sc = 0.f;
   for (int c = lane; c < C; c += 32) {

@@ -11,15 +11,12 @@ namespace mfx {
 // to memory that another kernel may write or read. Returns once the predecessor has finished and its writes are visible
 // (at once where the launch was an ordinary one). Every thread of every such kernel calls it before anything else that
 // touches global memory, so a kernel's end still means the end of everything before it in the stream.
-// The value is blockIdx.x as known behind the wait: loads through the read-only path, which the compiler may move across a
-// memory barrier, stay behind it where their addresses come from this value.
+// Such a kernel reads global memory by plain loads, TMA and cp.async only, never by the read-only path (__ldg, const
+// __restrict__): that path is for memory which nobody writes while the kernel lives, and this one lives while its
+// predecessor still writes. The compiler may also move its loads across the wait, a plain load not (the clobber below).
 // Without / with it, looped: 24 heads x 4608 tokens of attention back to back 241.5 / 232.1 us, a step of 380 launches (8-bit
 // single-stream model, 1613 tokens) 22.26 / 21.97 ms, a guidance pair of the dual-stream model at 7145 tokens 248.1 / 246.6.
-__device__ __forceinline__ unsigned wait_for_predecessor() {
-  unsigned block;
-  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, %%ctaid.x;" : "=r"(block) : : "memory");
-  return block;
-}
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // From here on the successor's blocks may be started. They only come to a SM as this kernel's blocks leave it room.
 __device__ __forceinline__ void allow_successor() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -96,7 +96,6 @@ __device__ __forceinline__ void deq8_word(uint32_t w, uint64_t sc2, uint64_t bi2
 // R = groups of 8 weight rows per warp (the A fragments are reused across them). BITS = 4 or 8.
 template <int BITS, int R>
 __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
-  const unsigned block = wait_for_predecessor();
   allow_successor();
   constexpr int KPL = 128 / BITS;            // k values a lane covers per slice with one 16-byte load: 32 or 16
   constexpr int SLICE = 4 * KPL;             // k per slice: 128 (4-bit) or 64 (8-bit)
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(THREADS) qmv_kernel(const Params p) {
   __shared__ float red[WARPS][R][32][4];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int n_base = block * (8 * R);
+  const int n_base = blockIdx.x * (8 * R);
   const int words_per_row = p.K * BITS / 32;
   const int slices = (p.K + SLICE - 1) / SLICE;
 
@@ -276,13 +275,13 @@ __device__ __noinline__ float direct_dot(const uint32_t* row, const uint32_t* sb
   const unsigned short* x = reinterpret_cast<const unsigned short*>(x_row);
   float sum = 0.f;
   for (int k = 0; k < K; ++k) {
-    const uint32_t pair = __ldg(sb + (k >> 6) * sb_stride);
+    const uint32_t pair = sb[(k >> 6) * sb_stride];
     constexpr int PER_WORD = 32 / BITS;
     const int e = k % PER_WORD;                // prepared order: nibbles e0,e2,e4,e6,e1,e3,e5,e7; bytes e0,e2,e1,e3
     const int at = BITS == 4 ? (e >> 1) + 4 * (e & 1) : (e >> 1) + 2 * (e & 1);
-    const uint32_t code = (__ldg(row + k / PER_WORD) >> (BITS * at)) & ((1u << BITS) - 1u);
+    const uint32_t code = (row[k / PER_WORD] >> (BITS * at)) & ((1u << BITS) - 1u);
     const float w = fmaf(static_cast<float>(code), __uint_as_float(pair << 16), __uint_as_float(pair & 0xFFFF0000u));
-    const float xv = __uint_as_float(static_cast<uint32_t>(__ldg(x + k)) << 16);
+    const float xv = __uint_as_float(static_cast<uint32_t>(x[k]) << 16);
     sum = fmaf(__bfloat162float(__float2bfloat16_rn(w)), xv, sum);
   }
   return sum;
@@ -299,8 +298,9 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) 
   using Codes = typename std::conditional<BITS == 4, uint2, uint4>::type;   // a lane's 16 codes of a group
   constexpr int TILES = NWARPS / S;          // tiles a block works on at a time
   extern __shared__ __align__(128) uint8_t smem[];
-  const int block = static_cast<int>(wait_for_predecessor());
+  wait_for_predecessor();
   allow_successor();
+  const int block = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int part = warp % S, slot = warp / S;
@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) 
   for (int m = 0; m < p.M; ++m)
     for (int c = threadIdx.x; c < p.K / 8; c += NWARPS * 32)
       *reinterpret_cast<uint4*>(xs_mem + m * x_pitch + c * 16) =
-          __ldg(reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride) + c);
+          reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride)[c];
   const uint8_t* x_mine = xs_mem + min(g, p.M - 1) * x_pitch + t * 32;
 
   // X[group][m]: four lanes sum a group of one row, 16 activations each
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) 
     const int m = (i >> 2) / groups, grp = (i >> 2) - m * groups;
     const uint4* src =
         reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(m) * p.x_row_stride + grp * 64 + (i & 3) * 16);
-    const uint4 v0 = __ldg(src), v1 = __ldg(src + 1);
+    const uint4 v0 = src[0], v1 = src[1];
     const uint32_t w[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     float a = 0.f, b = 0.f;
 #pragma unroll

@@ -51,7 +51,7 @@ struct Values {
   __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
     for (int i = 0; i < PT / 8; ++i) {
-      const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p) + i);
+      const uint4 raw = reinterpret_cast<const uint4*>(p)[i];
       const Pair* r = reinterpret_cast<const Pair*>(&raw);
 #pragma unroll
       for (int j = 0; j < 4; ++j) h[4 * i + j] = r[j];
@@ -75,7 +75,7 @@ struct Values<float, PT> {
   __device__ __forceinline__ void load(const float* p) {
 #pragma unroll
     for (int i = 0; i < PT / 4; ++i) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(p) + i);
+      const float4 a = reinterpret_cast<const float4*>(p)[i];
       f[4 * i] = a.x; f[4 * i + 1] = a.y; f[4 * i + 2] = a.z; f[4 * i + 3] = a.w;
     }
   }
@@ -115,12 +115,12 @@ __device__ __forceinline__ float exact_code(float d, float scale, float n_bins) 
 // of at most n_bins + 1, so a product further than that from every k + 0.5 rounds like the quotient. Values nearer to one
 // (one in 1000 at 4 bits) are divided.
 template <typename T, int BITS, int QMODE, int PT>
-__global__ void __launch_bounds__(128) quantize_kernel(const T* __restrict__ w, int64_t n_groups_total,
-                                                       uint32_t* __restrict__ wq, T* __restrict__ scales,
-                                                       T* __restrict__ biases) {
-  const unsigned block = wait_for_predecessor();
+__global__ void __launch_bounds__(128) quantize_kernel(const T* w, int64_t n_groups_total,
+                                                       uint32_t* wq, T* scales,
+                                                       T* biases) {
+  wait_for_predecessor();
   allow_successor();
-  const int64_t tid = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
+  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   constexpr int LANES = 64 / PT;                  // of a group
   const int64_t group = tid / LANES;
   const bool active = group < n_groups_total;
@@ -238,13 +238,13 @@ __global__ void __launch_bounds__(128) quantize_kernel(const T* __restrict__ w, 
 
 // One thread: V (8 or 16) consecutive outputs of a row.
 template <typename SB, typename OUT, int BITS, int V>
-__global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restrict__ wq,
-                                                         const SB* __restrict__ scales,
-                                                         const SB* __restrict__ biases, int64_t n_chunks,
-                                                         bool wide, OUT* __restrict__ out) {
-  const unsigned block = wait_for_predecessor();
+__global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* wq,
+                                                         const SB* scales,
+                                                         const SB* biases, int64_t n_chunks,
+                                                         bool wide, OUT* out) {
+  wait_for_predecessor();
   allow_successor();
-  const int64_t tid = static_cast<int64_t>(block) * blockDim.x + threadIdx.x;
+  const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (tid >= n_chunks) return;
   const int64_t g = tid / (64 / V);
   const float s = to_f32<SB>(scales[g]);
@@ -254,12 +254,12 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
     constexpr int WORDS = V * BITS / 32;
     uint32_t words[WORDS];
     if constexpr (WORDS == 1) {
-      words[0] = __ldg(wq + tid);
+      words[0] = wq[tid];
     } else if constexpr (WORDS == 2) {
-      const uint2 v = __ldg(reinterpret_cast<const uint2*>(wq) + tid);
+      const uint2 v = reinterpret_cast<const uint2*>(wq)[tid];
       words[0] = v.x; words[1] = v.y;
     } else {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(wq) + tid);
+      const uint4 v = reinterpret_cast<const uint4*>(wq)[tid];
       words[0] = v.x; words[1] = v.y; words[2] = v.z; words[3] = v.w;
     }
 #pragma unroll
@@ -271,13 +271,13 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint32_t* __restr
       const uint8_t* src = reinterpret_cast<const uint8_t*>(wq) + tid * BITS;
       eight[0] = 0;
 #pragma unroll
-      for (int i = 0; i < BITS; ++i) eight[0] |= static_cast<unsigned long long>(__ldg(src + i)) << (8 * i);
+      for (int i = 0; i < BITS; ++i) eight[0] |= static_cast<unsigned long long>(src[i]) << (8 * i);
     } else {
       const uint16_t* src = reinterpret_cast<const uint16_t*>(wq) + tid * BITS;
       unsigned long long w0 = 0, w1 = 0;
 #pragma unroll
       for (int i = 0; i < BITS; ++i) {
-        const unsigned long long v = __ldg(src + i);
+        const unsigned long long v = src[i];
         if (i < 4) w0 |= v << (16 * i);
         else w1 |= v << (16 * (i & 3));
       }
