@@ -52,13 +52,79 @@ def _chain(rows, d, heads, sync):
     return step, x0
 
 
-@pytest.mark.parametrize("rows,d,heads", [(1, 256, 2), (40, 256, 2), (300, 768, 6), (2100, 512, 4)])
-def test_chain(lib_built, rows, d, heads):
+def _large_chain(batch, rows, sync):
+    """The kernels that only larger calls reach, each behind the producer of what it reads: few rows over weights of 24 M
+    and more (the ring form), prepared beforehand and in the call, the decoded form, attention with a key bias (both
+    kernels by the rows), an adapter, a fork to another stream and its join, and the element-wise kernels."""
+    from mflux_b200 import nn, ops
+    from mflux_b200.lora import LoRALinear
+
+    d, heads, wide = 3072, 24, 12288
+    g = torch.Generator(device="cuda").manual_seed(rows)
+
+    def rnd(*shape, scale=1.0, dtype=torch.bfloat16):
+        return (torch.randn(*shape, device="cuda", generator=g) * scale).to(dtype)
+
+    def linear(n, k, bits):
+        lin = nn.Linear(k, n, device="cuda")
+        lin.weight.data.copy_(rnd(n, k, scale=0.02))
+        layer = lin.to_quantized(bits=bits)
+        layer.prepared()
+        return layer
+
+    cond, cond8, qkv_l, out_l, up, down = (linear(3 * d, d, 4), linear(3 * d, d, 8), linear(3 * d, d, 4),
+                                           linear(d, d, 8), linear(wide, d, 8), linear(d, wide, 4))
+    lora = LoRALinear.from_linear(linear(d, d, 4), r=16, scale=0.5)
+    lora.lora_A.data.copy_(rnd(d, 16, scale=d ** -0.5))
+    lora.lora_B.data.copy_(rnd(16, d, scale=0.02))
+    assert bool(ops._scratch_bytes(rows, batch, wide, d, 8)) == (rows > 200)   # which of the cases decode
+    x0, vec0 = rnd(batch, rows, d, dtype=torch.float32), rnd(batch, d)
+    mask = torch.zeros(batch, rows, device="cuda")
+    mask[:, rows - rows // 5:] = 1e9
+    zeros, gates = torch.zeros_like(mask), rnd(batch, rows, d)
+    other = torch.cuda.Stream()
+
+    def step(x):
+        def s(t):
+            if sync:
+                torch.cuda.synchronize()
+            return t
+        vec = vec0.clone()
+        qkv, nbuf = x.new_empty(batch, rows, 3 * d, dtype=torch.bfloat16), x.new_empty(x.shape, dtype=torch.bfloat16)
+        side_out = torch.zeros_like(nbuf[:, :64])
+        for i in range(3):
+            mod = s(cond(s(ops.vec_sum_act(vec, act="silu"))))
+            mod8 = s(ops.qlinear(s(ops.vec_sum_act(vec, mod[:, :d].contiguous(), act="tanh")), *cond8._tensors(), bits=8))
+            s(ops.norm_modulate(x, mod[:, :d], mod8[:, d:2 * d], out=nbuf))
+            here = torch.cuda.current_stream()
+            other.wait_stream(here)
+            with torch.cuda.stream(other):
+                s(ops.qlinear(nbuf[:, :64], *out_l._tensors(), bits=8, prepared=out_l.prepared(), out=side_out))
+            s(qkv_l(nbuf, out=qkv))
+            here.wait_stream(other)
+            bias = s(ops.euler_step(zeros, mask, -1.0 if i < 2 else -1e-9))
+            s(ops.fmha(qkv, heads, out=nbuf, key_bias=bias))
+            s(ops.act_mul(nbuf, gates))
+            s(ops.gate_residual(s(out_l(nbuf)), mod[:, 2 * d:], x))
+            s(lora(nbuf, epilogue="gate_residual", gate=mod8[:, 2 * d:], residual=x, out=x))
+            s(ops.norm_modulate(x, mod[:, d:2 * d], mod8[:, :d], out=nbuf))
+            y = s(down(s(up(nbuf, epilogue="gelu"))))
+            y[:, :64] += side_out
+            comb = s(ops.cfg_combine(y[..., :64].contiguous(), nbuf[..., :64].contiguous(), 2.0))
+            x[..., :64] += comb
+            s(ops.gate_residual(y, mod8[:, :d], x))
+            vec = s(ops.vec_sum_act(vec, nbuf[:, 0].contiguous()))
+        return x
+    return step, x0
+
+
+def _same_bits(form, *args):
     from mflux_b200 import ops
 
-    step, x0 = _chain(rows, d, heads, True)
+    step, x0 = form(*args, True)
     ref = step(x0.clone())
-    step, x0 = _chain(rows, d, heads, False)
+    assert torch.isfinite(ref).all()
+    step, x0 = form(*args, False)
     for _ in range(3):
         assert torch.equal(step(x0.clone()), ref)
     side = torch.cuda.Stream()
@@ -79,3 +145,13 @@ def test_chain(lib_built, rows, d, heads):
         torch.cuda.synchronize()
         assert torch.equal(x, ref)
     assert ops.poll_device_status() == 0
+
+
+@pytest.mark.parametrize("rows,d,heads", [(1, 256, 2), (40, 256, 2), (300, 768, 6), (2100, 512, 4)])
+def test_chain(lib_built, rows, d, heads):
+    _same_bits(_chain, rows, d, heads)
+
+
+@pytest.mark.parametrize("batch,rows", [(2, 200), (2, 1100), (1, 4608)])
+def test_large_chain(lib_built, batch, rows):
+    _same_bits(_large_chain, batch, rows)
