@@ -3,7 +3,8 @@
 // ctypes (thirty attribute reads, a struct filled field by field) it took 12.8 us beside a kernel of 4.4 us.
 // linear() takes a call only when it would do exactly what ops.qlinear does with it; for everything else, and for every
 // error, it returns None and the Python path decides and raises. The library's functions come by address from the
-// loaded libmfx.so (bind()), so this module links against torch only.
+// loaded libmfx.so (bind()), so this module links against torch only. The interpreter lock is held for looking at the
+// arguments only: allocation and launch may wait for the device, and other threads run meanwhile.
 #include <Python.h>
 
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -65,6 +66,12 @@ bool same_weight(PyObject* key, const at::Tensor* const (&t)[3]) {
   return true;
 }
 
+// Lets other Python threads run while it lives.
+struct WithoutInterpreterLock {
+  PyThreadState* state = PyEval_SaveThread();
+  ~WithoutInterpreterLock() { PyEval_RestoreThread(state); }
+};
+
 // linear(x, weight, scales, biases, bias, prepared, bits, group_size, epilogue) -> Tensor or None
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -116,12 +123,21 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t n_out = epilogue == MFX_EPI_SWIGLU ? n / 2 : n;
   at::DimVector shape(x->sizes().begin(), x->sizes().end());
   shape[dims - 1] = n_out;
-  at::Tensor y = at::empty(shape, x->options().requires_grad(false));
-  a.y = y.data_ptr();
+  const at::TensorOptions options = x->options().requires_grad(false);
+  at::Tensor y;
+  int status;
   a.y_dtype = MFX_BF16;
   a.y_row_stride = n_out;
   a.y_batch_stride = dims == 3 ? a.rows * n_out : 0;
-  if (qlinear_fn(&a, c10::cuda::getCurrentCUDAStream(c10::cuda::current_device()).stream()) != MFX_OK) Py_RETURN_NONE;
+  {
+    // No Python object is touched in here, and none of the arguments' tensors (another thread may replace their data):
+    // what the call needs was copied out above, and the caller's references keep the objects.
+    WithoutInterpreterLock unlocked;
+    y = at::empty(shape, options);
+    a.y = y.data_ptr();
+    status = qlinear_fn(&a, c10::cuda::getCurrentCUDAStream(c10::cuda::current_device()).stream());
+  }
+  if (status != MFX_OK) Py_RETURN_NONE;
   return THPVariable_Wrap(std::move(y));
   END_HANDLE_TH_ERRORS
 }

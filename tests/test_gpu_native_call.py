@@ -134,3 +134,39 @@ def test_streams_and_capture(lib_built):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, ref)
+
+
+def test_other_threads_run_while_a_launch_waits(lib_built):
+    """With a full launch queue a call waits for the device; another Python thread goes on meanwhile."""
+    import threading
+    import time
+
+    layer = _layer()
+    x = torch.randn(2, 192, device="cuda").to(torch.bfloat16)
+    layer(x)
+    done, gaps = threading.Event(), []
+
+    def tick():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(1e-3)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    torch.cuda.synchronize()
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(3_000_000_000)       # one and a half seconds and more
+        longest = 0.0
+        for _ in range(3000):                  # more launches than the queue holds
+            begin = time.perf_counter()
+            layer(x)
+            longest = max(longest, time.perf_counter() - begin)
+    finally:
+        done.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert longest > 0.5, "no call had to wait"
+    assert max(gaps) < longest / 2, (max(gaps), longest)
