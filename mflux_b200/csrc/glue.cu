@@ -264,7 +264,8 @@ cudaError_t launch_norm_one(const NormParams& p, cudaStream_t st) {
   auto kern = norm_modulate_kernel<XT, BF, MAX_D, MOD, WEIGHT>;
   static const int per_sm = [&] {
     int n = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NORM_THREADS, 0) == cudaSuccess && n > 0 ? n : 4;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NORM_THREADS, 0) != cudaSuccess) cudaGetLastError();
+    return n > 0 ? n : 4;
   }();
   const int64_t total = static_cast<int64_t>(p.rows) * p.batch, resident = per_sm * device_sm_count();
   return launch_overlapped(kern, static_cast<unsigned>(total < resident ? total : resident), NORM_THREADS, 0, st, p);

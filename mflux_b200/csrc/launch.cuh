@@ -35,7 +35,10 @@ cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, 
   cfg.stream = stream;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  // a failure is the returned value's alone: left pending it would be the next ordinary launch's cudaGetLastError()
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 }  // namespace mfx
