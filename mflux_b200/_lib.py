@@ -8,6 +8,8 @@ errors as Python exceptions.
 from __future__ import annotations
 
 import ctypes
+import sysconfig
+import warnings
 from ctypes import c_char_p, c_int, c_int64, c_void_p
 from pathlib import Path
 
@@ -291,22 +293,40 @@ def load() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.restype = res
         fn.argtypes = args
-    _host().bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in
-                   ("mfx_qlinear_ex", "mfx_qlinear_scratch_bytes_batch", "mfx_qlinear_prepared_bytes")))
     _lib = lib
     return lib
 
 
-def _host():
-    """The native form of a quantized linear's call (csrc/host_call.cpp)."""
-    import torch  # noqa: F401  (brings the libraries the module is linked against)
+_host_module = None      # False: looked for, and not usable
 
-    try:
-        from . import _host as host
-    except ImportError as e:
-        raise RuntimeError("mflux_b200/_host.so is missing or was built for another torch: run `python -m "
-                           f"mflux_b200.build` ({e})") from e
-    return host
+
+def _host():
+    """The native form of a quantized linear's call (csrc/host_call.cpp), or None, with a warning, where the module is missing
+    or was built for another torch or Python: it only saves host time, ops.qlinear makes the same calls without it."""
+    global _host_module
+    if _host_module is None:
+        import torch  # brings the libraries the module is linked against
+
+        running = f"torch {torch.__version__} {sysconfig.get_config_var('SOABI')}"
+        why = None
+        try:
+            from . import _host as module
+
+            built_for = getattr(module, "BUILT_FOR", "an unknown torch")
+            if built_for != running:
+                why = f"was built for {built_for}, this is {running}"
+        except ImportError as e:
+            why = f"does not load: {e}"
+        if why is not None:
+            warnings.warn(f"mflux_b200/_host.so {why}. Calls of a few rows take about 7 us longer without it; "
+                          "`python -m mflux_b200.build` builds it again.", RuntimeWarning, stacklevel=3)
+            _host_module = False
+        else:
+            lib = load()
+            module.bind(*(ctypes.cast(getattr(lib, name), c_void_p).value for name in
+                          ("mfx_qlinear_ex", "mfx_qlinear_scratch_bytes_batch", "mfx_qlinear_prepared_bytes")))
+            _host_module = module
+    return _host_module or None
 
 
 def check(status: int, what: str) -> None:

@@ -50,20 +50,37 @@ def _stale(obj: Path, src: Path, headers: list[Path]) -> bool:
     return any(p.stat().st_mtime > t for p in [src, *headers])
 
 
+def host_builds_for() -> str:
+    """What the host module is tied to: the torch build whose inlined tensor layouts it has, and the Python ABI."""
+    spec = importlib.util.spec_from_file_location("_torch_version", _torch() / "version.py")
+    version = importlib.util.module_from_spec(spec)     # without importing torch itself
+    spec.loader.exec_module(version)
+    return f"torch {version.__version__} {sysconfig.get_config_var('SOABI')}"
+
+
+def _torch() -> Path:
+    return Path(importlib.util.find_spec("torch").origin).parent
+
+
 def build_host(force: bool, headers: list[Path]) -> None:
-    """The CPython module of csrc/host_call.cpp, against the headers and libraries of the installed torch."""
-    src = CSRC / "host_call.cpp"
-    if not force and not _stale(HOST, src, headers):
+    """The CPython module of csrc/host_call.cpp, against the headers and libraries of the installed torch. Stale, too, when
+    it was built for another torch or Python; the module carries the same text for the loader to compare."""
+    src, record = CSRC / "host_call.cpp", OBJ / "_host.built_for"
+    built_for = host_builds_for()
+    known = record.read_text() if record.exists() else None
+    if not force and known == built_for and not _stale(HOST, src, headers):
         return
-    torch = Path(importlib.util.find_spec("torch").origin).parent
+    torch = _torch()
     cuda = Path(_nvcc()).resolve().parent.parent
-    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall",
+    record.unlink(missing_ok=True)     # nothing is known about what a failure below leaves
+    cmd = [shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f'-DMFX_BUILT_FOR="{built_for}"',
            "-I", str(ROOT / "include"), "-I", str(torch / "include"), "-I", str(torch / "include/torch/csrc/api/include"),
            "-I", str(cuda / "include"), "-I", sysconfig.get_paths()["include"], str(src), "-o", str(HOST),
            "-L", str(torch / "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"build of {HOST.name} failed:\n{r.stdout}\n{r.stderr}")
+    record.write_text(built_for)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:

@@ -168,4 +168,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+  PyObject* m = PyModule_Create(&module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "BUILT_FOR", MFX_BUILT_FOR) != 0) Py_CLEAR(m);
+  return m;
+}

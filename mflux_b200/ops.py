@@ -336,8 +336,10 @@ def plain_qlinear(x, wq, scales, biases, bias, prepared, bits: int, group_size: 
     if TRACE is not None:
         return None
     if _native is None:
-        _lib.load()
-        _native = _lib._host().linear
+        module = _lib._host()
+        _native = False if module is None else module.linear
+    if _native is False:
+        return None
     y = _native(x, wq, scales, biases, bias, prepared, bits, group_size, _EPI[epilogue])
     if y is not None:
         LAUNCHES[0] += 1
