@@ -1,7 +1,8 @@
-"""Few rows over weights of 24 M (two or four rows) and 48 or 36 M (eight) and more: every share of a tile's pieces among warps (1, 2, 4, 8), one and several
-rounds of tiles, a last tile of eight rows, a last piece of one group, activations with row strides, against float64 on the
-packed weights. Bound: float32 sums of up to 15360 terms and, for 4 bits, the offset of 128 that is taken out again (2^-24 of
-128 Sum |x| per group against a result of about 5 |x| sqrt(64) codes: 2e-5 in the worst case, a tenth of it on average)."""
+"""Few rows over weights of 24 M (two or four rows) and 48 or 36 M (eight) and more: every share of a tile's pieces among
+warps (1, 2, 4, 8), one and several rounds of tiles, a last tile of eight rows, a last piece of one group, activations with
+row strides, against float64 on the packed weights. Bound: float32 sums of up to 15360 terms and, for 4 bits, the offset of
+128 that is taken out again (2^-24 of 128 Sum |x| per group against a result of about 5 |x| sqrt(64) codes: 2e-5 in the worst
+case, a tenth of it on average)."""
 import pytest
 import torch
 
