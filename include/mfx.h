@@ -196,6 +196,12 @@ typedef struct mfx_qlinear_args {
   int64_t lora_r;
   const mfx_tp_scatter* scatter; /* host pointer; required for MFX_EPI_PEER_SCATTER (then y may be NULL) */
 } mfx_qlinear_args;
+/* Which kernel takes a call, and with it the rounding of a row's result, depends on the sizes: one sample of at most 16
+ * rows without a low-rank term and with no epilogue beyond SiLU goes to one of two kernels that stream the weight, the
+ * rest to the tensor-core kernels. Those, and the streaming kernel for small weights or more rows, round each weight to
+ * bf16; the streaming kernel for large ones (from 24 M weights on up to two rows at 4 bits and four at 8, from 48 M and
+ * 36 M on up to eight) does not. So a row's result can change by about 1e-3 (relative 2-norm) with the number of rows in
+ * the call; within one kernel it does not. */
 int mfx_qlinear_ex(const mfx_qlinear_args* args /* host */, void* stream);
 
 /* mfx_qlinear_ex with scratch for the decoded weight. With at least 2 N K bytes (256-byte aligned device memory,

@@ -176,7 +176,8 @@ __device__ __forceinline__ float block_sum_128(float v, float* red) {
 constexpr int NORM_THREADS = 128;
 constexpr int NORM_MAX_D = 4096;
 
-// The kernels' largest row; D <= NORM_MID_D (the widest of the models but one) holds a quarter fewer registers.
+// The kernels' largest row; D <= NORM_MID_D (the widest of the models but one) holds a quarter fewer values per thread: 111
+// registers instead of 128 for float32 rows with shift and scale, 80 instead of 114 with a weight.
 constexpr int NORM_MID_D = 3072;
 
 // Blocks of 128 threads stride over the rows. Thread t holds the 16-byte vectors t, t+128, ... of its row in registers,
@@ -184,8 +185,8 @@ constexpr int NORM_MID_D = 3072;
 // (two-pass variance). The next row is on its way while this one is reduced, and the shift, scale and weight of a
 // channel stay in registers for all rows of a block: a block per row spent most of its life waiting for its own loads,
 // one after the other, and read 2/3 of the row's bytes again in shift and scale. HBM bounds it: 65536 x 3072 float32 rows
-// 308 -> 218 us (5.5 TB/s), 4608 rows 18.9 -> 14.3 us (from L2), 512 rows 5.6 -> 3.6 us; 1632 x 3840 with weight 12.7 ->
-// 9.3 us.
+// 308 -> 213 us (5.7 TB/s), from L2 4608 rows 18.8 -> 14.0 us, 512 rows 5.6 -> 3.6 us (3.2 where launches overlap), 1632 x
+// 3840 with weight 12.7 -> 8.1 us (5.2).
 template <typename XT, bool BF, int MAX_D, bool MOD, bool WEIGHT>
 __global__ void __launch_bounds__(NORM_THREADS) norm_modulate_kernel(const NormParams p) {
   wait_for_predecessor();
@@ -341,8 +342,8 @@ struct PostNormParams {
 // of the projection, so it cannot be an epilogue of a matmul tiled along N; this pass reads y once.
 // One 128-thread block per row, 4 elements per vector (8-byte loads of bf16 y, 16-byte of the f32 residual).
 // Everything of the first stage is asked for before its reduction, the second stage's vectors before the second one (with
-// the loads where the values are used a block waited for three trips to memory): 1632 x 3840 rows, both stages, 34.0 -> 19.2
-// us with the operands in HBM, 20.8 -> 12.1 us in L2; 8426 rows 104 -> 83 us.
+// the loads where the values are used a block waited for three trips to memory): 1632 x 3840 rows, both stages, 34.0 -> 16.1
+// us with the operands in HBM, 20.8 -> 11.1 us in L2; 8426 rows 104 -> 69 us.
 // With next_out the block goes on to the pre-norm of the following sub-layer on the row it just updated
 // (transformer_block.py:34 after :31, and the next block's :29-30 after :35), which saves reading the stream again.
 template <typename YT, bool BF>

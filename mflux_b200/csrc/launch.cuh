@@ -14,8 +14,10 @@ namespace mfx {
 // Such a kernel reads global memory by plain loads, TMA and cp.async only, never by the read-only path (__ldg, const
 // __restrict__): that path is for memory which nobody writes while the kernel lives, and this one lives while its
 // predecessor still writes. The compiler may also move its loads across the wait, a plain load not (the clobber below).
-// Without / with it, looped: 24 heads x 4608 tokens of attention back to back 241.5 / 232.1 us, a step of 380 launches (8-bit
-// single-stream model, 1613 tokens) 22.26 / 21.97 ms, a guidance pair of the dual-stream model at 7145 tokens 248.1 / 246.6.
+// Without / with it: kernels of a few microseconds one after the other 0.3 to 0.5 us less each (256 x 256 decoded 1.54 /
+// 1.13, 333 tokens x 24 heads of attention 10.2 / 9.1), 333 rows of N 9216, K 3072, 4 bits 25.4 / 24.4 us, a step of 380
+// launches (8-bit single-stream model, 1613 tokens) 22.21 / 21.82 ms; 24 heads x 4608 tokens of attention 239.5 / 239.1, which
+// is noise.
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // From here on the successor's blocks may be started. They only come to a SM as this kernel's blocks leave it room.
 __device__ __forceinline__ void allow_successor() {

@@ -629,8 +629,11 @@ int launch_epi(const CUtensorMap& tx, const CUtensorMap& tw, const CUtensorMap& 
   // Four epilogue warps keep up with the main loop where they add a bias or a residual, not where each value goes through
   // erff, tanhf or an exponential: a tile then waits for its predecessor's epilogue. Eight share the columns. M 4096, N
   // 12288, K 3072, 4 bits, us: erf form 299 -> 273 (260 -> 233 below the power limit), tanh form 280 -> 264 (240 -> 227),
-  // without activation 250; M 2000, N 3072, K 3072, SiLU 49.2 -> 42.8. Eight without one cost 1 % (146.6 -> 149.5 at 8
-  // bits, M 1632, N 11520, K 3840), and leave the gated residual 72 registers instead of 80.
+  // without activation 250; M 2000, N 3072, K 3072, SiLU 49.2 -> 42.8. 8 bits: M 512, N 12288, K 3072, erf form 45.9 -> 40.5,
+  // tanh form 41.4 -> 40.8; M 1024, N 3072, K 3072 27.8 -> 24.3; M 4096, N 12288 the same within noise. SwiGLU, 8 bits (4
+  // bits): M 1613, N 20480, K 3840 210.6 -> 206.4 (180.3 -> 179.0), M 2000, N 10240, K 2560 88.5 -> 85.2 (87 -> 75). Eight
+  // without one cost 1 % (146.6 -> 149.5 at 8 bits, M 1632, N 11520, K 3840), and leave the gated residual 72 registers
+  // instead of 80.
   constexpr int EPI_WARPS =
       EPI == MFX_EPI_GELU_ERF || EPI == MFX_EPI_GELU_TANH || EPI == MFX_EPI_SILU || EPI == MFX_EPI_SWIGLU ? 8 : 4;
   constexpr int NUM_THREADS = (FIRST_EPI_WARP + EPI_WARPS + TEAMS * NDQ) * 32;

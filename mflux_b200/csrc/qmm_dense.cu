@@ -370,9 +370,8 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, voi
                    static_cast<unsigned>((K + DEC_ITERS * 512 - 1) / (DEC_ITERS * 512)));
   if (dgrid.y > 65535) return MFX_ERR_TOO_LARGE;
   __nv_bfloat16* w = static_cast<__nv_bfloat16*>(scratch);
-  // An ordinary launch: its thousands of blocks, started early, would sit on the SMs that the kernel before is still to use
-  // (8 bits, M 4096, N 12288, K 3072: 252.1 us, overlapped 255.0, both kernels ordinary 252.5; M 73728, N 9216, 4 bits: 3018,
-  // 3027, 3032).
+  // An ordinary launch, by measurement (8 bits, M 4096, N 12288, K 3072: 252.1 us, overlapped 255.0, both kernels ordinary
+  // 252.5; M 73728, N 9216, 4 bits: 3018, 3027, 3032): the decoder does not wait for its predecessor.
   if (kb == 4) decode_kernel<4><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
   else decode_kernel<8><<<dgrid, 256, 0, st>>>(codes, sb, N, K, w);
   MFX_CUDA_TRY(cudaGetLastError());

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1) stream_kernel(const Params p) 
         const int row = 2 * t + i;
         if (row >= p.M) continue;
         float v = acc[2 * h + i];
-        if (!(fabsf(v) <= 3.0e38f)) 
+        if (!(fabsf(v) <= 3.0e38f))
           v = direct_dot<BITS>(p.codes + n * (row_bytes / 4), p.sb + n, p.N, p.x + row * p.x_row_stride, p.K);
         v += bias;
         if (p.epilogue == MFX_EPI_SILU) v = v / (1.0f + __expf(-v));
@@ -499,11 +499,12 @@ int run(const Params& p, cudaStream_t st) {
 // From 24 M weights on; with fewer the start of a block of this size is what a call takes (N 6144, K 3072, 4 bits, three
 // rows: 8.6 us against 7.5). The other kernel / this one, at 1, 4, 8 rows: 4 bits, N 9216, K 3072 10.1 / 8.6, 10.2 / 9.7,
 // 10.9 / 11.4; N 11520, K 4096 13.2 / 12.4, 13.3 / 13.5, 14.3 / 15.5; N 12288, K 4096 15.9 / 12.6, 15.9 / 13.8, 16.1 / 15.6;
-// N 20480, K 3840 21.5 / 19.4, 21.8 / 20.6, 22.5 / 22.3; 8 bits, N 8192, K 4096 14.1 / 11.5, 14.1 / 12.7, 14.1 / 14.6; N 12288, K
-// 3072 15.5 / 12.3, 15.5 / 13.4, 15.6 / 14.6; N 15360,
-// K 3840 21.1 / 17.7, 21.2 / 18.9, 21.3 / 20.7. Every row costs here (it is copied into each block's shared memory and its sums
-// per group are formed there) and almost nothing there, so more rows need more weights to read; at 4 bits, three rows, N
-// 10240, K 3840 13.1 / 13.4. A plain read of the 33 MB of the 8-bit N 8192, K 4096 takes 6.2 us.
+// N 20480, K 3840 21.5 / 19.4, 21.8 / 20.6, 22.5 / 22.3; 8 bits, N 8192, K 4096 14.1 / 11.5, 14.1 / 12.7, 14.1 / 14.6; N
+// 12288, K 3072 15.5 / 12.3, 15.5 / 13.4, 15.6 / 14.6; N 15360, K 3840 21.1 / 17.7, 21.2 / 18.9, 21.3 / 20.7. Every row costs
+// here (it is copied into each block's shared memory and its sums per group are formed there) and almost nothing there, so
+// more rows need more weights to read; at 4 bits, three rows, N 10240, K 3840 13.1 / 13.4. A plain read of the 33 MB of the
+// 8-bit N 8192, K 4096 takes 6.2 us. The two kernels round differently (weights to bf16 there, not here), so a row's result
+// may differ by about 1e-3 with the number of rows beside it; the C header says so.
 template <int BITS>
 bool pays(const Params& p) {
   const int64_t weights = static_cast<int64_t>(p.N) * p.K;
@@ -540,9 +541,11 @@ int run(const mfx_qlinear_args& a, const void* prepared, size_t codes_bytes, cud
   const unsigned blocks = static_cast<unsigned>(wide ? (a.N + 15) / 16 : (a.N + 7) / 8);
   auto kern = kernel_bits(a.bits) == 4 ? (wide ? qmv_kernel<4, 2> : qmv_kernel<4, 1>)
                                        : (wide ? qmv_kernel<8, 2> : qmv_kernel<8, 1>);
-  // An ordinary launch: with more blocks than fit at once, those that start early only hold back the ones before them
-  // (overlapped / ordinary: five rows, N 3840, K 12288, 4 bits 20.3 / 17.9 us, four rows, N 3072, K 4096, 8 bits 8.4 / 7.6;
-  // two rows, N 15360, K 256, 8 bits 3.9 / 4.1).
+  // An ordinary launch, before which everything in the stream has finished: this kernel does not wait for its predecessor.
+  // Overlapped, most calls would gain up to half a microsecond and some lose more, by no rule of blocks or bytes that we
+  // found. Overlapped / ordinary, us, one after the other: four rows, N 3072, K 4096, 8 bits 8.4 / 7.1, five rows, N 3840, K
+  // 12288, 4 bits 20.1 / 17.8, 16 rows, N 9216, K 3072, 4 bits 15.4 / 14.4, two rows, N 3072, K 768, 4 bits 2.56 / 2.45; two
+  // rows, N 15360, K 256, 8 bits 4.0 / 4.2, one row, N 3072, K 256, 8 bits 1.84 / 1.93, N 6144, K 3072, 4 bits 6.7 / 7.3.
   kern<<<blocks, THREADS, 0, st>>>(p);
   MFX_CUDA_TRY(cudaGetLastError());
   return MFX_OK;

@@ -58,3 +58,15 @@ def test_values_that_are_not_finite(lib_built, n, k, bits):
     assert torch.equal(torch.isinf(y), torch.isinf(ref)) and torch.equal(y[torch.isinf(y)], ref[torch.isinf(ref)])
     fine = torch.isfinite(ref)
     assert ((y[fine].double() - ref[fine].double()).norm() / ref[fine].double().norm()).item() <= 4e-3
+
+
+@pytest.mark.parametrize("n,k,bits,rows", [(9216, 3072, 4, (1, 2)), (9216, 3072, 4, (3, 5, 16)), (9216, 3072, 8, (1, 3, 4)),
+                                           (20480, 3840, 4, (1, 4, 8)), (3072, 256, 4, (1, 8, 9, 16))])
+def test_a_row_does_not_depend_on_the_others(lib_built, n, k, bits, rows):
+    """Within the sizes that one kernel takes (include/mfx.h): equal bits with any rows beside it."""
+    from mflux_b200 import ops
+
+    q, prepared, _ = _weight(n, k, bits)
+    x = torch.randn(16, k, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).to(torch.bfloat16)
+    first = [ops.qlinear(x[:m], *q, bits=bits, prepared=prepared, out_dtype=torch.float32)[0] for m in rows]
+    assert all(torch.equal(first[0], y) for y in first[1:])
