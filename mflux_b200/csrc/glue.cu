@@ -61,10 +61,9 @@ struct NormParams {
   int64_t y_row_stride, y_batch_stride;
 };
 
-// Loads of vectors that the kernel itself does not write. Volatile, so that they stay behind the wait for the predecessor and
-// behind bounds tests; with no claim on memory, so that they may move past the kernel's own stores, which a plain load may
-// not. With plain loads / with these, us: 4096 x 4096 float32 rows with shift and scale 21.9 / 19.4, q/k norm and RoPE of 1613
-// tokens, 30 heads 12.2 / 11.6; the post-norm's vectors are the other way round (1632 x 3840 rows 16.1 / 18.8).
+// Vectors that the kernel does not write, by loads that may pass its stores (scalar.cuh). With plain loads / with these, us:
+// 4096 x 4096 float32 rows with shift and scale 21.9 / 19.4, q/k norm and RoPE of 1613 tokens, 30 heads 12.2 / 11.6; the
+// post-norm's vectors are the other way round (1632 x 3840 rows 16.1 / 18.8).
 __device__ __forceinline__ uint4 load_uint4(const void* p) {
   uint4 v;
   asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -74,11 +73,6 @@ __device__ __forceinline__ uint2 load_uint2(const void* p) {
   uint2 v;
   asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
   return v;
-}
-__device__ __forceinline__ float load_half(const void* p, int64_t i) {
-  unsigned short v;
-  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(static_cast<const __half*>(p) + i));
-  return __half2float(__ushort_as_half(v));
 }
 __device__ __forceinline__ float4 load_float4(const void* p) {
   const uint4 v = load_uint4(p);
@@ -107,7 +101,7 @@ __device__ __forceinline__ void load_vec(const void* p, int dtype, int64_t off, 
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < E; ++i) o[i] = load_half(p, off + i);
+    for (int i = 0; i < E; ++i) o[i] = load_as_float(p, dtype, off + i);
   }
 }
 // 16 bytes of float32 or bf16 values as floats.
@@ -612,14 +606,16 @@ __global__ void __launch_bounds__(256) gate_residual_kernel(const void* y, int y
   float o[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float bv = bias ? load_as_float(bias, bias_dtype, col + j) : 0.f;
-    const float gv = load_as_float(gate, gate_dtype, b * gate_batch_stride + col + j);
+    const float bv = bias ? load_as_float<false>(bias, bias_dtype, col + j) : 0.f;
+    const float gv = load_as_float<false>(gate, gate_dtype, b * gate_batch_stride + col + j);
     o[j] = rv[j] + gv * (yv[j] + bv);
   }
   *reinterpret_cast<float4*>(out + roff) = make_float4(o[0], o[1], o[2], o[3]);
   *reinterpret_cast<float4*>(out + roff + 4) = make_float4(o[4], o[5], o[6], o[7]);
 }
 
+// Plain loads in this kernel and the one above: 2000 x 1024 float32 channels 12.4 us, 25.5 with loads that may pass its
+// stores; 512 rows of 3072 above 6.6 and 7.2.
 // Classifier-free-guidance combine of two noise predictions, one warp per token row of C <= 1024 channels.
 // mode 0: out = n + g * (n - n_neg)                              (z_image.py:209)
 // mode 1: comb = n_neg + g * (n - n_neg); out = comb * ||n|| / ||comb|| over the channel axis, eps 1e-12
@@ -634,7 +630,7 @@ __global__ void __launch_bounds__(256) cfg_combine_kernel(const void* n, const v
   if (row >= rows) return;
   float sn = 0.f, sc = 0.f;
   for (int c = lane; c < C; c += 32) {
-    const float a = load_as_float(n, dtype, row * C + c), b = load_as_float(nn, dtype, row * C + c);
+    const float a = load_as_float<false>(n, dtype, row * C + c), b = load_as_float<false>(nn, dtype, row * C + c);
     const float comb = mode == 0 ? a + g * (a - b) : b + g * (a - b);
     sn += a * a;
     sc += comb * comb;
@@ -642,7 +638,7 @@ __global__ void __launch_bounds__(256) cfg_combine_kernel(const void* n, const v
   float ratio = 1.f;
   if (mode == 1) ratio = sqrtf(warp_sum(sn) + 1e-12f) / sqrtf(warp_sum(sc) + 1e-12f);
   for (int c = lane; c < C; c += 32) {
-    const float a = load_as_float(n, dtype, row * C + c), b = load_as_float(nn, dtype, row * C + c);
+    const float a = load_as_float<false>(n, dtype, row * C + c), b = load_as_float<false>(nn, dtype, row * C + c);
     const float comb = mode == 0 ? a + g * (a - b) : b + g * (a - b);
     out[row * C + c] = comb * ratio;
   }
