@@ -184,7 +184,8 @@ class QuantizedLinear(Module):
                 residual: torch.Tensor | None = None, out: torch.Tensor | None = None,
                 out_dtype: torch.dtype | None = None) -> torch.Tensor:
         weight, scales, biases, bias = self._tensors()
-        if out is None and gate is None and residual is None and out_dtype is None and self._prepared is not None:
+        if (out is None and gate is None and residual is None and out_dtype is None and self._prepared is not None
+                and type(self).prepared is _PREPARED):
             y = ops.plain_qlinear(x, weight, scales, biases, bias, self._prepared, self.bits, self.group_size, epilogue)
             if y is not None:
                 return y
@@ -195,6 +196,9 @@ class QuantizedLinear(Module):
     def dequantize(self, dtype: torch.dtype | None = None) -> torch.Tensor:
         return ops.dequantize_affine(self.weight.data, self.scales.data, self.biases.data, self.group_size, self.bits,
                                      dtype)
+
+
+_PREPARED = QuantizedLinear.prepared     # a subclass with a prepared form of its own is asked for it on every call
 
 
 def quantize(model: torch.nn.Module, group_size: int = 64, bits: int = 4,

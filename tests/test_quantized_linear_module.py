@@ -59,6 +59,22 @@ def test_plain_parameters_and_no_bias(calls):
     assert (calls[1]["prepared"][1] == 6.0).all()
 
 
+class _OwnBlob(nn.QuantizedLinear):
+    def prepared(self):
+        return "own", super().prepared()
+
+
+def test_a_subclass_with_a_prepared_form_of_its_own(calls, monkeypatch):
+    monkeypatch.setattr(ops, "plain_qlinear", lambda *a: "the base class's form")
+    layer = _OwnBlob(64, 8)
+    for _ in range(2):       # the second time the base class's form is there, too
+        layer(torch.zeros(1, 64))
+    assert [c["prepared"][0] for c in calls] == ["own", "own"]
+    plain = _layer()
+    plain(torch.zeros(1, 64))
+    assert plain(torch.zeros(1, 64)) == "the base class's form"
+
+
 class _Tagged(nn.QuantizedLinear):
     def __init__(self, *args, **kw):
         super().__init__(*args, **kw)
