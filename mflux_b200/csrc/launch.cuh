@@ -11,9 +11,10 @@ namespace mfx {
 // to memory that another kernel may write or read. Returns once the predecessor has finished and its writes are visible
 // (at once where the launch was an ordinary one). Every thread of every such kernel calls it before anything else that
 // touches global memory, so a kernel's end still means the end of everything before it in the stream.
-// Such a kernel reads global memory by plain loads, TMA and cp.async only, never by the read-only path (__ldg, const
+// Such a kernel reads global memory by plain or volatile loads, TMA and cp.async, never by the read-only path (__ldg, const
 // __restrict__): that path is for memory which nobody writes while the kernel lives, and this one lives while its
-// predecessor still writes. The compiler may also move its loads across the wait, a plain load not (the clobber below).
+// predecessor still writes. The compiler may also move its loads across the wait, the others not (they come behind volatile assembly
+// that clobbers memory).
 // Without / with it: kernels of a few microseconds one after the other 0.3 to 0.5 us less each (256 x 256 decoded 1.54 /
 // 1.13, 333 tokens x 24 heads of attention 10.2 / 9.1), 333 rows of N 9216, K 3072, 4 bits 25.4 / 24.4 us, a step of 380
 // launches (8-bit single-stream model, 1613 tokens) 22.21 / 21.82 ms; 24 heads x 4608 tokens of attention 239.5 / 239.1, which

@@ -331,7 +331,8 @@ _native = None
 
 def plain_qlinear(x, wq, scales, biases, bias, prepared, bits: int, group_size: int, epilogue: str | None):
     """The common form of a module's call in native code, or None where qlinear() has to take it (csrc/host_call.cpp says
-    when; always without a usable module). `prepared` is nn.QuantizedLinear's (key, blob) pair; a key that no longer fits its tensors gives None too."""
+    when; always without a usable module). `prepared` is nn.QuantizedLinear's (key, blob) pair; a key that no longer fits its
+    tensors gives None too."""
     global _native
     if TRACE is not None:
         return None
